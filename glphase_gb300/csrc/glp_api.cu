@@ -105,6 +105,10 @@ struct glp_ctx {
   size_t mask_cap = 0;
   uint16_t *d_knn_dist = nullptr;  // kNN distances of a chunk of samples [2 n][H]
   size_t knn_dist_cap = 0;
+  double *d_vq_sums = nullptr;  // codebook training: block sums, counts, codebooks
+  uint32_t *d_vq_counts = nullptr;
+  float2 *d_vq_books = nullptr;
+  size_t vq_sums_cap = 0, vq_counts_cap = 0, vq_books_cap = 0;
   uint8_t *d_tr_slot = nullptr, *d_acc = nullptr;
   double *d_tr_u = nullptr, *d_like = nullptr, *d_evals = nullptr;
   float *d_tr_work = nullptr;
@@ -710,6 +714,9 @@ void glp_destroy(glp_ctx *c) {
   release(c->d_nbr);
   release(c->d_mask);
   release(c->d_knn_dist);
+  release(c->d_vq_sums);
+  release(c->d_vq_counts);
+  release(c->d_vq_books);
   release(c->d_tr_slot);
   release(c->d_acc);
   release(c->d_tr_u);
@@ -1477,38 +1484,33 @@ int glp_vq_train(glp_ctx *c, const float *gl, uint64_t P, uint32_t K, float *cod
   const size_t smem = glp::vq_assign_smem(K);
   GLP_CUDA(c, cudaFuncSetAttribute(glp::vq_assign_kernel,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  double *d_sums = nullptr, *d_var = nullptr;
-  uint32_t *d_counts = nullptr;
-  float2 *d_cb = nullptr;
-  if (cudaMalloc((void **)&d_sums, (size_t)nb * (2 * K + 1) * sizeof(double)) != cudaSuccess ||
-      cudaMalloc((void **)&d_counts, (size_t)nb * K * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc((void **)&d_cb, K * sizeof(float2)) != cudaSuccess ||
-      cudaMalloc((void **)&d_var, sizeof(double)) != cudaSuccess) {
-    release(d_sums);
-    release(d_counts);
-    release(d_cb);
-    release(d_var);
-    return fail(c, GLP_ERR_NOMEM, "codebook training scratch");
-  }
+  // workspace of the context: block sums, block counts, two codebooks (the
+  // assignment's and the next) and the total squared distance
+  const size_t n_sums = (size_t)nb * (2 * K + 1);
+  if ((rc = ensure(c, c->d_vq_sums, c->vq_sums_cap, n_sums)) ||
+      (rc = ensure(c, c->d_vq_counts, c->vq_counts_cap, (size_t)nb * K)) ||
+      (rc = ensure(c, c->d_vq_books, c->vq_books_cap, 2 * (size_t)glp::kVQMaxCodes + 1)))
+    return rc;
+  float2 *const books[2] = {c->d_vq_books, c->d_vq_books + glp::kVQMaxCodes};
+  double *const d_var = reinterpret_cast<double *>(c->d_vq_books + 2 * glp::kVQMaxCodes);
   cudaStream_t st = c->stream;
-  auto assign = [&] {
-    glp::vq_assign_kernel<<<nb, glp::kVQThreads, smem, st>>>(gl, P, d_cb, K, d_sums, d_counts);
-  };
-  // totals of the last assignment: its squared distance, and with `move` the
-  // next entries (iteration `it`)
-  auto totals = [&](uint32_t it, bool move, double *var) -> cudaError_t {
-    glp::vq_update_kernel<<<1, 64, 0, st>>>(gl, P, nb, d_sums, d_counts, K, seed, it,
-                                            move ? d_cb : nullptr, d_var);
+  uint32_t it = 0, cur_book = 0;
+  // assigns every point to the current entries; var = their total squared
+  // distance, and the other codebook receives the entries of update it + 1
+  auto assign = [&](double *var) -> cudaError_t {
+    glp::vq_assign_kernel<<<nb, glp::kVQThreads, smem, st>>>(gl, P, books[cur_book], K,
+                                                             c->d_vq_sums, c->d_vq_counts);
+    glp::vq_update_kernel<<<1, glp::kVQUpdThreads, 0, st>>>(gl, P, nb, c->d_vq_sums,
+                                                            c->d_vq_counts, K, seed, it + 1,
+                                                            books[cur_book ^ 1], d_var);
     cudaError_t e = cudaMemcpyAsync(var, d_var, sizeof(double), cudaMemcpyDeviceToHost, st);
     return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
   };
-  cudaError_t e = cudaMemcpyAsync(d_cb, codebook, K * sizeof(float2), cudaMemcpyHostToDevice, st);
-  double cur = 0.0, prev = std::numeric_limits<double>::max(), dummy = 0.0;
-  uint32_t it = 0;
-  if (e == cudaSuccess) {
-    assign();
-    e = totals(0, false, &cur);
-  }
+  cudaError_t e =
+      cudaMemcpyAsync(books[0], codebook, K * sizeof(float2), cudaMemcpyHostToDevice, st);
+  double cur = 0.0, prev = std::numeric_limits<double>::max();
+  if (e == cudaSuccess)
+    e = assign(&cur);
   // GLVQ::BuildCodeBook's loop (glVQ.cpp:78-89)
   while (e == cudaSuccess && std::fabs(cur - prev) > cur / 100) {
     if (++it > max_iter) {
@@ -1517,20 +1519,17 @@ int glp_vq_train(glp_ctx *c, const float *gl, uint64_t P, uint32_t K, float *cod
       break;
     }
     prev = cur;
-    e = totals(it, true, &dummy);
-    if (e != cudaSuccess)
-      break;
-    assign();
-    e = totals(it, false, &cur);
+    cur_book ^= 1;
+    e = assign(&cur);
   }
-  if (e == cudaSuccess && rc == GLP_OK)
-    e = cudaMemcpy(codebook, d_cb, K * sizeof(float2), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && rc == GLP_OK) {
+    e = cudaMemcpyAsync(codebook, books[cur_book], K * sizeof(float2), cudaMemcpyDeviceToHost,
+                        st);
+    if (e == cudaSuccess)
+      e = cudaStreamSynchronize(st);
+  }
   if (e == cudaSuccess)
     e = cudaGetLastError();
-  release(d_sums);
-  release(d_counts);
-  release(d_cb);
-  release(d_var);
   if (e != cudaSuccess)
     return fail(c, GLP_ERR_CUDA, "codebook training: %s", cudaGetErrorString(e));
   if (iterations)
@@ -1553,10 +1552,11 @@ int glp_vq_pack(glp_ctx *c, const float *gl, uint32_t N, uint32_t S, const float
   glp::VQBook book;
   for (uint32_t k = 0; k < K; ++k)
     book.e[k] = make_float2(codebook[2 * k], codebook[2 * k + 1]);
-  const uint32_t per = 32u / bits;
-  const uint64_t total = (uint64_t)((S + per - 1) / per) * N;
-  glp::vq_pack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(gl, N, S, book, K,
-                                                                            bits, packed);
+  const uint64_t tiles =
+      (uint64_t)((N + glp::kVQPackSamples - 1) / glp::kVQPackSamples) *
+      ((S + (uint64_t)glp::kVQPackSites - 1) / glp::kVQPackSites);
+  glp::vq_pack_kernel<<<(unsigned)tiles, glp::kVQPackThreads, 0, c->stream>>>(
+      gl, N, S, book, K, bits, packed);
   GLP_CUDA(c, cudaGetLastError());
   return GLP_OK;
 }
