@@ -364,8 +364,8 @@ MultiFn multi_kernel(Shape sh, bool vq) {
 }
 
 // hmm_work of a generation: the recursions (blocks of two warps over 32
-// samples, backward and forward at once), then the sampling (one warp per
-// sample).  The recursions' staging tiles take more than the default 48 KB
+// samples, backward and forward at once), then the sampling (one warp per part
+// of a sample).  The recursions' staging tiles take more than the default 48 KB
 // of shared memory: allow_chain_smem opts the kernels in on the current
 // device (at context creation, before any launch or graph capture).
 cudaError_t allow_chain_smem() {
@@ -377,15 +377,51 @@ cudaError_t allow_chain_smem() {
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)glp::kChainSmem);
   return e;
 }
+uint64_t chain_blocks(uint64_t N) { return (N + glp::kChainSamples - 1) / glp::kChainSamples; }
 void launch_work(const glp::GenParams &p, uint64_t samples, cudaStream_t st) {
-  glp::work_chains_kernel<><<<(unsigned)((samples + glp::kPairRows - 1) / glp::kPairRows),
-                              glp::kChainThreads, glp::kChainSmem, st>>>(p);
-  glp::work_sample_kernel<><<<(unsigned)(samples * glp::sample_parts(p.wn)), 32, 0, st>>>(p);
+  glp::work_chains_kernel<><<<(unsigned)chain_blocks(samples), glp::kChainThreads,
+                              glp::kChainSmem, st>>>(p);
+  glp::work_sample_kernel<><<<(unsigned)(samples * glp::sample_parts(p.wn)), glp::kWorkThreads, 0,
+                              st>>>(p);
 }
-void launch_work(const glp::MultiParams &mp, uint64_t samples, cudaStream_t st) {
-  glp::work_chains_multi_kernel<><<<(unsigned)((samples + glp::kPairRows - 1) / glp::kPairRows),
-                                    glp::kChainThreads, glp::kChainSmem, st>>>(mp);
-  glp::work_sample_multi_kernel<><<<(unsigned)samples, 32, 0, st>>>(mp);
+
+// Grids of a batch's hmm_work kernels (0: no chunk runs it).
+struct WorkGrids {
+  unsigned chains = 0, samples = 0;
+};
+void launch_work(const glp::MultiParams &mp, WorkGrids g, cudaStream_t st) {
+  if (!g.chains)
+    return;
+  glp::work_chains_multi_kernel<><<<g.chains, glp::kChainThreads, glp::kChainSmem, st>>>(mp);
+  glp::work_sample_multi_kernel<><<<g.samples, glp::kWorkThreads, 0, st>>>(mp);
+}
+
+// The device tables of a batch (glp::MultiParams) into out[batch_words(count)].
+WorkGrids batch_tables(const glp::GenParams *chunks, uint32_t count, uint32_t *out) {
+  uint32_t *offsets = out, *order = out + count + 1, *blocks = order + count,
+           *warps = blocks + count + 1;
+  uint32_t total = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    offsets[i] = total;
+    total += chunks[i].N;
+    order[i] = i;
+  }
+  offsets[count] = total;
+  std::stable_sort(order, order + count,
+                   [&](uint32_t a, uint32_t b) { return chunks[a].S > chunks[b].S; });
+  WorkGrids g;
+  for (uint32_t i = 0; i < count; ++i) {
+    const glp::GenParams &p = chunks[order[i]];
+    blocks[i] = g.chains;
+    warps[i] = g.samples;
+    if (p.do_work) {
+      g.chains += (unsigned)chain_blocks(p.N);
+      g.samples += p.N * glp::sample_parts(p.wn);
+    }
+  }
+  blocks[count] = g.chains;
+  warps[count] = g.samples;
+  return g;
 }
 
 // Threads of the generation kernel with P lanes per sample that the GPU keeps
@@ -864,13 +900,13 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     c->h_offsets = nullptr;
     c->h_cap = 0;
     GLP_CUDA(c, cudaMallocHost((void **)&c->h_table, sizeof(glp::GenParams) * count));
-    GLP_CUDA(c, cudaMallocHost((void **)&c->h_offsets, sizeof(uint32_t) * (count + 1)));
+    GLP_CUDA(c, cudaMallocHost((void **)&c->h_offsets,
+                               sizeof(uint32_t) * glp::batch_words(count)));
     c->h_cap = count;
   }
   // the staging buffers are reused: wait for the previous batch's upload
   GLP_CUDA(c, cudaStreamSynchronize(c->stream));
   uint64_t total = 0, chain_cycles = 0;
-  c->h_offsets[0] = 0;
   for (uint32_t i = 0; i < count; ++i) {
     glp_problem *pb = problems[i];
     if (!pb || pb->ctx != c)
@@ -883,14 +919,15 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     chain_cycles += (uint64_t)args[i].num_samples * args[i].num_cycles;
     if (total > 0xffffffffull)
       return fail(c, GLP_ERR_ARG, "a batch holds at most 2^32-1 samples");
-    c->h_offsets[i + 1] = (uint32_t)total;
   }
+  const WorkGrids work = batch_tables(c->h_table, count, c->h_offsets);
   if ((rc = ensure(c, c->d_table, c->table_cap, count)) ||
-      (rc = ensure(c, c->d_offsets, c->offsets_cap, (size_t)count + 1)))
+      (rc = ensure(c, c->d_offsets, c->offsets_cap, glp::batch_words(count))))
     return rc;
   GLP_CUDA(c, cudaMemcpyAsync(c->d_table, c->h_table, sizeof(glp::GenParams) * count,
                               cudaMemcpyHostToDevice, c->stream));
-  GLP_CUDA(c, cudaMemcpyAsync(c->d_offsets, c->h_offsets, sizeof(uint32_t) * (count + 1),
+  GLP_CUDA(c, cudaMemcpyAsync(c->d_offsets, c->h_offsets,
+                              sizeof(uint32_t) * glp::batch_words(count),
                               cudaMemcpyHostToDevice, c->stream));
   glp::MultiParams mp;
   mp.chunks = c->d_table;
@@ -912,7 +949,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   fn<<<grid, glp::kThreads, glp::stage_bytes((int)P), c->stream>>>(mp);
   GLP_CUDA(c, cudaGetLastError());
   GLP_CUDA(c, cudaEventRecord(ev[1], c->stream));
-  launch_work(mp, total, c->stream);
+  launch_work(mp, work, c->stream);
   GLP_CUDA(c, cudaEventRecord(ev[2], c->stream));
   GLP_CUDA(c, cudaGetLastError());
   c->lanes_used = P;
@@ -925,7 +962,8 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
 struct glp_batch {
   glp_ctx *c = nullptr;
   uint32_t count = 0;
-  uint64_t total = 0, chain_cycles = 0;
+  uint64_t chain_cycles = 0;
+  WorkGrids work;
   uint32_t P = 8;
   unsigned grid = 1;
   glp::GenParams *d_table = nullptr;
@@ -944,7 +982,7 @@ int batch_enqueue(glp_batch *b, cudaStream_t st) {
   GLP_CUDA(c, cudaMemsetAsync(c->d_stats, 0, glp::kStats * sizeof(unsigned long long), st));
   b->fn<<<b->grid, glp::kThreads, glp::stage_bytes((int)b->P), st>>>(b->mp);
   GLP_CUDA(c, cudaGetLastError());
-  launch_work(b->mp, b->total, st);
+  launch_work(b->mp, b->work, st);
   GLP_CUDA(c, cudaGetLastError());
   glp::advance_kernel<<<(b->count + 127) / 128, 128, 0, st>>>(b->d_table, b->count);
   GLP_CUDA(c, cudaGetLastError());
@@ -981,7 +1019,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   *out = nullptr;
   const bool vq = (args[0].flags & GLP_GEN_VQ) != 0;
   std::vector<glp::GenParams> table(count);
-  std::vector<uint32_t> offsets(count + 1, 0);
+  std::vector<uint32_t> offsets(glp::batch_words(count), 0);
   uint64_t total = 0, chain_cycles = 0;
   for (uint32_t i = 0; i < count; ++i) {
     glp_problem *pb = problems[i];
@@ -999,12 +1037,11 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     chain_cycles += (uint64_t)args[i].num_samples * args[i].num_cycles;
     if (total > 0xffffffffull)
       return fail(c, GLP_ERR_ARG, "a batch holds at most 2^32-1 samples");
-    offsets[i + 1] = (uint32_t)total;
   }
   glp_batch *b = new glp_batch();
   b->c = c;
   b->count = count;
-  b->total = total;
+  b->work = batch_tables(table.data(), count, offsets.data());
   b->chain_cycles = chain_cycles;
   cudaStream_t cs = nullptr;
   auto bail = [&](int code) {
@@ -1014,11 +1051,11 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     return code;
   };
   if (cudaMalloc((void **)&b->d_table, sizeof(glp::GenParams) * count) != cudaSuccess ||
-      cudaMalloc((void **)&b->d_offsets, sizeof(uint32_t) * (count + 1)) != cudaSuccess)
+      cudaMalloc((void **)&b->d_offsets, sizeof(uint32_t) * offsets.size()) != cudaSuccess)
     return bail(fail(c, GLP_ERR_NOMEM, "batch descriptor allocation failed"));
   if (cudaMemcpy(b->d_table, table.data(), sizeof(glp::GenParams) * count,
                  cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b->d_offsets, offsets.data(), sizeof(uint32_t) * (count + 1),
+      cudaMemcpy(b->d_offsets, offsets.data(), sizeof(uint32_t) * offsets.size(),
                  cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(c, GLP_ERR_CUDA, "batch descriptor upload failed"));
   b->mp.chunks = b->d_table;

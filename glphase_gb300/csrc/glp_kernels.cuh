@@ -634,11 +634,6 @@ __device__ __forceinline__ double eval_pair(const GenParams &p, const E &em, uin
 // (impute.cpp:380-485): explicit _rn intrinsics keep nvcc from contracting
 // products and sums into FMAs, so results are bit-identical to the CPU code.
 
-__device__ __forceinline__ float pick(const float4 e, uint32_t i) {
-  return (i & 2u) ? ((i & 1u) ? e.w : e.z) : ((i & 1u) ? e.y : e.x);
-}
-
-
 __device__ __forceinline__ float fma3_rn(float a0, float b0, float a1, float b1, float a2,
                                          float b2, float a3, float b3) {
   // ((a0*b0 + a1*b1) + a2*b2) + a3*b3, every product and sum rounded.
@@ -647,460 +642,320 @@ __device__ __forceinline__ float fma3_rn(float a0, float b0, float a1, float b1,
                    __fmul_rn(a3, b3));
 }
 
-// The reference's normalisation factor 1.0f / sum (impute.cpp:404, 441): the
-// correctly rounded reciprocal, which is what __frcp_rn returns for every
-// input, with a shorter dependency chain than the general division.
-__device__ __forceinline__ float recip_rn(float x) { return __frcp_rn(x); }
-
 // hmm_work is split in two passes with the reference's arithmetic unchanged.
 // The forward state l_m of impute.cpp:416-447 does not depend on the sampled
 // bits, so (1) the two sequential recursions -- the backward vectors beta_m
 // (impute.cpp:389-414) and the forward l_m -- run per sample and leave
-// p_m = l_m * beta_m (the products of impute.cpp:449-452) in the scratch:
-// work_chains_pair runs them at the same time on two warps (a lane pair per
-// recursion), work_chains one after the other on one thread (chunks mixed
-// within a warp); (2) the
-// sampling of impute.cpp:453-484 then runs for every site in parallel, one
-// warp per part of a sample and 32 sites per instruction.
-
-__device__ __forceinline__ uint32_t clamp_site(int m, uint32_t S) {
-  return m < 0 ? 0u : ((uint32_t)m >= S ? S - 1 : (uint32_t)m);
-}
-
-// Rows of one 4-site step of pass 1: emission and transition rows (and, in
-// the forward recursion, the backward vectors).  Steps are aligned to
-// multiples of 4 sites, so a step never straddles a parent word; indices
-// outside [0, S) are clamped (the rows loaded there are never used).
-struct WorkRows {
-  float4 e[4], t[4];
-};
-struct WorkRowsB {
-  float4 e[4], t[4], b[4];
-};
-
-__device__ __forceinline__ void load_rows(WorkRows &r, const float4 *e, const float4 *tr,
-                                          int m0, uint32_t S) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t m = clamp_site(m0 + j, S);
-    r.e[j] = __ldg(e + m);
-    r.t[j] = __ldg(tr + m);
-  }
-}
-
-__device__ __forceinline__ void load_rows(WorkRowsB &r, const float4 *e, const float4 *tr,
-                                          const float4 *beta, int m0, uint32_t S) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t m = clamp_site(m0 + j, S);
-    r.e[j] = __ldg(e + m);
-    r.t[j] = __ldg(tr + m);
-    r.b[j] = beta[m];
-  }
-}
-
-// Pass 1 of hmm_work for sample s with final quadruple q: beta_m for
-// m = S-1 .. 0, then l_m for m = 0 .. S-1, leaving p_m = l_m * beta_m in
-// p.beta[s][m].  The next 4-site step's rows are loaded before the current
-// step is computed.
-__device__ __forceinline__ void work_chains(const GenParams &p, uint32_t s, uint4 q) {
-  const uint32_t S = p.S, wn = p.wn;
-  const uint64_t *f0 = p.haps + (size_t)q.x * wn, *f1 = p.haps + (size_t)q.y * wn,
-                 *m0 = p.haps + (size_t)q.z * wn, *m1 = p.haps + (size_t)q.w * wn;
-  const float4 *e = p.emit + (size_t)s * S;
-  const float4 *tr = p.tran4;
-  float4 *beta = p.beta + (size_t)s * S;
-  // backward recursion (impute.cpp:389-414): sites S-1 .. 1
-  {
-    float b0 = 1.f, b1 = 1.f, b2 = 1.f, b3 = 1.f;
-    beta[S - 1] = make_float4(1.f, 1.f, 1.f, 1.f);
-    const int top = (int)((S - 1) & ~3u);
-    WorkRows cur, nxt;
-    load_rows(cur, e, tr, top, S);
-    for (int c0 = top; c0 >= 0; c0 -= 4) {
-      // emission sites [c0 - 96, c0 - 64) into L2, two 32-site blocks ahead
-      if ((c0 & 31) == 0 && c0 >= 96)
-        prefetch_l2_bulk(e + (c0 - 96), 32 * sizeof(float4));
-      load_rows(nxt, e, tr, c0 - 4, S);
-      const uint32_t w = (uint32_t)c0 >> 6;
-      const uint64_t A0 = __ldg(f0 + w), A1 = __ldg(f1 + w), C0 = __ldg(m0 + w),
-                     C1 = __ldg(m1 + w);
-#pragma unroll
-      for (int j = 3; j >= 0; --j) {
-        const int m = c0 + j;
-        if (m >= 1 && m <= (int)S - 1) {
-          const uint32_t sh = (uint32_t)m & 63u;
-          const uint32_t a0 = (uint32_t)(A0 >> sh) & 1u, a1 = (uint32_t)(A1 >> sh) & 1u,
-                         c0b = (uint32_t)(C0 >> sh) & 1u, c1b = (uint32_t)(C1 >> sh) & 1u;
-          const float4 em = cur.e[j], t = cur.t[j];
-          const float b00 = __fmul_rn(b0, pick(em, (a0 << 1) | c0b));
-          const float b01 = __fmul_rn(b1, pick(em, (a0 << 1) | c1b));
-          const float b10 = __fmul_rn(b2, pick(em, (a1 << 1) | c0b));
-          const float b11 = __fmul_rn(b3, pick(em, (a1 << 1) | c1b));
-          b0 = __fadd_rn(__fadd_rn(__fmul_rn(b00, t.x), __fmul_rn(__fadd_rn(b01, b10), t.y)),
-                         __fmul_rn(b11, t.z));
-          b1 = __fadd_rn(__fadd_rn(__fmul_rn(b01, t.x), __fmul_rn(__fadd_rn(b00, b11), t.y)),
-                         __fmul_rn(b10, t.z));
-          b2 = __fadd_rn(__fadd_rn(__fmul_rn(b10, t.x), __fmul_rn(__fadd_rn(b00, b11), t.y)),
-                         __fmul_rn(b01, t.z));
-          b3 = __fadd_rn(__fadd_rn(__fmul_rn(b11, t.x), __fmul_rn(__fadd_rn(b01, b10), t.y)),
-                         __fmul_rn(b00, t.z));
-          const float sum = __fdiv_rn(1.0f, __fadd_rn(__fadd_rn(__fadd_rn(b0, b1), b2), b3));
-          b0 = __fmul_rn(b0, sum);
-          b1 = __fmul_rn(b1, sum);
-          b2 = __fmul_rn(b2, sum);
-          b3 = __fmul_rn(b3, sum);
-          beta[m - 1] = make_float4(b0, b1, b2, b3);
-        }
-      }
-      cur = nxt;
-    }
-  }
-  // forward recursion (impute.cpp:416-452): sites 0 .. S-1, p_m = l_m * beta_m
-  float l00 = 0, l01 = 0, l10 = 0, l11 = 0;
-  WorkRowsB cur, nxt;
-  load_rows(cur, e, tr, beta, 0, S);
-  for (uint32_t c0 = 0; c0 < S; c0 += 4) {
-    // emission and backward sites [c0 + 64, c0 + 96) into L2, two blocks ahead
-    if ((c0 & 31u) == 0 && c0 + 96 <= S) {
-      prefetch_l2_bulk(e + c0 + 64, 32 * sizeof(float4));
-      prefetch_l2_bulk(beta + c0 + 64, 32 * sizeof(float4));
-    }
-    load_rows(nxt, e, tr, beta, (int)c0 + 4, S);
-    const uint32_t w = c0 >> 6;
-    const uint64_t A0 = __ldg(f0 + w), A1 = __ldg(f1 + w), C0 = __ldg(m0 + w),
-                   C1 = __ldg(m1 + w);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t m = c0 + (uint32_t)j;
-      if (m < S) {
-        const uint32_t sh = m & 63u;
-        const uint32_t a0 = (uint32_t)(A0 >> sh) & 1u, a1 = (uint32_t)(A1 >> sh) & 1u,
-                       c0b = (uint32_t)(C0 >> sh) & 1u, c1b = (uint32_t)(C1 >> sh) & 1u;
-        const uint32_t s00 = (a0 << 1) | c0b, s01 = (a0 << 1) | c1b, s10 = (a1 << 1) | c0b,
-                       s11 = (a1 << 1) | c1b;
-        const float4 em = cur.e[j], t = cur.t[j], bb = cur.b[j];
-        if (m) {
-          const float b00 = fma3_rn(l00, t.x, l01, t.y, l10, t.y, l11, t.z);
-          const float b01 = fma3_rn(l00, t.y, l01, t.x, l10, t.z, l11, t.y);
-          const float b10 = fma3_rn(l00, t.y, l01, t.z, l10, t.x, l11, t.y);
-          const float b11 = fma3_rn(l00, t.z, l01, t.y, l10, t.y, l11, t.x);
-          l00 = __fmul_rn(b00, pick(em, s00));
-          l01 = __fmul_rn(b01, pick(em, s01));
-          l10 = __fmul_rn(b10, pick(em, s10));
-          l11 = __fmul_rn(b11, pick(em, s11));
-        } else {
-          l00 = __fmul_rn(0.25f, pick(em, s00));
-          l01 = __fmul_rn(0.25f, pick(em, s01));
-          l10 = __fmul_rn(0.25f, pick(em, s10));
-          l11 = __fmul_rn(0.25f, pick(em, s11));
-        }
-        const float sum = __fdiv_rn(1.0f, __fadd_rn(__fadd_rn(__fadd_rn(l00, l01), l10), l11));
-        l00 = __fmul_rn(l00, sum);
-        l01 = __fmul_rn(l01, sum);
-        l10 = __fmul_rn(l10, sum);
-        l11 = __fmul_rn(l11, sum);
-        beta[m] = make_float4(__fmul_rn(l00, bb.x), __fmul_rn(l01, bb.y), __fmul_rn(l10, bb.z),
-                              __fmul_rn(l11, bb.w));
-      }
-    }
-    cur = nxt;
-  }
-}
-
-// Staging of pass 1 for the 16 samples of a warp that share one chunk (two
-// lanes a sample): each 16-site tile of the 16 per-sample rows (emission,
-// and stored vectors) is copied into shared memory by the whole warp, one
-// 256-byte row segment per half-warp instruction (cp.async, one tile in
-// flight ahead), so every lane then reads its sample's row from shared
-// memory.
-constexpr int kTile = 16;
-constexpr int kTileStrideF4 = kTile + 1;  // odd number of 16-byte units: no bank conflicts
-constexpr int kPairRows = 16;             // samples per warp of pass 1
-
-struct ChainTiles {
-  float4 e[2][kPairRows * kTileStrideF4];
-  float4 b[2][kPairRows * kTileStrideF4];
-  float4 t[2][kTile];
-  const float4 *erow[kPairRows];
-  float4 *brow[kPairRows];
-};
-
-// Copy sites [base, base + kTile) of every row (rows with a null pointer are
-// skipped); indices are clamped to [0, S).
-__device__ __forceinline__ void stage_tile(float4 *dst, const float4 *const *rows, int base,
-                                           uint32_t S, uint32_t lane) {
-  const uint32_t half = lane >> 4, j = lane & 15u;
-  const uint32_t m = clamp_site(base + (int)j, S);
-#pragma unroll
-  for (uint32_t r = 0; r < (uint32_t)kPairRows; r += 2) {
-    const float4 *row = rows[r + half];
-    if (row)
-      cp_async16(dst + (r + half) * kTileStrideF4 + j, row + m);
-  }
-}
-
-// The emission e[(abit << 1) | cbit] of impute.cpp:338-342 for bit j of the
-// father word a and the mother word c.
-__device__ __forceinline__ float pick_bits(const float4 e, uint32_t a, uint32_t c, int j) {
-  const bool ab = (a >> j) & 1u, cb = (c >> j) & 1u;
-  return ab ? (cb ? e.w : e.z) : (cb ? e.y : e.x);
-}
-
-// Pass 1 on lane pairs.  A generation has only 2N recursions of S
-// sequential steps, so one lane a recursion leaves about one warp a
-// scheduler, which then waits on each step's latency; here two lanes share a
-// recursion, which doubles the warps.  Lane role 0 owns the states 00 and
-// 11, role 1 the states 01 and 10: each lane computes the reference's
-// formula for its own two states (impute.cpp:389-414 backward, 416-447
-// forward) in the reference's binary32 operation order, one shuffle hands
-// the pair the other two, and both lanes form the normalising sum in the
-// reference's order, so both hold the same, bit-identical vector.
+// p_m = l_m * beta_m (the products of impute.cpp:449-452) in the scratch;
+// (2) the sampling of impute.cpp:453-484 then runs for every site in parallel,
+// one warp per part of a sample and 32 sites per instruction.
 //
-// The backward state is kept relative to the lane: (o1, o2) its own states,
-// (p1, p2) the partner's -- role 0: (b0, b3, b1, b2), role 1: (b1, b2, b0,
-// b3).  With the mother words of role 1 swapped (cf, cs), own state k picks
-// its emission from (father word k, cf) for k = 1 and (father word 2, cs)
-// for k = 2, and the partner's from the opposite mother word.
-struct PairBwd {
-  float o1, o2, p1, p2;
-  __device__ __forceinline__ void step(float e_o1, float e_o2, float e_p1, float e_p2,
-                                       const float4 t, bool r0) {
-    const float xo1 = __fmul_rn(o1, e_o1), xo2 = __fmul_rn(o2, e_o2);
-    const float pair = __fadd_rn(__fmul_rn(p1, e_p1), __fmul_rn(p2, e_p2));
-    const float py = __fmul_rn(pair, t.y);
-    const float A = __fadd_rn(__fadd_rn(__fmul_rn(xo1, t.x), py), __fmul_rn(xo2, t.z));
-    const float B = __fadd_rn(__fadd_rn(__fmul_rn(xo2, t.x), py), __fmul_rn(xo1, t.z));
-    const float pA = __shfl_xor_sync(0xffffffffu, A, 1), pB = __shfl_xor_sync(0xffffffffu, B, 1);
-    // ((b0 + b1) + b2) + b3: role 0 holds b0 = A, b3 = B; role 1 b1 = A, b2 = B
-    const float sum = __fadd_rn(__fadd_rn(__fadd_rn(A, pA), r0 ? pB : B), r0 ? B : pB);
-    const float inv = recip_rn(sum);
-    o1 = __fmul_rn(A, inv);
-    o2 = __fmul_rn(B, inv);
-    p1 = __fmul_rn(pA, inv);
-    p2 = __fmul_rn(pB, inv);
-  }
-  // (b0, b1, b2, b3) for role 0
-  __device__ __forceinline__ float4 vec() const { return make_float4(o1, p1, p2, o2); }
+// Pass 1: a block of two warps takes 32 samples of one chunk, one lane a
+// sample.  Warp 0 runs the backward recursion from the top site, warp 1 the
+// forward recursion from site 0, at the same time.  Neither depends on the other
+// until p, so each runs to the middle storing its vectors; after a block barrier
+// each goes on through the other half, where it multiplies its vectors with the
+// stored ones.
+//
+// What bounds it: with a recursion warp a scheduler or less, the instructions
+// that a step issues, each about two cycles apart (a step's dependent chain, 16
+// instructions and a reciprocal, is shorter); with more, the 80 bytes a site and
+// sample that it moves (at 10,000 samples 4.2 TB/s).  So the four states sit in
+// one lane as two register pairs (shared between two lanes, every step waits for
+// a shuffle) whose products are packed binary32 instructions, the reciprocal is a
+// Newton step without a range test, and rows come (cp.async) and vectors go a
+// tile of 8 sites at a time, 8 lanes a row.  Pass 1 before (a lane pair a
+// recursion, blocks of 16 samples) and now: 256 x 1,024 0.156 and 0.099 ms, 2,000
+// x 8,192 1.19 and 0.81, 10,000 x 4,096 1.16 and 0.80.  Measured and not kept:
+// warps that pick the emissions and store the vectors beside each recursion warp
+// (0.084 ms at 256 x 1,024, but 1.02 at 10,000 x 4,096: a barrier a tile couples
+// them to the slowest), and the vectors of a half recomputed from states at the
+// tiles' starts with the sampling in the same kernel (48 bytes a site instead of
+// 108 for both passes, but ten warps in step: 0.127 against 0.117 ms for both
+// passes and 1.2 against 1.05).
+constexpr int kChainTile = 8;           // sites
+constexpr int kChainRing = 4;           // tiles: one read, one next, two in flight
+constexpr uint32_t kChainSamples = 32;  // samples per block
+// A tile in shared memory keeps a sample's sites together, as in global memory
+// (a copy of 8 lanes lands as one 128-byte write; sites apart, it took eight),
+// rows 9 float4 apart: 1 mod 8, so that 8 samples' reads of a site fall in 8 quads.
+constexpr uint32_t kRowF4 = kChainTile + 1;
+constexpr uint32_t kTileF4 = kChainSamples * kRowF4;
+constexpr int kChainThreads = 64;
+
+// A vector over the four states, as the pairs (00, 01) and (11, 10): packed
+// binary32 products then round each component as the scalar ones do.
+struct States {
+  float2 P, Q;
+};
+__device__ __forceinline__ States states_of(const float4 v) {
+  return States{make_float2(v.x, v.y), make_float2(v.z, v.w)};
+}
+__device__ __forceinline__ float4 f4_of(const States v) {
+  return make_float4(v.P.x, v.P.y, v.Q.x, v.Q.y);
+}
+__device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
+// The sums of two pairs as scalar additions: a packed addition of a packed
+// product is contracted to a fused multiply-add, which rounds once.
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+  return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+
+struct ChainTiles {  // of one recursion
+  float4 e[kChainRing][kTileF4];  // emission rows
+  float4 v[kChainRing][kTileF4];  // vectors: the stored ones in, the new ones out
+  float4 t[kChainRing][kChainTile];  // transition rows
 };
 
-// The forward state is the reference's (l00, l01, l10, l11) in both lanes.
-// Role 0 computes c00 and c11, role 1 c01 and c10 (the coefficient rows of
-// T for those states), each times its own emission.
-struct PairFwd {
-  float l00, l01, l10, l11;
-  __device__ __forceinline__ void finish(float A, float B, bool r0) {
-    const float pA = __shfl_xor_sync(0xffffffffu, A, 1), pB = __shfl_xor_sync(0xffffffffu, B, 1);
-    const float n00 = r0 ? A : pA, n01 = r0 ? pA : A, n10 = r0 ? pB : B, n11 = r0 ? B : pB;
-    const float inv = recip_rn(__fadd_rn(__fadd_rn(__fadd_rn(n00, n01), n10), n11));
-    l00 = __fmul_rn(n00, inv);
-    l01 = __fmul_rn(n01, inv);
-    l10 = __fmul_rn(n10, inv);
-    l11 = __fmul_rn(n11, inv);
-  }
-  __device__ __forceinline__ void step(float e_o1, float e_o2, const float4 t, bool r0) {
-    // role 0: c00 (x, y, y, z), c11 (z, y, y, x); role 1: c01 (y, x, z, y), c10 (y, z, x, y)
-    const float cA = fma3_rn(l00, r0 ? t.x : t.y, l01, r0 ? t.y : t.x, l10, r0 ? t.y : t.z, l11,
-                             r0 ? t.z : t.y);
-    const float cB = fma3_rn(l00, r0 ? t.z : t.y, l01, r0 ? t.y : t.z, l10, r0 ? t.y : t.x, l11,
-                             r0 ? t.x : t.y);
-    finish(__fmul_rn(cA, e_o1), __fmul_rn(cB, e_o2), r0);
-  }
-  __device__ __forceinline__ void first(float e_o1, float e_o2, bool r0) {
-    finish(__fmul_rn(0.25f, e_o1), __fmul_rn(0.25f, e_o2), r0);
-  }
-  __device__ __forceinline__ float4 vec() const { return make_float4(l00, l01, l10, l11); }
-};
+// 1.0f / x correctly rounded, for x in [2^-126, 2^126): one Newton step from
+// the approximate reciprocal.  Equal to __frcp_rn for every float of that
+// range (checked exhaustively), without its range test and branch in the
+// dependent chain.  Outside it: NaN below, 0 above.
+__device__ __forceinline__ float recip_newton(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
 
-// Pass 1 split over two warps that share the same 16 samples (two lanes per
-// sample in each): warp 0 runs the backward recursion from the top site and
-// warp 1 the forward recursion from site 0, at the same time.  Neither
-// depends on the other until p_m = l_m * beta_m, so each runs to the middle
-// site mid storing its vectors -- beta_{m-1} for m >= mid (backward; index
-// mid-1 upwards) and l_m for m <= mid-2 (forward; l_{mid-1} stays in
-// registers) -- then, after a block barrier, each continues through the other
-// half reading what the other stored and writing p there: the backward warp
-// p_m for m <= mid-2 (beta_m fresh, l_m stored), the forward warp p_{mid-1}
-// and p_m for m >= mid (l_m fresh, beta_m stored).  The operations on every
-// vector are those of work_chains, so p is bit-identical.  Role-0 lanes store
-// the vectors.  Both warps call this together, every lane (lanes of samples
-// past the end compute on whatever their rows hold and store nothing).
-__device__ __forceinline__ void work_chains_pair(const GenParams &p, uint32_t s, uint4 q,
-                                                 bool valid, uint32_t lane, bool fwd,
-                                                 ChainTiles &sm) {
-  const uint32_t S = p.S, wn = p.wn;
-  const float4 *tr = p.tran4;
-  const bool r0 = (lane & 1u) == 0;
-  const bool writer = valid && r0;
-  const uint32_t row = lane >> 1;
-  const uint64_t *f0 = p.haps + (size_t)q.x * wn, *f1 = p.haps + (size_t)q.y * wn,
-                 *m0 = p.haps + (size_t)q.z * wn, *m1 = p.haps + (size_t)q.w * wn;
-  // role 1 owns 01 and 10: its first own state takes the second mother word
-  const uint64_t *mf = r0 ? m0 : m1, *ms = r0 ? m1 : m0;
-  float4 *beta = p.beta + (size_t)s * S;
-  if (r0) {
-    sm.erow[row] = valid ? p.emit + (size_t)s * S : nullptr;
-    sm.brow[row] = valid ? beta : nullptr;
-  }
-  if (!fwd && writer)
-    beta[S - 1] = make_float4(1.f, 1.f, 1.f, 1.f);
-  __syncwarp();
-  const int ntiles = (int)((S + kTile - 1) / kTile);
-  const int top = (int)((S - 1) & ~(uint32_t)(kTile - 1));
-  const int mid = kTile * (ntiles / 2);            // first site of the upper half
-  const int n_hi = (top - mid) / kTile + 1;        // tiles [mid, S)
-  const int n_lo = mid / kTile;                    // tiles [0, mid)
-  const float4 *const *erows = sm.erow;
-  const float4 *const *brows = sm.brow;
-  // emission rows of the tile at base, stored vectors from bbase (with_b)
-  auto stage = [&](int buf, int base, bool with_b, int bbase) {
-    stage_tile(sm.e[buf], erows, base, S, lane);
-    if (with_b)
-      stage_tile(sm.b[buf], brows, bbase, S, lane);
-    if (lane < kTile)
-      cp_async16(&sm.t[buf][lane], tr + clamp_site(base + (int)lane, S));
+// The normalisation of a step (impute.cpp:404-409, 441-446): the sum in the
+// reference's order, its reciprocal (kSafe: the division for any sum) and the
+// four products.  seen turns NaN with the reciprocal.
+template <bool kSafe>
+__device__ __forceinline__ States work_normalise(const States n, float &seen) {
+  const float sum = __fadd_rn(__fadd_rn(__fadd_rn(n.P.x, n.P.y), n.Q.y), n.Q.x);
+  const float inv = kSafe ? __frcp_rn(sum) : recip_newton(sum);
+  seen = fmaf(inv, 0.0f, seen);
+  return States{__fmul2_rn(n.P, dup2(inv)), __fmul2_rn(n.Q, dup2(inv))};
+}
+
+// One step of the backward recursion from beta_m to beta_{m-1}
+// (impute.cpp:389-414): emissions s and transition row t of site m.
+template <bool kSafe>
+__device__ __forceinline__ States work_bwd_step(const States v, const States s, const float4 t,
+                                                float &seen) {
+  const float2 P = __fmul2_rn(v.P, s.P), Q = __fmul2_rn(v.Q, s.Q);
+  // (b01 + b10, b00 + b11) y
+  const float2 c = __fmul2_rn(make_float2(__fadd_rn(P.y, Q.y), __fadd_rn(P.x, Q.x)),
+                              dup2(t.y));
+  const float2 x = dup2(t.x), z = dup2(t.z);
+  return work_normalise<kSafe>(
+      States{add_pair(add_pair(__fmul2_rn(P, x), c), __fmul2_rn(Q, z)),
+             add_pair(add_pair(__fmul2_rn(Q, x), c), __fmul2_rn(P, z))},
+      seen);
+}
+
+// One step of the forward recursion from l_{m-1} to l_m (impute.cpp:416-447):
+// emissions s and transition row t of site m.  Site 0's row is the identity, so
+// from the uniform 1/4 its step is the reference's first one, l = e / 4.
+template <bool kSafe>
+__device__ __forceinline__ States work_fwd_step(const States v, const States s, const float4 t,
+                                                float &seen) {
+  const float2 xy = make_float2(t.x, t.y), yx = make_float2(t.y, t.x), yz = make_float2(t.y, t.z),
+               zy = make_float2(t.z, t.y);
+  const float2 l00 = dup2(v.P.x), l01 = dup2(v.P.y), l10 = dup2(v.Q.y), l11 = dup2(v.Q.x);
+  // ((l00 . + l01 .) + l10 .) + l11 . for (00, 01) and for (11, 10)
+  const float2 P = add_pair(add_pair(add_pair(__fmul2_rn(l00, xy), __fmul2_rn(l01, yx)),
+                                         __fmul2_rn(l10, yz)),
+                              __fmul2_rn(l11, zy));
+  const float2 Q = add_pair(add_pair(add_pair(__fmul2_rn(l00, zy), __fmul2_rn(l01, yz)),
+                                         __fmul2_rn(l10, yx)),
+                              __fmul2_rn(l11, xy));
+  return work_normalise<kSafe>(States{__fmul2_rn(P, s.P), __fmul2_rn(Q, s.Q)}, seen);
+}
+
+__device__ __forceinline__ States mul_states(const States a, const States b) {
+  return States{__fmul2_rn(a.P, b.P), __fmul2_rn(a.Q, b.Q)};
+}
+
+// The emissions of a site for the parents' bits a0, a1 (father), c0, c1 (mother).
+__device__ __forceinline__ States pick_states(const float4 e, bool a0, bool a1, bool c0, bool c1) {
+  States s;
+  select4(e, a0, a1, c0, c1, s.P.x, s.P.y, s.Q.y, s.Q.x);
+  return s;
+}
+
+__device__ __forceinline__ void cp_async16_cg(void *smem, const void *gmem) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// One recursion over n tiles from state v: ascending from base0 (kFwd) or
+// descending.  kComb: the other recursion's vectors are staged with the
+// emissions and the products p are stored; else the vectors are.  Lane l has
+// sample s0 + l with the final quadruple q (lanes past the chunk's end repeat its
+// last sample and store nothing).
+template <bool kFwd, bool kComb>
+__device__ __forceinline__ void chain_run(const GenParams &p, ChainTiles &sm, uint32_t lane,
+                                          uint32_t s0, uint4 q, States &v, float &seen, int base0,
+                                          int n) {
+  if (n <= 0)
+    return;
+  const uint32_t S = p.S, unit = lane & 7u, r0 = lane >> 3;  // staging: 8 lanes a row
+  const uint32_t last = min(kChainSamples, p.N - s0) - 1;  // rows past it repeat it
+  const float4 *const emit = p.emit + (size_t)s0 * S;
+  float4 *const beta = p.beta + (size_t)s0 * S;
+  auto base_of = [&](int k) { return kFwd ? base0 + kChainTile * k : base0 - kChainTile * k; };
+  auto stage = [&](int k) {
+    if (k < n) {
+      const uint32_t b = (uint32_t)base_of(k), m = min(b + unit, S - 1u);
+      const int slot = k & (kChainRing - 1);
+#pragma unroll
+      for (uint32_t i = 0; i < 8; ++i) {
+        const uint32_t at = (r0 + 4 * i) * kRowF4 + unit;
+        const size_t from = (size_t)min(r0 + 4 * i, last) * S + m;
+        cp_async16_cg(&sm.e[slot][at], emit + from);
+        if (kComb)
+          cp_async16_cg(&sm.v[slot][at], beta + from);
+      }
+      if (lane < (uint32_t)kChainTile)
+        cp_async16(&sm.t[slot][lane], p.tran4 + m);
+    }
     cp_async_commit();
   };
-  PairBwd vb;
-  vb.o1 = vb.o2 = vb.p1 = vb.p2 = 1.f;
-  PairFwd vf;
-  vf.l00 = vf.l01 = vf.l10 = vf.l11 = 0.f;
-  // the four parent words of the current 64-site word, mother words by role
-  uint64_t wa0 = 0, wa1 = 0, wcf = 0, wcs = 0;
-  int wcur = -1;
-  auto words = [&](uint32_t w) {
-    if ((int)w != wcur) {
-      wa0 = __ldg(f0 + w);
-      wa1 = __ldg(f1 + w);
-      wcf = __ldg(mf + w);
-      wcs = __ldg(ms + w);
-      wcur = (int)w;
-    }
+  // the rows of four sites of a tile, in step order
+  struct Rows {
+    float4 e[4], t[4], o[4];
   };
-
-  // backward (impute.cpp:389-414) over n tiles from the tile at first down;
-  // comb: store p_{m-1} = l_{m-1} * beta_{m-1} (l staged one site lower)
-  auto run_bwd = [&](int first, int n, bool comb) {
-    if (n <= 0)
-      return;
-    stage(0, first, comb, first - 1);
-    for (int i = 0; i < n; ++i) {
-      const int base = first - kTile * i, buf = i & 1;
-      if (i + 1 < n)
-        stage(buf ^ 1, base - kTile, comb, base - kTile - 1);
-      else
-        cp_async_commit();
-      words((uint32_t)base >> 6);
-      const uint32_t A0 = (uint32_t)(wa0 >> (base & 63)), A1 = (uint32_t)(wa1 >> (base & 63)),
-                     CF = (uint32_t)(wcf >> (base & 63)), CS = (uint32_t)(wcs >> (base & 63));
-      cp_async_wait<1>();
-      __syncwarp();
-      const float4 *erow = sm.e[buf] + row * kTileStrideF4;
-      const float4 *lrow = sm.b[buf] + row * kTileStrideF4;
-      auto store = [&](int j) {  // beta_{m-1} (or p_{m-1}) for site m = base + j
-        if (!writer)
-          return;
-        const float4 v = vb.vec();
-        if (comb) {
-          const float4 l = lrow[j];
-          beta[base + j - 1] = make_float4(__fmul_rn(l.x, v.x), __fmul_rn(l.y, v.y),
-                                           __fmul_rn(l.z, v.z), __fmul_rn(l.w, v.w));
-        } else {
-          beta[base + j - 1] = v;
-        }
-      };
-      auto one = [&](int j) {
-        const float4 e = erow[j];
-        vb.step(pick_bits(e, A0, CF, j), pick_bits(e, A1, CS, j), pick_bits(e, A0, CS, j),
-                pick_bits(e, A1, CF, j), sm.t[buf][j], r0);
-        store(j);
-      };
-      if (base >= 1 && base + kTile - 1 <= (int)S - 1) {
+  auto load = [&](Rows &r, int k, int half) {
+    const int slot = k & (kChainRing - 1);
 #pragma unroll
-        for (int j = kTile - 1; j >= 0; --j)
-          one(j);
-      } else {
-#pragma unroll 1
-        for (int j = kTile - 1; j >= 0; --j)
-          if (base + j >= 1 && base + j <= (int)S - 1)
-            one(j);
-      }
-      __syncwarp();  // the buffer is refilled next iteration
+    for (int j = 0; j < 4; ++j) {
+      const int i = 4 * half + j, o = kFwd ? i : kChainTile - 1 - i;
+      r.e[j] = sm.e[slot][lane * kRowF4 + o];
+      r.t[j] = sm.t[slot][o];
+      if (kComb)
+        r.o[j] = sm.v[slot][lane * kRowF4 + o];
     }
   };
-
-  // forward (impute.cpp:416-452) over n tiles from the tile at first up;
-  // comb: store p_m = l_m * beta_m (beta staged), else l_m for m <= mid - 2
-  auto run_fwd = [&](int first, int n, bool comb) {
-    if (n <= 0)
-      return;
-    stage(0, first, comb, first);
-    for (int i = 0; i < n; ++i) {
-      const int base = first + kTile * i, buf = i & 1;
-      if (i + 1 < n)
-        stage(buf ^ 1, base + kTile, comb, base + kTile);
-      else
-        cp_async_commit();
-      words((uint32_t)base >> 6);
-      const uint32_t A0 = (uint32_t)(wa0 >> (base & 63)), A1 = (uint32_t)(wa1 >> (base & 63)),
-                     CF = (uint32_t)(wcf >> (base & 63)), CS = (uint32_t)(wcs >> (base & 63));
-      cp_async_wait<1>();
-      __syncwarp();
-      const float4 *erow = sm.e[buf] + row * kTileStrideF4;
-      const float4 *brow = sm.b[buf] + row * kTileStrideF4;
-      auto store = [&](int j) {  // l_m (or p_m) for site m = base + j
-        const int m = base + j;
-        if (!writer)
-          return;
-        const float4 v = vf.vec();
-        if (comb) {
-          const float4 bb = brow[j];
-          beta[m] = make_float4(__fmul_rn(v.x, bb.x), __fmul_rn(v.y, bb.y),
-                                __fmul_rn(v.z, bb.z), __fmul_rn(v.w, bb.w));
-        } else if (m <= mid - 2) {
-          beta[m] = v;
-        }
-      };
-      auto one = [&](int j) {
-        const float4 e = erow[j];
-        const float e1 = pick_bits(e, A0, CF, j), e2 = pick_bits(e, A1, CS, j);
-        if (base + j == 0)
-          vf.first(e1, e2, r0);
-        else
-          vf.step(e1, e2, sm.t[buf][j], r0);
-        store(j);
-      };
-      if (base >= 1 && base + kTile <= (int)S) {
+  int w = base0 >> 6;
+  const int w_end = base_of(n - 1) >> 6, dir = kFwd ? 1 : -1;
+  Parents cur = load_parents(p.haps, p.wn, q, (uint32_t)w), next = cur;
+  if (w != w_end)
+    next = load_parents(p.haps, p.wn, q, (uint32_t)(w + dir));
+  stage(0);
+  stage(1);
+  cp_async_wait<1>();
+  __syncwarp();
+  Rows ra, rb;
+  load(ra, 0, 0);
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    const int slot = k & (kChainRing - 1), base = base_of(k);
+    stage(k + 2);  // the slot's last tile was stored two tiles ago
+    if ((base >> 6) != w) {
+      w = base >> 6;
+      cur = next;
+      if (w != w_end)
+        next = load_parents(p.haps, p.wn, q, (uint32_t)(w + dir));
+    }
+    const int sh = base & 63;
+    const uint32_t A0 = (uint32_t)(cur.f0 >> sh), A1 = (uint32_t)(cur.f1 >> sh),
+                   C0 = (uint32_t)(cur.m0 >> sh), C1 = (uint32_t)(cur.m1 >> sh);
+    float4 *const out = &sm.v[slot][lane * kRowF4];
+    auto step = [&](int o, const float4 e, const float4 t, const float4 other) {
+      const uint32_t bit = 1u << o;
+      const States s = pick_states(e, A0 & bit, A1 & bit, C0 & bit, C1 & bit);
+      if (kFwd)
+        v = work_fwd_step<false>(v, s, t, seen);
+      out[o] = f4_of(kComb ? mul_states(v, states_of(other)) : v);
+      if (!kFwd)
+        v = work_bwd_step<false>(v, s, t, seen);
+    };
+    auto four = [&](const Rows &r, int half) {
 #pragma unroll
-        for (int j = 0; j < kTile; ++j)
-          one(j);
-      } else {
-#pragma unroll 1
-        for (int j = 0; j < kTile; ++j)
-          if (base + j < (int)S)
-            one(j);
+      for (int j = 0; j < 4; ++j) {
+        const int i = 4 * half + j;
+        step(kFwd ? i : kChainTile - 1 - i, r.e[j], r.t[j], r.o[j]);
       }
-      __syncwarp();
+    };
+    const bool whole = base + kChainTile <= (int)S;
+    if (whole) {
+      load(rb, k, 1);
+      four(ra, 0);
     }
-  };
-
-  if (fwd)
-    run_fwd(0, n_lo, false);
-  else
-    run_bwd(top, n_hi, false);
-  // both halves' vectors are stored (block barrier: the two warps)
-  __syncthreads();
-  if (fwd) {
-    if (writer && mid >= 1) {  // p_{mid-1}: l_{mid-1} still in registers
-      const float4 bb = beta[mid - 1];
-      const float4 v = vf.vec();
-      beta[mid - 1] = make_float4(__fmul_rn(v.x, bb.x), __fmul_rn(v.y, bb.y),
-                                  __fmul_rn(v.z, bb.z), __fmul_rn(v.w, bb.w));
+    cp_async_wait<1>();
+    __syncwarp();  // tile k + 1 has arrived
+    if (k + 1 < n)
+      load(ra, k + 1, 0);
+    if (whole) {
+      four(rb, 1);
+    } else {  // the ragged top tile
+#pragma unroll 1
+      for (int j = 0; j < (int)S - base; ++j) {
+        const int o = kFwd ? j : (int)S - base - 1 - j;
+        step(o, sm.e[slot][lane * kRowF4 + o], sm.t[slot][o], out[o]);
+      }
     }
-    run_fwd(mid, n_hi, true);
-  } else {
-    run_bwd(mid - kTile, n_lo, true);
+    __syncwarp();
+    // the tile's vectors leave together
+    if ((uint32_t)base + unit < S) {
+#pragma unroll
+      for (uint32_t i = 0; i < 8; ++i)
+        if (r0 + 4 * i <= last)
+          beta[(size_t)(r0 + 4 * i) * S + (uint32_t)base + unit] =
+              sm.v[slot][(r0 + 4 * i) * kRowF4 + unit];
+    }
   }
+  cp_async_wait<0>();
+  __syncwarp();
+}
+
+// The recursions of 32 samples by one warp, one after the other, with the
+// reference's division: for sums outside the fast reciprocal's range.
+inline __device__ __noinline__ void chains_any_sum(const GenParams &p, uint32_t s, uint4 q,
+                                                   bool valid) {
+  const float4 *e = p.emit + (size_t)s * p.S;
+  float4 *const beta = p.beta + (size_t)s * p.S;
+  float seen = 0.f;
+  auto picked = [&](uint32_t m) {
+    const Parents w = load_parents(p.haps, p.wn, q, m >> 6);
+    const uint32_t j = m & 63u;
+    return pick_states(__ldg(e + m), (w.f0 >> j) & 1, (w.f1 >> j) & 1, (w.m0 >> j) & 1,
+                       (w.m1 >> j) & 1);
+  };
+  States v = States{dup2(1.f), dup2(1.f)};
+  for (int m = (int)p.S - 1; m >= 0; --m) {
+    if (valid)
+      beta[m] = f4_of(v);
+    v = work_bwd_step<true>(v, picked((uint32_t)m), __ldg(p.tran4 + m), seen);
+  }
+  v = States{dup2(0.25f), dup2(0.25f)};
+  for (uint32_t m = 0; m < p.S; ++m) {
+    v = work_fwd_step<true>(v, picked(m), __ldg(p.tran4 + m), seen);
+    if (valid)
+      beta[m] = f4_of(mul_states(v, states_of(beta[m])));
+  }
+}
+
+// A block's samples s0 .. s0 + 31 of one chunk; tiles[0] backward, tiles[1]
+// forward.
+__device__ __forceinline__ void work_chains(const GenParams &p, uint32_t s0, ChainTiles *tiles) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool fwd = threadIdx.x >= 32;
+  const uint32_t s = min(s0 + lane, p.N - 1);
+  const uint4 q = make_uint4(p.quad_out[s], p.quad_out[p.N + s], p.quad_out[2 * (size_t)p.N + s],
+                             p.quad_out[3 * (size_t)p.N + s]);
+  const int n = ((int)p.S + kChainTile - 1) / kChainTile, n_lo = n / 2, n_hi = n - n_lo;
+  float seen = 0.f;
+  States v = fwd ? States{dup2(0.25f), dup2(0.25f)} : States{dup2(1.f), dup2(1.f)};
+  if (fwd)
+    chain_run<true, false>(p, tiles[1], lane, s0, q, v, seen, 0, n_lo);
+  else
+    chain_run<false, false>(p, tiles[0], lane, s0, q, v, seen, kChainTile * (n - 1), n_hi);
+  __syncthreads();  // both halves' vectors are stored
+  if (fwd)
+    chain_run<true, true>(p, tiles[1], lane, s0, q, v, seen, kChainTile * n_lo, n_hi);
+  else
+    chain_run<false, true>(p, tiles[0], lane, s0, q, v, seen, kChainTile * (n_lo - 1), n_lo);
+  // a sum below the fast reciprocal's range left NaN in seen; one above it left
+  // zeros, and with them such a sum (or no unit sum at the end)
+  const bool special = !(seen == 0.f && v.P.x + v.P.y + v.Q.x + v.Q.y > 0.5f);
+  if (__syncthreads_or(special) && !fwd)
+    chains_any_sum(p, s, q, s0 + lane < p.N);
+}
+
+inline __device__ __noinline__ float4 pow4(const float4 c, float pen) {
+  return make_float4(powf(c.x, pen), powf(c.y, pen), powf(c.z, pen), powf(c.w, pen));
 }
 
 // Pass 2 of hmm_work: the sampling of impute.cpp:453-484 for site m of
@@ -1118,34 +973,33 @@ __device__ __forceinline__ uint32_t work_sample_site(const GenParams &p, const f
   const uint32_t sh = m & 63u;
   const uint32_t a0 = (uint32_t)(A0 >> sh) & 1u, a1 = (uint32_t)(A1 >> sh) & 1u,
                  c0b = (uint32_t)(C0 >> sh) & 1u, c1b = (uint32_t)(C1 >> sh) & 1u;
-  const uint32_t s00 = (a0 << 1) | c0b, s01 = (a0 << 1) | c1b, s10 = (a1 << 1) | c0b,
-                 s11 = (a1 << 1) | c1b;
-  const float4 pp = p.beta[(size_t)s * S + m];
+  const States pp = states_of(__ldg(p.beta + (size_t)s * S + m));
   const float *pr = p.prob + ((size_t)s * S + m) * 3;
   const float g0 = __ldg(pr), g1 = __ldg(pr + 1), g2 = __ldg(pr + 2);
-  const float4 r00 = pcr[s00], r01 = pcr[s01], r10 = pcr[s10], r11 = pcr[s11];
-  const float inner0 = fma3_rn(pp.x, r00.x, pp.y, r01.x, pp.z, r10.x, pp.w, r11.x);
-  const float inner1 = fma3_rn(pp.x, r00.y, pp.y, r01.y, pp.z, r10.y, pp.w, r11.y);
-  const float inner2 = fma3_rn(pp.x, r00.z, pp.y, r01.z, pp.z, r10.z, pp.w, r11.z);
-  const float inner3 = fma3_rn(pp.x, r00.w, pp.y, r01.w, pp.z, r10.w, pp.w, r11.w);
-  float c[4] = {__fmul_rn(g0, inner0), __fmul_rn(g1, inner1), __fmul_rn(g1, inner2),
-                __fmul_rn(g2, inner3)};
-  if (p.pen != 1.0f) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      c[k] = powf(c[k], p.pen);
-  }
+  const float4 r00 = pcr[(a0 << 1) | c0b], r01 = pcr[(a0 << 1) | c1b],
+               r10 = pcr[(a1 << 1) | c0b], r11 = pcr[(a1 << 1) | c1b];
+  const float2 p00 = dup2(pp.P.x), p01 = dup2(pp.P.y), p10 = dup2(pp.Q.y), p11 = dup2(pp.Q.x);
+  // ((p00 r00 + p01 r01) + p10 r10) + p11 r11, two columns at a time
+  auto inner = [&](float2 a, float2 b, float2 c, float2 d) {
+    return add_pair(add_pair(add_pair(__fmul2_rn(p00, a), __fmul2_rn(p01, b)),
+                                 __fmul2_rn(p10, c)),
+                      __fmul2_rn(p11, d));
+  };
+  const float2 i01 = inner(make_float2(r00.x, r00.y), make_float2(r01.x, r01.y),
+                           make_float2(r10.x, r10.y), make_float2(r11.x, r11.y));
+  const float2 i23 = inner(make_float2(r00.z, r00.w), make_float2(r01.z, r01.w),
+                           make_float2(r10.z, r10.w), make_float2(r11.z, r11.w));
+  const float2 c01 = __fmul2_rn(make_float2(g0, g1), i01),
+               c23 = __fmul2_rn(make_float2(g1, g2), i23);
+  float4 c = make_float4(c01.x, c01.y, c23.x, c23.y);
+  if (p.pen != 1.0f)
+    c = pow4(c, p.pen);
   const float u = p.tr_work ? __ldg(p.tr_work + (size_t)s * S + m) : glp_u24(u_bits);
-  const float c01 = __fadd_rn(c[0], c[1]);
-  const float c012 = __fadd_rn(c01, c[2]);
-  const float r = __fmul_rn(u, __fadd_rn(c012, c[3]));
-  if (r < c[0])
-    return 0u;  // (0, 0)
-  if (r < c01)
-    return 2u;  // (0, 1)
-  if (r < c012)
-    return 1u;  // (1, 0)
-  return 3u;    // (1, 1)
+  const float s01 = __fadd_rn(c.x, c.y);
+  const float s012 = __fadd_rn(s01, c.z);
+  const float r = __fmul_rn(u, __fadd_rn(s012, c.w));
+  // (0, 0), (0, 1), (1, 0), (1, 1)
+  return r < c.x ? 0u : r < s01 ? 2u : r < s012 ? 1u : 3u;
 }
 
 // Pass 2 for words [w_lo, w_hi) of sample s (called by a whole warp; w_lo
@@ -1209,9 +1063,9 @@ __device__ __forceinline__ void set_slot(uint4 &q, uint32_t r, uint32_t v) {
 // Work sources.  One chunk: the kernel parameter.  Many chunks: a descriptor
 // table in global memory; the samples of all chunks form one queue, chunk by
 // chunk, so a group's neighbours in the queue usually share its chunk.
-// Pass 2 of one chunk splits each sample's words into parts of
-// kSampleWords, one warp a part, so that its warps are many and short and the
-// last of them leave little of the GPU idle (many chunks: one part a sample).
+// Pass 2 splits each sample's words into parts of kSampleWords, one warp a
+// part, so that its warps are many and short and the last of them leave little
+// of the GPU idle.
 #ifndef GLP_SAMPLE_WORDS
 #define GLP_SAMPLE_WORDS 16
 #endif
@@ -1225,17 +1079,38 @@ struct OneChunk {
   static constexpr bool kMulti = false;
   const GenParams &p;
   __device__ __forceinline__ uint32_t total() const { return p.N; }
-  __device__ __forceinline__ uint32_t parts() const { return sample_parts(p.wn); }
   __device__ __forceinline__ const GenParams &chunk(uint32_t) const { return p; }
   __device__ __forceinline__ void locate(uint32_t g, uint32_t &c, uint32_t &s) const {
     c = 0;
     s = g;
   }
+  __device__ __forceinline__ void locate_block(uint32_t b, uint32_t &c, uint32_t &s0) const {
+    c = 0;
+    s0 = b * kChainSamples;
+  }
+  __device__ __forceinline__ void locate_part(uint32_t g, uint32_t &c, uint32_t &s,
+                                              uint32_t &part) const {
+    const uint32_t parts = sample_parts(p.wn);
+    c = 0;
+    s = g / parts;
+    part = g % parts;
+  }
 };
+
+// Device tables of a batch of n chunks, one array of batch_words(n) words:
+//   [0, n]            prefix sums of the chunks' N (the generation kernel's queue)
+//   [n + 1, 2n]       the chunks in order of falling S (hmm_work starts the
+//                     longest recursions first)
+//   [2n + 1, 3n + 1]  in that order, prefix sums of the blocks of hmm_work's
+//                     pass 1 (ceil(N / kChainSamples) each)
+//   [3n + 2, 4n + 2]  in that order, prefix sums of the warps of its pass 2
+//                     (N sample_parts(wn) each)
+// Chunks without hmm_work have no blocks and no warps.
+__host__ __device__ inline size_t batch_words(uint32_t n) { return 4 * (size_t)n + 3; }
 
 struct MultiParams {
   const GenParams *chunks;   // [nchunks]
-  const uint32_t *offsets;   // [nchunks + 1] prefix sums of the chunks' N
+  const uint32_t *offsets;   // the tables above
   uint32_t nchunks;
   uint32_t *counter;
   unsigned long long *stats;
@@ -1246,19 +1121,38 @@ struct ManyChunks {
   static constexpr bool kMulti = true;
   const MultiParams &mp;
   __device__ __forceinline__ uint32_t total() const { return __ldg(mp.offsets + mp.nchunks); }
-  __device__ __forceinline__ uint32_t parts() const { return 1; }
   __device__ __forceinline__ const GenParams &chunk(uint32_t c) const { return mp.chunks[c]; }
-  __device__ __forceinline__ void locate(uint32_t g, uint32_t &c, uint32_t &s) const {
-    uint32_t lo = 0, hi = mp.nchunks;  // largest c with offsets[c] <= g
+  // largest i < nchunks with prefix[i] <= g
+  __device__ __forceinline__ uint32_t find(const uint32_t *prefix, uint32_t g) const {
+    uint32_t lo = 0, hi = mp.nchunks;
     while (hi - lo > 1) {
       const uint32_t mid = (lo + hi) >> 1;
-      if (__ldg(mp.offsets + mid) <= g)
+      if (__ldg(prefix + mid) <= g)
         lo = mid;
       else
         hi = mid;
     }
-    c = lo;
-    s = g - __ldg(mp.offsets + lo);
+    return lo;
+  }
+  __device__ __forceinline__ void locate(uint32_t g, uint32_t &c, uint32_t &s) const {
+    c = find(mp.offsets, g);
+    s = g - __ldg(mp.offsets + c);
+  }
+  __device__ __forceinline__ void locate_block(uint32_t b, uint32_t &c, uint32_t &s0) const {
+    const uint32_t *order = mp.offsets + mp.nchunks + 1, *blocks = order + mp.nchunks;
+    const uint32_t i = find(blocks, b);
+    c = __ldg(order + i);
+    s0 = (b - __ldg(blocks + i)) * kChainSamples;
+  }
+  __device__ __forceinline__ void locate_part(uint32_t g, uint32_t &c, uint32_t &s,
+                                              uint32_t &part) const {
+    const uint32_t *order = mp.offsets + mp.nchunks + 1,
+                   *warps = order + 2 * mp.nchunks + 1;
+    const uint32_t i = find(warps, g);
+    c = __ldg(order + i);
+    const uint32_t parts = sample_parts(mp.chunks[c].wn);
+    s = (g - __ldg(warps + i)) / parts;
+    part = (g - __ldg(warps + i)) % parts;
   }
 };
 
@@ -1530,7 +1424,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       }
     }
 
-    // finished chains: publish (hmm_work_kernel samples their haplotypes)
+    // finished chains: publish (hmm_work samples their haplotypes)
     const bool done = active && e > C;
     if (done && li == 0) {
       p.quad_out[s] = q.x;
@@ -1584,84 +1478,46 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 }
 
 // hmm_work after the generation kernel, over the published final
-// quadruples.  Pass 1: blocks of two warps over 16 samples, a lane pair per
-// sample and recursion direction in each warp (work_chains_pair), so the
-// thousand-odd blocks of a generation spread over every SM.  Pass 2: one
-// warp per part of a sample (kSampleWords words) samples its sites.  Chunks
-// without hmm_work skip both.
+// quadruples.  Pass 1: a block of two warps per 32 samples of a chunk.  Pass 2:
+// one warp per part of a sample (kSampleWords words) samples its sites.
 constexpr int kWorkThreads = 32;
-constexpr int kChainThreads = 64;
-constexpr size_t kChainSmem = 2 * sizeof(ChainTiles);  // dynamic: one per warp
-
-template <class Src>
-__device__ __forceinline__ uint4 final_quad(const Src &, const GenParams &p, uint32_t s) {
-  const uint32_t N = p.N;
-  return make_uint4(p.quad_out[s], p.quad_out[N + s], p.quad_out[2 * (size_t)N + s],
-                    p.quad_out[3 * (size_t)N + s]);
-}
+constexpr size_t kChainSmem = 2 * sizeof(ChainTiles);  // dynamic: one per recursion
 
 template <class Src>
 __device__ __forceinline__ void chains_body(const Src &src) {
   extern __shared__ __align__(16) unsigned char glp_chain_smem[];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  ChainTiles &s_tiles = reinterpret_cast<ChainTiles *>(glp_chain_smem)[warp];
-  // both warps: the block's 16 samples, two lanes each
-  const uint32_t g = blockIdx.x * (uint32_t)kPairRows + (lane >> 1);
-  const uint32_t total = src.total();
-  uint32_t c = 0, s = 0;
-  if (g < total)
-    src.locate(g, c, s);
-  else
-    src.locate(total - 1, c, s);  // idle lanes borrow a valid chunk (they skip the work)
-  const GenParams &p = src.chunk(c);
-  const bool valid = g < total && p.do_work;
-  // the warps stage rows together when all their lanes share one chunk (the
-  // two warps see the same samples, so they take the same branch and either
-  // both or neither reach the barrier in work_chains_pair)
-  int same = 0;
-  __match_all_sync(0xffffffffu, c, &same);
-  if (same) {
-    if (__any_sync(0xffffffffu, valid))
-      work_chains_pair(p, s, valid ? final_quad(src, p, s) : make_uint4(0, 0, 0, 0), valid,
-                       lane, warp == 1, s_tiles);
-  } else if (valid && warp == 0 && (lane & 1u) == 0) {
-    work_chains(p, s, final_quad(src, p, s));
-  }
+  uint32_t c, s0;
+  src.locate_block(blockIdx.x, c, s0);
+  work_chains(src.chunk(c), s0, reinterpret_cast<ChainTiles *>(glp_chain_smem));
 }
 
 template <class Src>
 __device__ __forceinline__ void sample_body(const Src &src) {
-  __shared__ float4 s_pcr[kWorkThreads / 32][4];  // the warp's mutation-matrix rows
-  __shared__ __align__(16) uint32_t s_u[kWorkThreads / 32][128];  // a span's uniforms
-  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-  // one part of one sample per warp
-  const uint64_t g = (uint64_t)blockIdx.x * (blockDim.x >> 5) + wib;
-  const uint32_t parts = src.parts();
-  if (g >= (uint64_t)src.total() * parts)
-    return;
-  const uint32_t gs = (uint32_t)(g / parts), part = (uint32_t)(g % parts);
-  uint32_t c, s;
-  src.locate(gs, c, s);
+  __shared__ float4 s_pcr[4];  // the mutation-matrix rows
+  __shared__ __align__(16) uint32_t s_u[128];  // a span's uniforms
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t c, s, part;
+  src.locate_part(blockIdx.x, c, s, part);
   const GenParams &p = src.chunk(c);
-  if (!p.do_work)
-    return;
-  const uint32_t w_lo = parts > 1 ? part * kSampleWords : 0u;
-  const uint32_t w_hi = parts > 1 ? min(p.wn, w_lo + kSampleWords) : p.wn;
+  const uint32_t w_lo = part * kSampleWords, w_hi = min(p.wn, w_lo + kSampleWords);
   if (lane < 4)
-    s_pcr[wib][lane] = make_float4(p.pc[4 * lane], p.pc[4 * lane + 1], p.pc[4 * lane + 2],
-                                   p.pc[4 * lane + 3]);
+    s_pcr[lane] = make_float4(p.pc[4 * lane], p.pc[4 * lane + 1], p.pc[4 * lane + 2],
+                              p.pc[4 * lane + 3]);
   __syncwarp();
-  work_sample(p, s_pcr[wib], s, final_quad(src, p, s), lane, s_u[wib], w_lo, w_hi);
+  const uint32_t N = p.N;
+  const uint4 q = make_uint4(p.quad_out[s], p.quad_out[N + s], p.quad_out[2 * (size_t)N + s],
+                             p.quad_out[3 * (size_t)N + s]);
+  work_sample(p, s_pcr, s, q, lane, s_u, w_lo, w_hi);
 }
 
 template <int = 0>
-__global__ void __launch_bounds__(kChainThreads) work_chains_kernel(const GenParams p) {
+__global__ void __launch_bounds__(kChainThreads, 3) work_chains_kernel(const GenParams p) {
   const OneChunk src{p};
   chains_body(src);
 }
 
 template <int = 0>
-__global__ void __launch_bounds__(kChainThreads) work_chains_multi_kernel(const MultiParams mp) {
+__global__ void __launch_bounds__(kChainThreads, 3) work_chains_multi_kernel(const MultiParams mp) {
   const ManyChunks src{mp};
   chains_body(src);
 }

@@ -89,7 +89,7 @@ __device__ __forceinline__ float2 vq_entry(const float2 *codebook, uint32_t K, u
 // the first smallest squared distance is the answer unless an earlier entry's
 // squared distance rounds to the same square root; those (within a few ulps)
 // are checked with the root itself.
-__device__ __noinline__ uint32_t vq_nearest_exact(const float2 *cb, uint32_t K, float rr,
+inline __device__ __noinline__ uint32_t vq_nearest_exact(const float2 *cb, uint32_t K, float rr,
                                                   float het, float lim) {
   uint32_t cand = 0;
   for (uint32_t k = 0; k < K; ++k) {
@@ -164,7 +164,7 @@ __device__ __forceinline__ void vq_nearest(const float2 *cb, uint32_t K, const f
 
 // A binary32 value as binary64 by integer operations (conversions run on the
 // narrow binary64 pipe); zeros, subnormals, infinities and NaN convert.
-__device__ __noinline__ double vq_widen_any(float x) { return (double)x; }
+inline __device__ __noinline__ double vq_widen_any(float x) { return (double)x; }
 __device__ __forceinline__ double vq_widen(float x) {
   const uint32_t b = __float_as_uint(x), e = (b >> 23) & 0xffu;
   if (e - 1u >= 254u && x != 0.0f)  // subnormal, infinity or NaN
