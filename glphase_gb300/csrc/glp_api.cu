@@ -1617,36 +1617,39 @@ int glp_knn_neighbors(glp_ctx *c, const uint64_t *haps, uint32_t H, uint32_t S, 
   const uint32_t wn = (S + 63) / 64;
   if ((rc = ensure(c, c->d_mask, c->mask_cap, wn)))
     return rc;
-  glp::common_sites_kernel<<<wn, 64, 0, c->stream>>>(haps, H, wn, S, lb, ub, use_maf,
+  glp::common_sites_kernel<<<wn, glp::kCommonThreads, 0, c->stream>>>(haps, H, wn, S, lb, ub, use_maf,
                                                      c->d_mask);
   GLP_CUDA(c, cudaGetLastError());
-  const size_t smem = glp::knn_smem_bytes(H);
   // tiled distances of a chunk of samples (at most 256 MB of them) into
   // global memory, then the selection, chunk by chunk
-  GLP_CUDA(c, cudaFuncSetAttribute(glp::knn_select_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const uint32_t NS = H / 2;
-  const uint32_t chunk =
-      (uint32_t)std::min<size_t>(NS, std::max<size_t>(64, ((size_t)256 << 20) / (4 * (size_t)H)));
-  if ((rc = ensure(c, c->d_knn_dist, c->knn_dist_cap, (size_t)2 * chunk * H)))
+  const uint32_t NS = H / 2, pitch = glp::knn_pitch(H);
+  const uint32_t chunk = (uint32_t)std::min<size_t>(
+      NS, std::max<size_t>(64, ((size_t)256 << 20) / (4 * (size_t)pitch)));
+  if ((rc = ensure(c, c->d_knn_dist, c->knn_dist_cap, (size_t)2 * chunk * pitch)))
     return rc;
+  const uint32_t per = 8 * glp::kKnnThreads;  // distances a vector of each thread covers
+  auto select = H <= per ? glp::knn_select_kernel<1>
+                : H <= 2 * per ? glp::knn_select_kernel<2>
+                : H <= 5 * per ? glp::knn_select_kernel<5>
+                               : glp::knn_select_kernel<13>;
+  static_assert(13 * 8 * glp::kKnnThreads >= glp::kKnnMaxHaps, "the widest selection");
   const bool tract = c->knn_metric == GLP_KNN_TRACT;
   for (uint32_t s0 = 0; s0 < NS; s0 += chunk) {
     const uint32_t n = std::min(chunk, NS - s0);
     if (tract) {
-      const dim3 grid((H + glp::kTractH - 1) / glp::kTractH,
+      const dim3 grid((pitch + glp::kTractH - 1) / glp::kTractH,
                       (2 * n + glp::kTractQ - 1) / glp::kTractQ);
       glp::knn_tract_dist_kernel<<<grid, glp::kDistThreads, 0, c->stream>>>(
-          haps, H, wn, c->d_mask, 2 * s0, 2 * n, c->d_knn_dist);
+          haps, H, wn, c->d_mask, 2 * s0, 2 * n, pitch, c->d_knn_dist);
     } else {
-      const dim3 grid((H + glp::kDistH - 1) / glp::kDistH,
+      const dim3 grid((pitch + glp::kDistH - 1) / glp::kDistH,
                       (2 * n + glp::kDistQ - 1) / glp::kDistQ);
       glp::knn_dist_kernel<<<grid, glp::kDistThreads, 0, c->stream>>>(haps, H, wn, c->d_mask,
-                                                                      2 * s0, 2 * n,
+                                                                      2 * s0, 2 * n, pitch,
                                                                       c->d_knn_dist);
     }
-    glp::knn_select_kernel<<<n, glp::kKnnThreads, smem, c->stream>>>(c->d_knn_dist, H, s0, half,
-                                                                    S, neighbors);
+    select<<<n, glp::kKnnThreads, 0, c->stream>>>(c->d_knn_dist, pitch, H, s0, half, S,
+                                                  neighbors);
     GLP_CUDA(c, cudaGetLastError());
   }
   return GLP_OK;

@@ -16,12 +16,8 @@
 // through global memory: Hamming (knn_dist_kernel), or the tract length
 // (knn_tract_dist_kernel: each word's runs of agreeing common sites --
 // before its first disagreement, after its last, the longest between --
-// joined in site order, glp_tract.h).  Selection (knn_select_kernel): one
-// CTA per sample with the distances of both its haplotypes to all H
-// haplotypes in shared memory as uint16 (H <= kKnnMaxHaps); the ceil(K/2)
-// nearest are found by binary search on the distance threshold, ties at the
-// threshold are taken in index order through a block scan, and the chosen
-// list is put in (distance, index) order by a bitonic sort.
+// joined in site order, glp_tract.h).  Selection (knn_select_kernel): one CTA
+// per sample, its two rows of distances in registers.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,37 +27,57 @@
 
 namespace glp {
 
-constexpr int kKnnThreads = 256;
+constexpr int kKnnThreads = 512;
 constexpr uint32_t kKnnMaxHaps = 50000;
 constexpr uint32_t kKnnMaxHalf = 1024;
 constexpr uint16_t kKnnExcluded = 0xffffu;
 
-// Bit m of mask: site m's alt-allele frequency (or MAF) lies in [lb, ub].
-__global__ void common_sites_kernel(const uint64_t *__restrict__ haps, uint32_t H,
-                                    uint32_t wn, uint32_t S, double lb, double ub,
-                                    int use_maf, uint64_t *__restrict__ mask) {
-  const uint32_t w = blockIdx.x;
-  const uint32_t lane = threadIdx.x;  // 64 threads: one site each
-  const uint32_t m = w * 64 + lane;
-  uint32_t alt = 0;
-  if (m < S)
-    for (uint32_t h = 0; h < H; ++h)
-      alt += (uint32_t)((__ldg(haps + (size_t)h * wn + w) >> lane) & 1u);
-  double af = (double)alt / H;
-  if (use_maf)
-    af = fabs(fabs(af - 0.5) - 0.5);
-  const bool keep = m < S && af >= lb && af <= ub;
-  const unsigned lo = __ballot_sync(0xffffffffu, lane < 32 ? keep : false);
-  __shared__ unsigned hi_bits;
-  if (lane == 32)
-    hi_bits = 0;
+// The bits of 32 lanes transposed: lane l gets bit l of every lane's x (in some
+// order, which a population count does not see).
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, uint32_t lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int s = 16; s; s >>= 1, m ^= m << s) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
+    x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
+  }
+  return x;
+}
+
+// Bit m of mask: site m's alt-allele frequency (or MAF) lies in [lb, ub].  One
+// block per word: each warp takes 32 haplotypes at a time and counts the 64
+// sites by transposing their bits.  Bound: the words' latency, a few loads a
+// thread (20,000 haplotypes x 64 words: 1,757 us with one thread a site walking
+// all haplotypes, 22 us this way).
+constexpr int kCommonThreads = 1024;
+__global__ void __launch_bounds__(kCommonThreads)
+    common_sites_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn, uint32_t S,
+                        double lb, double ub, int use_maf, uint64_t *__restrict__ mask) {
+  __shared__ uint32_t cnt[64];
+  const uint32_t w = blockIdx.x, lane = threadIdx.x & 31u;
+  if (threadIdx.x < 64)
+    cnt[threadIdx.x] = 0;
   __syncthreads();
-  const unsigned hb = __ballot_sync(0xffffffffu, keep);
-  if (lane == 32)
-    hi_bits = hb;
+  uint32_t lo = 0, hi = 0;  // of sites `lane` and 32 + lane
+#pragma unroll 4
+  for (uint32_t h0 = threadIdx.x - lane; h0 < H; h0 += kCommonThreads) {
+    const uint32_t h = h0 + lane;
+    const uint64_t x = h < H ? __ldg(haps + (size_t)h * wn + w) : 0ull;
+    lo += __popc(warp_transpose((uint32_t)x, lane));
+    hi += __popc(warp_transpose((uint32_t)(x >> 32), lane));
+  }
+  atomicAdd(&cnt[lane], lo);
+  atomicAdd(&cnt[32 + lane], hi);
   __syncthreads();
-  if (lane == 0)
-    mask[w] = (uint64_t)lo | ((uint64_t)hi_bits << 32);
+  if (threadIdx.x < 64) {
+    const uint32_t m = w * 64 + threadIdx.x;
+    double af = (double)cnt[threadIdx.x] / H;
+    if (use_maf)
+      af = fabs(fabs(af - 0.5) - 0.5);
+    const uint32_t bits = __ballot_sync(0xffffffffu, m < S && af >= lb && af <= ub);
+    if (lane == 0)
+      reinterpret_cast<uint32_t *>(mask + w)[threadIdx.x >> 5] = bits;
+  }
 }
 
 __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *red) {
@@ -106,80 +122,83 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *red,
   return base + inc - v;
 }
 
-// Choose the `half` smallest (d, index) among entries of d that are not
-// kKnnExcluded, write them sorted to out[0..half).
-__device__ void select_nearest(const uint16_t *d, uint32_t H, uint32_t half, uint32_t dmax,
-                               uint32_t *keys, uint32_t *red, uint32_t *out) {
+// The selection.  A block takes one sample; each of its two rows of distances is
+// read once, into registers (8 consecutive ones a vector).  A bound on the half-th smallest
+// comes from the threads' minima -- at least `half` distances are at most the
+// half-th smallest minimum -- by a binary search that costs one counting barrier a
+// step; the entries up to the bound are collected and put in (distance, index)
+// order by counting, for each, how many are smaller.  Rows that leave more
+// than kSelectMost entries (many equal distances) or have too few threads for a
+// useful bound take the general path: the exact threshold by a binary search over
+// all distances, ties in index order by a block scan, a bitonic sort.
+// Bound: instructions and the search's barriers (10,000 samples, 20,000
+// haplotypes, half = 100: 0.40 ms; 2.29 ms with the general path for every row,
+// one block an SM with its rows in shared memory).
+constexpr uint32_t kSelectMost = 1024;
+
+// The general path: the `half` smallest (d, index) of the entries of row d that
+// are not kKnnExcluded and not in `taken` (may be null), written sorted to
+// out[0 .. half).  keys: 2 * kKnnMaxHalf words.
+__device__ __noinline__ void select_general(const uint16_t *__restrict__ d, uint32_t H,
+                                            uint32_t half, uint32_t dmax, const uint32_t *taken,
+                                            uint32_t *keys, uint32_t *red, uint32_t *out) {
   const uint32_t tid = threadIdx.x;
+  auto at = [&](uint32_t h) -> uint32_t {
+    return taken && ((taken[h >> 5] >> (h & 31u)) & 1u) ? (uint32_t)kKnnExcluded
+                                                        : (uint32_t)__ldg(d + h);
+  };
   // smallest t with #{d <= t} >= half
   uint32_t lo = 0, hi = dmax;
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
     uint32_t c = 0;
     for (uint32_t h = tid; h < H; h += kKnnThreads)
-      c += (d[h] != kKnnExcluded && d[h] <= mid) ? 1u : 0u;
+      c += at(h) <= mid ? 1u : 0u;  // mid < kKnnExcluded
     if (block_sum(c, red) >= half)
       hi = mid;
     else
       lo = mid + 1;
   }
   const uint32_t t = lo;
-  uint32_t below = 0;
-  for (uint32_t h = tid; h < H; h += kKnnThreads)
-    below += (d[h] != kKnnExcluded && d[h] < t) ? 1u : 0u;
-  below = block_sum(below, red);
-  const uint32_t need = half - below;  // ties at t, taken in index order
   const uint32_t chunk = (H + kKnnThreads - 1) / kKnnThreads;
   const uint32_t b0 = min(H, tid * chunk), b1 = min(H, b0 + chunk);
-  uint32_t ties = 0;
-  for (uint32_t h = b0; h < b1; ++h)
-    ties += (d[h] == t) ? 1u : 0u;
-  uint32_t total;
+  uint32_t ties = 0, nless = 0;
+  for (uint32_t h = b0; h < b1; ++h) {
+    const uint32_t v = at(h);
+    ties += v == t ? 1u : 0u;
+    nless += v < t ? 1u : 0u;
+  }
+  uint32_t total, below;
   uint32_t rank = block_exclusive(ties, red, &total);
-  uint32_t nless = 0;
-  for (uint32_t h = b0; h < b1; ++h)
-    nless += (d[h] != kKnnExcluded && d[h] < t) ? 1u : 0u;
-  uint32_t pos = block_exclusive(nless, red, &total);
+  uint32_t pos = block_exclusive(nless, red, &below);
+  const uint32_t need = half - below;  // ties at t, taken in index order
   // entries below the threshold first (positions [0, below)), then ties
   for (uint32_t h = b0; h < b1; ++h) {
-    const uint16_t v = d[h];
-    if (v == kKnnExcluded)
-      continue;
+    const uint32_t v = at(h);
     if (v < t) {
-      keys[pos++] = ((uint32_t)v << 16) | 0u;
-      keys[kKnnMaxHalf + pos - 1] = h;
+      keys[pos++] = (v << 16) | h;
     } else if (v == t) {
-      if (rank < need) {
-        keys[below + rank] = ((uint32_t)v << 16);
-        keys[kKnnMaxHalf + below + rank] = h;
-      }
+      if (rank < need)
+        keys[below + rank] = (v << 16) | h;
       ++rank;
     }
   }
-  __syncthreads();
   // bitonic sort of (distance, index) over the next power of two
   uint32_t n2 = 1;
   while (n2 < half)
     n2 <<= 1;
-  for (uint32_t i = tid; i < n2; i += kKnnThreads)
-    if (i >= half) {
-      keys[i] = 0xffffffffu;
-      keys[kKnnMaxHalf + i] = 0xffffffffu;
-    }
+  for (uint32_t i = half + tid; i < n2; i += kKnnThreads)
+    keys[i] = 0xffffffffu;
   __syncthreads();
   for (uint32_t k = 2; k <= n2; k <<= 1) {
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
       for (uint32_t i = tid; i < n2; i += kKnnThreads) {
         const uint32_t l = i ^ j;
         if (l > i) {
-          const uint64_t a = ((uint64_t)keys[i] << 32) | keys[kKnnMaxHalf + i];
-          const uint64_t b = ((uint64_t)keys[l] << 32) | keys[kKnnMaxHalf + l];
-          const bool up = (i & k) == 0;
-          if ((a > b) == up) {
-            keys[i] = (uint32_t)(b >> 32);
-            keys[kKnnMaxHalf + i] = (uint32_t)b;
-            keys[l] = (uint32_t)(a >> 32);
-            keys[kKnnMaxHalf + l] = (uint32_t)a;
+          const uint32_t x = keys[i], y = keys[l];
+          if ((x > y) == ((i & k) == 0)) {
+            keys[i] = y;
+            keys[l] = x;
           }
         }
       }
@@ -187,34 +206,88 @@ __device__ void select_nearest(const uint16_t *d, uint32_t H, uint32_t half, uin
     }
   }
   for (uint32_t i = tid; i < half; i += kKnnThreads)
-    out[i] = keys[kKnnMaxHalf + i];
+    out[i] = keys[i] & 0xffffu;
   __syncthreads();
 }
 
-// The sample's neighbour list from the distances dA, dB of its two
-// haplotypes (shared memory; its own two excluded): the `half` nearest to
-// the first, then the `half` nearest to the second among those not taken,
-// interleaved into out (KNN::ClusterHaps, kNN.cpp:170-206).
-__device__ __forceinline__ void knn_choose(uint16_t *dA, uint16_t *dB, uint32_t H,
-                                           uint32_t half, uint32_t dmax, uint32_t *keys,
-                                           uint32_t *red, uint32_t *chosen, uint32_t *taken,
-                                           uint32_t *out) {
+// The `half` nearest of row d into out, sorted; kV vectors of 8 distances a
+// thread cover the row.
+template <int kV>
+__device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, uint32_t H,
+                                               uint32_t half, uint32_t dmax,
+                                               const uint32_t *taken, uint32_t want,
+                                               uint32_t *keys, uint32_t *red, uint32_t *out) {
   const uint32_t tid = threadIdx.x;
-  select_nearest(dA, H, half, dmax, keys, red, chosen);
-  for (uint32_t i = tid; i < half; i += kKnnThreads) {
-    const uint32_t h = chosen[i];
-    atomicOr(&taken[h >> 5], 1u << (h & 31u));
+  __shared__ uint32_t found;
+  uint4 v[kV];
+#pragma unroll
+  for (int i = 0; i < kV; ++i) {
+    const uint32_t h = 8 * (i * kKnnThreads + tid);
+    v[i] = h < H ? __ldg(reinterpret_cast<const uint4 *>(d + h))
+                 : make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+  }
+  if (tid == 0)
+    found = 0;
+  // the least distance of each thread; the pitch's padding is excluded like an own
+  // haplotype
+  uint32_t least = 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < kV; ++i) {
+    least = __vminu2(least, __vminu2(__vminu2(v[i].x, v[i].y), __vminu2(v[i].z, v[i].w)));
+  }
+  least = min(least & 0xffffu, least >> 16);
+  // smallest u with at least `want` threads' minima <= u (all distances when
+  // there are too few)
+  uint32_t lo = 0, hi = dmax + 1;
+  const bool bounded = __syncthreads_count(least <= dmax) >= (int)want;
+  while (bounded && lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__syncthreads_count(least <= mid) >= (int)want)
+      hi = mid;
+    else
+      lo = mid + 1;
+  }
+  const uint32_t u = bounded ? lo : dmax;
+  if (least <= u) {
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t dist = (x[j >> 1] >> (16 * (j & 1))) & 0xffffu;
+        if (dist <= u) {
+          const uint32_t h = 8 * (i * kKnnThreads + tid) + j;
+          if (!(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
+            const uint32_t n = atomicAdd(&found, 1u);
+            if (n < kSelectMost)
+              keys[n] = (dist << 16) | h;
+          }
+        }
+      }
+    }
   }
   __syncthreads();
-  for (uint32_t h = tid; h < H; h += kKnnThreads)
-    if ((taken[h >> 5] >> (h & 31u)) & 1u)
-      dB[h] = kKnnExcluded;
-  __syncthreads();
-  select_nearest(dB, H, half, dmax, keys, red, chosen + kKnnMaxHalf);
-  for (uint32_t i = tid; i < half; i += kKnnThreads) {
-    out[2 * i] = chosen[i];
-    out[2 * i + 1] = chosen[kKnnMaxHalf + i];
+  const uint32_t n = found;
+  if (n > kSelectMost || n < half) {  // the same for every thread
+    __syncthreads();
+    select_general(d, H, half, dmax, taken, keys, red, out);
+    return;
   }
+  for (uint32_t i = tid; i < ((n + 3) & ~3u); i += kKnnThreads)
+    if (i >= n)
+      keys[i] = 0xffffffffu;
+  __syncthreads();
+  for (uint32_t i = tid; i < n; i += kKnnThreads) {
+    const uint32_t key = keys[i];
+    uint32_t rank = 0;
+    for (uint32_t j = 0; j < n; j += 4) {
+      const uint4 o = *reinterpret_cast<const uint4 *>(keys + j);
+      rank += (o.x < key) + (o.y < key) + (o.z < key) + (o.w < key);
+    }
+    if (rank < half)
+      out[rank] = key & 0xffffu;
+  }
+  __syncthreads();
 }
 
 // Tiled Hamming distances for the kNN build, as a product of bit matrices:
@@ -228,7 +301,7 @@ __device__ __forceinline__ void knn_choose(uint16_t *dA, uint16_t *dB, uint32_t 
 constexpr uint32_t kDistQ = 64, kDistH = 128, kDistW = 8, kDistThreads = 256;
 __global__ void __launch_bounds__(kDistThreads)
     knn_dist_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn,
-                    const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq,
+                    const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq, uint32_t pitch,
                     uint16_t *__restrict__ dist) {
   __shared__ uint64_t sq[kDistW][kDistQ];
   __shared__ uint64_t sh[kDistW][kDistH];
@@ -280,8 +353,9 @@ __global__ void __launch_bounds__(kDistThreads)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const uint32_t h = hb + tx + 16 * j;
-      if (h < H)
-        dist[(size_t)q * H + h] = (h >> 1) == s ? kKnnExcluded : (uint16_t)acc[i][j];
+      if (h < pitch)  // excluded past H too
+        dist[(size_t)q * pitch + h] =
+            (h >> 1) == s || h >= H ? kKnnExcluded : (uint16_t)acc[i][j];
     }
   }
 }
@@ -296,7 +370,7 @@ constexpr uint32_t kTractQ = 32, kTractH = 64;
 __global__ void __launch_bounds__(kDistThreads)
     knn_tract_dist_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn,
                           const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq,
-                          uint16_t *__restrict__ dist) {
+                          uint32_t pitch, uint16_t *__restrict__ dist) {
   __shared__ uint64_t sq[kDistW][kTractQ];
   __shared__ uint64_t sh[kDistW][kTractH];
   __shared__ uint64_t smask[kDistW];
@@ -347,44 +421,47 @@ __global__ void __launch_bounds__(kDistThreads)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t h = hb + tx + 16 * j;
-      if (h < H)
-        dist[(size_t)q * H + h] =
-            (h >> 1) == s ? kKnnExcluded : (uint16_t)(run[i][j].len - run[i][j].best);
+      if (h < pitch)  // excluded past H too
+        dist[(size_t)q * pitch + h] = (h >> 1) == s || h >= H
+                                          ? kKnnExcluded
+                                          : (uint16_t)(run[i][j].len - run[i][j].best);
     }
   }
 }
 
 // The neighbour lists of the samples s0 + blockIdx.x from their rows of
-// knn_dist_kernel's distances (rows 2 i and 2 i + 1 for the chunk's i-th
-// sample).  Dynamic shared memory (knn_smem_bytes): dA, dB [H] uint16, keys
-// [2*kKnnMaxHalf] uint32, chosen [2*kKnnMaxHalf] uint32, taken bits
-// [ceil(H/32)] uint32.
+// distances (rows 2 i and 2 i + 1 of the chunk's i-th sample, `pitch` entries
+// apart, those past H excluded): the `half` nearest to its first haplotype, then
+// the `half` nearest to the second among those not taken, interleaved
+// (KNN::ClusterHaps, kNN.cpp:170-206).
+template <int kV>
 __global__ void __launch_bounds__(kKnnThreads)
-    knn_select_kernel(const uint16_t *__restrict__ dist, uint32_t H, uint32_t s0, uint32_t half,
-                      uint32_t dmax, uint32_t *__restrict__ neighbors) {
-  extern __shared__ uint4 knn_smem[];
-  uint16_t *dA = reinterpret_cast<uint16_t *>(knn_smem);
-  uint16_t *dB = dA + H;
-  uint32_t *keys = reinterpret_cast<uint32_t *>(dA + 2 * ((H + 1) & ~1u));
-  uint32_t *chosen = keys + 2 * kKnnMaxHalf;
-  uint32_t *taken = chosen + 2 * kKnnMaxHalf;
+    knn_select_kernel(const uint16_t *__restrict__ dist, uint32_t pitch, uint32_t H, uint32_t s0,
+                      uint32_t half, uint32_t dmax, uint32_t *__restrict__ neighbors) {
+  __shared__ __align__(16) uint32_t keys[kKnnMaxHalf];
+  __shared__ uint32_t chosen[2 * kKnnMaxHalf];
+  __shared__ uint32_t taken[kKnnMaxHaps / 32 + 1];
   __shared__ uint32_t red[kKnnThreads / 32];
+  static_assert(kSelectMost <= kKnnMaxHalf, "keys");
   const uint32_t tid = threadIdx.x;
-  // the two rows, 2 H uint16 in a row of the distances (H even: 4-byte units)
-  const uint32_t *row = reinterpret_cast<const uint32_t *>(dist + (size_t)2 * blockIdx.x * H);
-  uint32_t *d32 = reinterpret_cast<uint32_t *>(dA);
-  for (uint32_t i = tid; i < H; i += kKnnThreads)
-    d32[i] = __ldg(row + i);
+  const uint16_t *const row = dist + (size_t)2 * blockIdx.x * pitch;
   for (uint32_t i = tid; i < (H + 31) / 32; i += kKnnThreads)
     taken[i] = 0;
+  select_nearest<kV>(row, H, half, dmax, nullptr, half, keys, red, chosen);
+  for (uint32_t i = tid; i < half; i += kKnnThreads)
+    atomicOr(&taken[chosen[i] >> 5], 1u << (chosen[i] & 31u));
   __syncthreads();
-  knn_choose(dA, dB, H, half, dmax, keys, red, chosen, taken,
-             neighbors + (size_t)(s0 + blockIdx.x) * 2 * half);
+  // at most `half` of the second row's nearest are taken
+  select_nearest<kV>(row + pitch, H, half, dmax, taken, 2 * half, keys, red,
+                     chosen + kKnnMaxHalf);
+  uint32_t *const out = neighbors + (size_t)(s0 + blockIdx.x) * 2 * half;
+  for (uint32_t i = tid; i < half; i += kKnnThreads) {
+    out[2 * i] = chosen[i];
+    out[2 * i + 1] = chosen[kKnnMaxHalf + i];
+  }
 }
 
-inline size_t knn_smem_bytes(uint32_t H) {
-  return sizeof(uint16_t) * 2 * ((H + 1) & ~1u) + sizeof(uint32_t) * 4 * kKnnMaxHalf +
-         sizeof(uint32_t) * ((H + 31) / 32);
-}
+// Row length of the distances, in entries: whole 16-byte vectors.
+inline uint32_t knn_pitch(uint32_t H) { return (H + 127u) & ~127u; }
 
 }  // namespace glp
