@@ -25,6 +25,7 @@
 #include "../../include/glphase_gpu.h"
 #include "glp_server_core.h"
 #include "glp_knn.cuh"
+#include "glp_knn_gemm.cuh"
 #include "glp_launch.h"
 #include "glp_tally.cuh"
 #include "glp_vq.cuh"
@@ -103,8 +104,10 @@ struct glp_ctx {
   size_t quad_cap = 0, quad_out_cap = 0, props_cap = 0, nbr_cap = 0;
   uint64_t *d_mask = nullptr;  // kNN common-site mask
   size_t mask_cap = 0;
-  uint16_t *d_knn_dist = nullptr;  // kNN distances of a chunk of samples [2 n][H]
-  size_t knn_dist_cap = 0;
+  uint16_t *d_knn_dist = nullptr;  // kNN distances of a chunk of samples [2 n][pitch]
+  uint4 *d_knn_ops = nullptr;      // kNN operand rows (glp_knn_gemm.cuh)
+  uint32_t *d_knn_sites = nullptr;  // number of common sites
+  size_t knn_dist_cap = 0, knn_ops_cap = 0, knn_sites_cap = 0;
   double *d_vq_sums = nullptr;  // codebook training: block sums, counts, codebooks
   uint32_t *d_vq_counts = nullptr;
   float2 *d_vq_books = nullptr;
@@ -662,6 +665,133 @@ int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
 
 }  // namespace
 
+namespace {
+
+// How a neighbour table is built: the samples whose distances are held at a
+// time, and for the Hamming metric the operand rows.
+struct KnnPlan {
+  bool tract = false, whole = false, sym = false;
+  uint32_t pitch = 0;    // entries of a row of distances
+  uint32_t chunk = 0;    // samples
+  uint32_t bytes = 0;    // of an operand row
+  uint32_t slab = 0;     // operand rows of queries, and of haplotypes, at a time
+};
+// The whole panel's operand is kept when it takes at most 1 GB (20,000 x 4,096:
+// 82 MB), else slabs of queries and of haplotypes share that.  With it, and all
+// distances in at most 1 GB, only the tiles on and above the diagonal are
+// computed; else chunks of 256 MB of distances.
+constexpr size_t kKnnOperandBytes = (size_t)1 << 30, kKnnSymBytes = (size_t)1 << 30;
+
+KnnPlan knn_plan(uint32_t H, uint32_t S, bool tract) {
+  KnnPlan p;
+  p.tract = tract;
+  p.pitch = glp::knn_pitch(H);
+  p.bytes = glp::knn_operand_pitch(S);
+  p.whole = (size_t)H * p.bytes <= kKnnOperandBytes;
+  p.slab = p.whole ? H : (uint32_t)(kKnnOperandBytes / 2 / p.bytes / 256 * 256);
+  p.sym = !tract && p.whole && (size_t)H * p.pitch * sizeof(uint16_t) <= kKnnSymBytes;
+  p.chunk = p.sym ? H / 2
+                  : (uint32_t)std::min<size_t>(
+                        H / 2, std::max<size_t>(64, ((size_t)256 << 20) / (4 * (size_t)p.pitch)));
+  return p;
+}
+
+using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                                   const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                   const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// Tensor map of `rows` operand rows: boxes of 128 rows x 128 bytes, rows swizzled
+// by 128 bytes in shared memory, zeros past the last row.
+int operand_map(glp_ctx *c, void *base, uint32_t rows, uint32_t bytes, CUtensorMap *map) {
+  static const EncodeTiledFn encode = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault,
+                                         &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(f);
+  }();
+  const cuuint64_t dims[2] = {bytes, rows}, strides[1] = {bytes};
+  const cuuint32_t box[2] = {glp::kGemmK, glp::kGemmM}, steps[2] = {1, 1};
+  if (!encode || encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, dims, strides, box, steps,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return fail(c, GLP_ERR_CUDA, "cuTensorMapEncodeTiled failed for %u x %u", rows, bytes);
+  return GLP_OK;
+}
+
+int expand_rows(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t h0, uint32_t rows,
+                uint32_t wn, uint4 *out) {
+  const uint64_t units = (uint64_t)rows * (p.bytes / 16);
+  glp::knn_expand_kernel<<<(unsigned)((units + 255) / 256), 256, 0, c->stream>>>(
+      haps, h0, rows, wn, c->d_mask, p.bytes, out);
+  GLP_CUDA(c, cudaGetLastError());
+  return GLP_OK;
+}
+
+// Workspace of the Hamming distances, the number of common sites, and the whole
+// panel's operand when it is kept.
+int knn_operands(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t H, uint32_t wn) {
+  int rc;
+  const size_t rows = p.whole ? (size_t)H : 2 * (size_t)p.slab;
+  if ((rc = ensure(c, c->d_knn_ops, c->knn_ops_cap, rows * (p.bytes / 16))) ||
+      (rc = ensure(c, c->d_knn_sites, c->knn_sites_cap, 1)))
+    return rc;
+  GLP_CUDA(c, cudaFuncSetAttribute(glp::knn_gemm_kernel<false>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)glp::kGemmSmem));
+  GLP_CUDA(c, cudaFuncSetAttribute(glp::knn_gemm_kernel<true>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)glp::kGemmSmem));
+  glp::knn_sites_kernel<<<1, 32, 0, c->stream>>>(c->d_mask, wn, c->d_knn_sites);
+  GLP_CUDA(c, cudaGetLastError());
+  return p.whole ? expand_rows(c, p, haps, 0, H, wn, c->d_knn_ops) : GLP_OK;
+}
+
+// Distances of the queries [q0, q0 + nq) to all H haplotypes.
+int knn_products(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t H, uint32_t wn,
+                 uint32_t q0, uint32_t nq) {
+  int rc;
+  const uint32_t steps = p.bytes / glp::kGemmK;
+  auto tiles = [](uint32_t n, uint32_t t) { return (n + t - 1) / t; };
+  CUtensorMap am, bm;
+  if (p.whole) {
+    if ((rc = operand_map(c, c->d_knn_ops, H, p.bytes, &am)))
+      return rc;
+    const dim3 grid(tiles(nq, glp::kGemmM), tiles(p.pitch, glp::kGemmN));
+    auto fn = p.sym ? glp::knn_gemm_kernel<true> : glp::knn_gemm_kernel<false>;
+    fn<<<grid, glp::kGemmThreads, glp::kGemmSmem, c->stream>>>(
+        am, am, q0, 0, nq, H, q0, 0, H, steps, c->d_knn_sites, p.pitch, c->d_knn_dist,
+        c->d_error);
+    GLP_CUDA(c, cudaGetLastError());
+    return GLP_OK;
+  }
+  uint4 *const a = c->d_knn_ops, *const b = a + (size_t)p.slab * (p.bytes / 16);
+  for (uint32_t i = 0; i < nq; i += p.slab) {
+    const uint32_t na = std::min(p.slab, nq - i);
+    if ((rc = expand_rows(c, p, haps, q0 + i, na, wn, a)) ||
+        (rc = operand_map(c, a, na, p.bytes, &am)))
+      return rc;
+    for (uint32_t h = 0; h < H; h += p.slab) {
+      const uint32_t nb = std::min(p.slab, H - h);
+      if ((rc = expand_rows(c, p, haps, h, nb, wn, b)) ||
+          (rc = operand_map(c, b, nb, p.bytes, &bm)))
+        return rc;
+      const dim3 grid(tiles(na, glp::kGemmM), tiles(nb, glp::kGemmN));
+      glp::knn_gemm_kernel<false><<<grid, glp::kGemmThreads, glp::kGemmSmem, c->stream>>>(
+          am, bm, 0, 0, na, nb, q0 + i, h, H, steps, c->d_knn_sites, p.pitch,
+          c->d_knn_dist + (size_t)i * p.pitch, c->d_error);
+      GLP_CUDA(c, cudaGetLastError());
+    }
+  }
+  return GLP_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 int glp_check_device(int device, int *device_count, int *cc_major, int *cc_minor,
@@ -750,6 +880,8 @@ void glp_destroy(glp_ctx *c) {
   release(c->d_nbr);
   release(c->d_mask);
   release(c->d_knn_dist);
+  release(c->d_knn_ops);
+  release(c->d_knn_sites);
   release(c->d_vq_sums);
   release(c->d_vq_counts);
   release(c->d_vq_books);
@@ -1617,36 +1749,30 @@ int glp_knn_neighbors(glp_ctx *c, const uint64_t *haps, uint32_t H, uint32_t S, 
   const uint32_t wn = (S + 63) / 64;
   if ((rc = ensure(c, c->d_mask, c->mask_cap, wn)))
     return rc;
-  glp::common_sites_kernel<<<wn, glp::kCommonThreads, 0, c->stream>>>(haps, H, wn, S, lb, ub, use_maf,
-                                                     c->d_mask);
+  glp::common_sites_kernel<<<wn, glp::kCommonThreads, 0, c->stream>>>(haps, H, wn, S, lb, ub,
+                                                                     use_maf, c->d_mask);
   GLP_CUDA(c, cudaGetLastError());
-  // tiled distances of a chunk of samples (at most 256 MB of them) into
-  // global memory, then the selection, chunk by chunk
-  const uint32_t NS = H / 2, pitch = glp::knn_pitch(H);
-  const uint32_t chunk = (uint32_t)std::min<size_t>(
-      NS, std::max<size_t>(64, ((size_t)256 << 20) / (4 * (size_t)pitch)));
-  if ((rc = ensure(c, c->d_knn_dist, c->knn_dist_cap, (size_t)2 * chunk * pitch)))
-    return rc;
   const uint32_t per = 8 * glp::kKnnThreads;  // distances a vector of each thread covers
   auto select = H <= per ? glp::knn_select_kernel<1>
                 : H <= 2 * per ? glp::knn_select_kernel<2>
                 : H <= 5 * per ? glp::knn_select_kernel<5>
                                : glp::knn_select_kernel<13>;
   static_assert(13 * 8 * glp::kKnnThreads >= glp::kKnnMaxHaps, "the widest selection");
-  const bool tract = c->knn_metric == GLP_KNN_TRACT;
-  for (uint32_t s0 = 0; s0 < NS; s0 += chunk) {
-    const uint32_t n = std::min(chunk, NS - s0);
-    if (tract) {
+  const KnnPlan plan = knn_plan(H, S, c->knn_metric == GLP_KNN_TRACT);
+  const uint32_t pitch = plan.pitch;
+  if ((rc = ensure(c, c->d_knn_dist, c->knn_dist_cap, (size_t)2 * plan.chunk * pitch)))
+    return rc;
+  if (!plan.tract && (rc = knn_operands(c, plan, haps, H, wn)))
+    return rc;
+  for (uint32_t s0 = 0; s0 < H / 2; s0 += plan.chunk) {
+    const uint32_t n = std::min(plan.chunk, H / 2 - s0);
+    if (plan.tract) {
       const dim3 grid((pitch + glp::kTractH - 1) / glp::kTractH,
                       (2 * n + glp::kTractQ - 1) / glp::kTractQ);
       glp::knn_tract_dist_kernel<<<grid, glp::kDistThreads, 0, c->stream>>>(
           haps, H, wn, c->d_mask, 2 * s0, 2 * n, pitch, c->d_knn_dist);
-    } else {
-      const dim3 grid((pitch + glp::kDistH - 1) / glp::kDistH,
-                      (2 * n + glp::kDistQ - 1) / glp::kDistQ);
-      glp::knn_dist_kernel<<<grid, glp::kDistThreads, 0, c->stream>>>(haps, H, wn, c->d_mask,
-                                                                      2 * s0, 2 * n, pitch,
-                                                                      c->d_knn_dist);
+    } else if ((rc = knn_products(c, plan, haps, H, wn, 2 * s0, 2 * n))) {
+      return rc;
     }
     select<<<n, glp::kKnnThreads, 0, c->stream>>>(c->d_knn_dist, pitch, H, s0, half, S,
                                                   neighbors);

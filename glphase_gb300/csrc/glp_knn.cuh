@@ -12,8 +12,8 @@
 // with the unstable std::sort (kNN.cpp:172-173), so its tie order is
 // implementation-defined.
 //
-// Distances as tiled products of bit matrices, a chunk of samples at a time
-// through global memory: Hamming (knn_dist_kernel), or the tract length
+// Distances, a chunk of samples at a time through global memory: Hamming as a
+// matrix product (knn_gemm_kernel, glp_knn_gemm.cuh), or the tract length
 // (knn_tract_dist_kernel: each word's runs of agreeing common sites --
 // before its first disagreement, after its last, the longest between --
 // joined in site order, glp_tract.h).  Selection (knn_select_kernel): one CTA
@@ -290,83 +290,14 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
   __syncthreads();
 }
 
-// Tiled Hamming distances for the kNN build, as a product of bit matrices:
-// dist[q][h] = popcount((hap q0+q XOR hap h) AND mask) over the words, for
-// the query haplotypes [q0, q0 + nq) (2 s and 2 s + 1 for the samples s of a
-// chunk) and every haplotype h; a sample's own two are marked excluded.  A
-// CTA takes 64 queries x 128 haplotypes and walks the words 8 at a time,
-// staged word-major in shared memory (a warp's reads of a word are
-// consecutive); each thread keeps 4 x 8 sums.  Each panel word is read from
-// L2 once per 64 queries instead of once per sample.
-constexpr uint32_t kDistQ = 64, kDistH = 128, kDistW = 8, kDistThreads = 256;
-__global__ void __launch_bounds__(kDistThreads)
-    knn_dist_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn,
-                    const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq, uint32_t pitch,
-                    uint16_t *__restrict__ dist) {
-  __shared__ uint64_t sq[kDistW][kDistQ];
-  __shared__ uint64_t sh[kDistW][kDistH];
-  __shared__ uint64_t smask[kDistW];
-  const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
-  const uint32_t hb = blockIdx.x * kDistH, qb = blockIdx.y * kDistQ;
-  uint32_t acc[4][8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      acc[i][j] = 0;
-  for (uint32_t w0 = 0; w0 < wn; w0 += kDistW) {
-    for (uint32_t i = tid; i < kDistQ * kDistW; i += kDistThreads) {
-      const uint32_t r = i / kDistW, k = i % kDistW, w = w0 + k;
-      sq[k][r] = (qb + r < nq && w < wn) ? __ldg(haps + (size_t)(q0 + qb + r) * wn + w) : 0ull;
-    }
-    for (uint32_t i = tid; i < kDistH * kDistW; i += kDistThreads) {
-      const uint32_t r = i / kDistW, k = i % kDistW, w = w0 + k;
-      sh[k][r] = (hb + r < H && w < wn) ? __ldg(haps + (size_t)(hb + r) * wn + w) : 0ull;
-    }
-    if (tid < kDistW)
-      smask[tid] = w0 + tid < wn ? __ldg(mask + w0 + tid) : 0ull;
-    __syncthreads();
-#pragma unroll
-    for (uint32_t k = 0; k < kDistW; ++k) {
-      const uint64_t mk = smask[k];
-      uint64_t qv[4], hv[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        qv[i] = sq[k][4 * ty + i] & mk;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        hv[j] = sh[k][tx + 16 * j] & mk;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          acc[i][j] += __popcll(qv[i] ^ hv[j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t q = qb + 4 * ty + i;
-    if (q >= nq)
-      continue;
-    const uint32_t s = (q0 + q) >> 1;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t h = hb + tx + 16 * j;
-      if (h < pitch)  // excluded past H too
-        dist[(size_t)q * pitch + h] =
-            (h >> 1) == s || h >= H ? kKnnExcluded : (uint16_t)acc[i][j];
-    }
-  }
-}
-
-// Tiled tract-length distances (-T), laid out as knn_dist_kernel's: each
-// pair carries the runs of agreeing common sites of the words so far --
+// Tiled tract-length distances (-T) of the query haplotypes [q0, q0 + nq) (2 s
+// and 2 s + 1 for the samples s of a chunk) against every haplotype: the words
+// 8 at a time, word-major in shared memory; each pair carries the runs of agreeing common sites of the words so far --
 // before the first disagreement, after the last, the longest -- and joins
 // every next word's (tract_word) to them in site order; the distance is the
 // common sites minus the longest run.  A CTA takes 32 queries x 64
 // haplotypes, each thread 2 x 4 pairs.
-constexpr uint32_t kTractQ = 32, kTractH = 64;
+constexpr uint32_t kTractQ = 32, kTractH = 64, kDistW = 8, kDistThreads = 256;
 __global__ void __launch_bounds__(kDistThreads)
     knn_tract_dist_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn,
                           const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq,

@@ -91,3 +91,37 @@ def test_common_sites_of_many_haplotypes(dev):
     keep = (bits.sum(axis=0) >= 300) & (bits.sum(axis=0) <= 900)
     got = gpu_knn(dev, mdl.pack_haplotypes(bits), S, K, lo, hi)
     assert np.array_equal(got[[0, 700, 1500]], want(bits[:, keep], K, [0, 700, 1500]))
+
+
+def want_words(words, K, samples):
+    half = (K + 1) // 2
+    out = []
+    for s in samples:
+        lists, taken = [], np.zeros(len(words), bool)
+        taken[2 * s:2 * s + 2] = True
+        for h in (2 * s, 2 * s + 1):
+            d = np.bitwise_count(words ^ words[h]).sum(axis=1, dtype=np.int64)
+            d[taken] = 1 << 20
+            lists.append(np.argsort(d, kind="stable")[:half])
+            taken[lists[-1]] = True
+        out.append(np.stack(lists, axis=1).reshape(-1))
+    return np.array(out, np.uint32)
+
+
+@pytest.mark.parametrize("H,S,K", [(300, 65534, 40), (24002, 64, 100), (50000, 22000, 200)])
+def test_words(dev, H, S, K):
+    """The most sites (sums near 2^16), distances held a chunk at a time, and
+    operand rows a slab at a time."""
+    rng = np.random.default_rng(H)
+    wn = (S + 63) // 64
+    words = rng.integers(0, 2**64, size=(H, wn), dtype=np.uint64)
+    words[:, -1] &= np.uint64((1 << (S - 64 * (wn - 1))) - 1 if S % 64 else 2**64 - 1)
+    if H == 300:
+        words[:100] = words[0]                     # equal haplotypes: a product of S
+        words[100:200] = ~words[0]                 # and opposite ones: of -S
+        words[100:200, -1] &= np.uint64((1 << (S - 64 * (wn - 1))) - 1)
+        for i in range(200):                       # one to 200 sites apart
+            words[i, :i // 64 + 1] ^= np.uint64((1 << (i % 64 + 1)) - 1)
+    samples = [0, 1, 60, H // 4, H // 2 - 1]
+    got = gpu_knn(dev, words, S, K)
+    assert np.array_equal(got[samples], want_words(words, K, samples))
