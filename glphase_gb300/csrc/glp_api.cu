@@ -677,9 +677,9 @@ struct KnnPlan {
   uint32_t slab = 0;     // operand rows of queries, and of haplotypes, at a time
 };
 // The whole panel's operand is kept when it takes at most 1 GB (20,000 x 4,096:
-// 82 MB), else slabs of queries and of haplotypes share that.  With it, and all
-// distances in at most 1 GB, only the tiles on and above the diagonal are
-// computed; else chunks of 256 MB of distances.
+// 82 MB), else slabs of queries and of haplotypes share that.  With all distances
+// in at most 1 GB (and the operand whole), only the tiles on and above the
+// diagonal are computed; else chunks of 256 MB of distances.
 constexpr size_t kKnnOperandBytes = (size_t)1 << 30, kKnnSymBytes = (size_t)1 << 30;
 
 KnnPlan knn_plan(uint32_t H, uint32_t S, bool tract) {
@@ -689,7 +689,7 @@ KnnPlan knn_plan(uint32_t H, uint32_t S, bool tract) {
   p.bytes = glp::knn_operand_pitch(S);
   p.whole = (size_t)H * p.bytes <= kKnnOperandBytes;
   p.slab = p.whole ? H : (uint32_t)(kKnnOperandBytes / 2 / p.bytes / 256 * 256);
-  p.sym = !tract && p.whole && (size_t)H * p.pitch * sizeof(uint16_t) <= kKnnSymBytes;
+  p.sym = (tract || p.whole) && (size_t)H * p.pitch * sizeof(uint16_t) <= kKnnSymBytes;
   p.chunk = p.sym ? H / 2
                   : (uint32_t)std::min<size_t>(
                         H / 2, std::max<size_t>(64, ((size_t)256 << 20) / (4 * (size_t)p.pitch)));
@@ -1769,7 +1769,8 @@ int glp_knn_neighbors(glp_ctx *c, const uint64_t *haps, uint32_t H, uint32_t S, 
     if (plan.tract) {
       const dim3 grid((pitch + glp::kTractH - 1) / glp::kTractH,
                       (2 * n + glp::kTractQ - 1) / glp::kTractQ);
-      glp::knn_tract_dist_kernel<<<grid, glp::kDistThreads, 0, c->stream>>>(
+      auto fn = plan.sym ? glp::knn_tract_dist_kernel<true> : glp::knn_tract_dist_kernel<false>;
+      fn<<<grid, glp::kDistThreads, 0, c->stream>>>(
           haps, H, wn, c->d_mask, 2 * s0, 2 * n, pitch, c->d_knn_dist);
     } else if ((rc = knn_products(c, plan, haps, H, wn, 2 * s0, 2 * n))) {
       return rc;

@@ -292,28 +292,45 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
 
 // Tiled tract-length distances (-T) of the query haplotypes [q0, q0 + nq) (2 s
 // and 2 s + 1 for the samples s of a chunk) against every haplotype: the words
-// 8 at a time, word-major in shared memory; each pair carries the runs of agreeing common sites of the words so far --
-// before the first disagreement, after the last, the longest -- and joins
-// every next word's (tract_word) to them in site order; the distance is the
-// common sites minus the longest run.  A CTA takes 32 queries x 64
-// haplotypes, each thread 2 x 4 pairs.
+// 8 at a time, word-major in shared memory; each pair carries its open and its
+// longest run of agreeing common sites through the words (words whose sites are
+// all common, nearly all of them, as two 32-bit halves); the distance is the common
+// sites minus the longest run.  A CTA takes 32 queries x 64 haplotypes, each
+// thread 2 x 4 pairs.  kSym: the queries are the whole panel; tiles below the
+// diagonal are not computed, their distances are written transposed.
+// Bound: the ALU instructions of a pair's word (89 % of that pipe).  4,990
+// haplotypes x 1,024 sites: 1.82 ms with all tiles and each 64-bit word's longest
+// run found on its own, 0.92 with the tiles of one half, 0.85 with `best` raised
+// inside one pass (it rises mostly in the first words, and every lane waits), 0.63
+// ms in two passes; 20,000 x 4,096 the table 119 -> 33 ms.
 constexpr uint32_t kTractQ = 32, kTractH = 64, kDistW = 8, kDistThreads = 256;
+template <bool kSym>
 __global__ void __launch_bounds__(kDistThreads)
     knn_tract_dist_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn,
                           const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq,
                           uint32_t pitch, uint16_t *__restrict__ dist) {
+  const uint32_t hb = blockIdx.x * kTractH, qb = blockIdx.y * kTractQ;
+  if (kSym && hb + kTractH <= qb)
+    return;
   __shared__ uint64_t sq[kDistW][kTractQ];
   __shared__ uint64_t sh[kDistW][kTractH];
   __shared__ uint64_t smask[kDistW];
+  __shared__ uint16_t st[kSym ? kTractH : 1][kTractQ + 2];  // the tile transposed
   const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
-  const uint32_t hb = blockIdx.x * kTractH, qb = blockIdx.y * kTractQ;
-  Tract run[2][4];
+  uint32_t common = 0;
+  OpenRun run[2][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      run[i][j] = Tract{0, 0, 0, 0};
-  for (uint32_t w0 = 0; w0 < wn; w0 += kDistW) {
+      run[i][j] = OpenRun{0, kRunFloor};
+  // twice over the words: the runs that cross 32-site boundaries (and the words
+  // with sites that are not common), which leave `best` near the longest; then the
+  // runs inside, which seldom exceed it
+#pragma unroll 1
+  for (uint32_t chunk = 0, chunks = (wn + kDistW - 1) / kDistW; chunk < 2 * chunks; ++chunk) {
+    const bool inside = chunk >= chunks;
+    const uint32_t w0 = (inside ? chunk - chunks : chunk) * kDistW;
     for (uint32_t i = tid; i < kTractQ * kDistW; i += kDistThreads) {
       const uint32_t r = i / kDistW, k = i % kDistW, w = w0 + k;
       sq[k][r] = (qb + r < nq && w < wn) ? __ldg(haps + (size_t)(q0 + qb + r) * wn + w) : 0ull;
@@ -335,27 +352,68 @@ __global__ void __launch_bounds__(kDistThreads)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         hv[j] = sh[k][tx + 16 * j];
+      if (inside) {
+        if (m == ~0ull) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+          for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          run[i][j] = tract_join(run[i][j], tract_word((qv[i] ^ hv[j]) & m, m));
+            for (int j = 0; j < 4; ++j) {
+              tract_inside32(run[i][j].best, (uint32_t)(qv[i] ^ hv[j]));
+              tract_inside32(run[i][j].best, (uint32_t)((qv[i] ^ hv[j]) >> 32));
+            }
+        }
+        continue;
+      }
+      common += tract_popc(m);
+      if (m == ~0ull) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            tract_extend32(run[i][j], (uint32_t)(qv[i] ^ hv[j]));
+            tract_extend32(run[i][j], (uint32_t)((qv[i] ^ hv[j]) >> 32));
+          }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            tract_extend(run[i][j], (qv[i] ^ hv[j]) & m, m);
+      }
     }
     __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const uint32_t q = qb + 2 * ty + i;
-    if (q >= nq)
-      continue;
-    const uint32_t s = (q0 + q) >> 1;
+    const uint32_t q = qb + 2 * ty + i, s = (q0 + q) >> 1;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t h = hb + tx + 16 * j;
-      if (h < pitch)  // excluded past H too
-        dist[(size_t)q * pitch + h] = (h >> 1) == s || h >= H
-                                          ? kKnnExcluded
-                                          : (uint16_t)(run[i][j].len - run[i][j].best);
+      uint32_t best = run[i][j].best;
+      if (best == kRunFloor && q < nq && h < H) {  // no longer run: its exact length
+        const uint64_t *const x = haps + (size_t)(q0 + q) * wn, *const y = haps + (size_t)h * wn;
+        Tract t{0, 0, 0, 0};
+        for (uint32_t w = 0; w < wn; ++w) {
+          const uint64_t m = __ldg(mask + w);
+          t = tract_join(t, tract_word((__ldg(x + w) ^ __ldg(y + w)) & m, m));
+        }
+        best = t.best;
+      }
+      const uint16_t d = (h >> 1) == s || h >= H ? kKnnExcluded : (uint16_t)(common - best);
+      if (q < nq && h < pitch)  // excluded past H too
+        dist[(size_t)q * pitch + h] = d;
+      if (kSym)
+        st[tx + 16 * j][2 * ty + i] = d;
+    }
+  }
+  if (kSym) {
+    __syncthreads();
+    const uint32_t q = qb + (tid & 31u);
+    for (uint32_t r = tid >> 5; r < kTractH; r += kDistThreads / 32) {
+      // row h, column q: its own tile is not computed when it lies below the diagonal
+      const uint32_t h = hb + r;
+      if (h < H && q < nq && (qb & ~(kTractH - 1)) + kTractH <= (h & ~(kTractQ - 1)))
+        dist[(size_t)h * pitch + q] = st[r][tid & 31u];
     }
   }
 }

@@ -106,4 +106,48 @@ GLP_TRACT_FN Tract tract_join(const Tract l, const Tract r) {
   return t;
 }
 
+// The runs of a pair over the stretch so far: `best` the longest, `open` the one
+// that reaches its end.  best starts at kRunFloor: a pair that still has it at the
+// end has no longer run, and its longest is found by tract_join.
+struct OpenRun {
+  uint32_t open, best;
+};
+constexpr uint32_t kRunFloor = 7;
+
+// The stretch followed by one word (x the disagreements at common sites, m the
+// common sites).
+GLP_TRACT_FN void tract_extend(OpenRun &r, uint64_t x, uint64_t m) {
+  const Tract t = tract_word(x, m);
+  r.best = tract_max(tract_max(r.best, t.best), r.open + t.pre);
+  r.open = x == 0 ? r.open + t.len : t.suf;
+}
+
+// The stretch followed by 32 sites that are all common, but for the runs inside
+// them: the runs that touch their ends come from the counts of leading and
+// trailing zeros.
+GLP_TRACT_FN void tract_extend32(OpenRun &r, uint32_t x) {
+#if defined(__CUDA_ARCH__)
+  const uint32_t low = (uint32_t)__clz((int)__brev(x)), high = (uint32_t)__clz((int)x);
+#else
+  const uint32_t low = x ? (uint32_t)__builtin_ctz(x) : 32u,
+                 high = x ? (uint32_t)__builtin_clz(x) : 32u;
+#endif
+  r.best = tract_max(r.best, r.open + low);
+  r.open = high + (x == 0 ? r.open : 0u);
+}
+
+// The runs inside 32 sites that are all common, which matter only beyond `best`
+// (at least kRunFloor): two shifted starts of runs of 8 (or 16) tell whether there
+// is one, and `best` goes up while there is.
+GLP_TRACT_FN void tract_inside32(uint32_t &best, uint32_t x) {
+  const uint32_t r1 = ~x, r2 = r1 & (r1 >> 1), r4 = r2 & (r2 >> 2), r8 = r4 & (r4 >> 4),
+                 r16 = r8 & (r8 >> 8);
+  for (;;) {  // bit i of `from`: a run of 8 (16) starts at i; none starts past 24 (16)
+    const uint32_t from = best < 15 ? r8 : r16, by = best - (best < 15 ? 7u : 15u);
+    if (!(from & (from >> (by < 31u ? by : 31u))))
+      break;
+    ++best;
+  }
+}
+
 }  // namespace glp
