@@ -1617,7 +1617,9 @@ int glp_tally(glp_ctx *c, const uint64_t *haps, uint32_t N, uint32_t S, uint32_t
     return rc;
   if (!haps || !hsum || N == 0 || S == 0)
     return fail(c, GLP_ERR_ARG, "haps, hsum, num_samples and num_sites are required");
-  glp::replace_kernel<<<N, glp::kTallyThreads, 0, c->stream>>>(haps, N, S, (S + 63) / 64, hsum);
+  auto fn = (S & 3u) == 0 && ((uintptr_t)hsum & 15u) == 0 ? glp::replace_kernel<4>
+                                                          : glp::replace_kernel<1>;
+  fn<<<N, glp::tally_threads(S), 0, c->stream>>>(haps, N, S, (S + 63) / 64, hsum);
   GLP_CUDA(c, cudaGetLastError());
   return GLP_OK;
 }
@@ -1629,10 +1631,13 @@ int glp_result(glp_ctx *c, const uint32_t *hsum, uint32_t N, uint32_t S, uint32_
     return rc;
   if (!hsum || !prob_out || N == 0 || S == 0 || sn == 0)
     return fail(c, GLP_ERR_ARG, "hsum, prob_out, sizes and sampling_generations are required");
-  const uint64_t total = (uint64_t)2 * N * S;
   const float norm = (float)(1.0 / sn);
-  glp::result_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(hsum, N, S, norm,
-                                                                          prob_out);
+  const uint32_t site_tiles = (uint32_t)(((uint64_t)S + glp::kResultTile - 1) / glp::kResultTile);
+  const uint64_t tiles =
+      site_tiles * (((uint64_t)2 * N + glp::kResultTile - 1) / glp::kResultTile);
+  glp::result_kernel<<<(unsigned)tiles, glp::kResultThreads, 0, c->stream>>>(hsum, N, S,
+                                                                           site_tiles, norm,
+                                                                           prob_out);
   GLP_CUDA(c, cudaGetLastError());
   return GLP_OK;
 }
