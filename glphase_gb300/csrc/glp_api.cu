@@ -83,6 +83,7 @@ struct glp_problem {
 struct glp_ctx {
   int device = 0;
   int sms = 0;
+  size_t l2_bytes = 0;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   std::string err;
@@ -442,20 +443,25 @@ double resident_threads(Fn fn, uint32_t P, int sms) {
   return (double)occ * glp::kThreads * sms;
 }
 
-// Speculation width for N samples at acceptance rate a.  A group of P lanes
-// scores n = P/2 positions of the chain a round (one per lane pair), of which
-// (1 - (1-a)^n) / (a n) are useful.  A lane-round costs kLaneRoundCost[P]
-// relative to P = 8 when the GPU is full (narrow groups stage more rows per
-// lane, and at 2 lanes the staging rings cap the resident blocks).  The
-// kernels are issue-bound, so lane-rounds run at a rate that saturates with
-// the share u = min(N P, threads resident with P lanes) / the most resident
-// for any P: rate(u) = u (1 + h) / (u + h), h = 0.08 (0.93 of the full rate
-// at half the warps).  The score is useful fraction x rate / cost.
-constexpr double kLaneRoundCost[6] = {0.0, 2.44, 1.34, 1.0, 0.955, 0.953};
+// Speculation width for N samples at acceptance rate a.  A generation lasts as
+// long as its longest chain while every sample has a group of its own, so the
+// rule compares, for each width, the rounds of a chain that accepts more often
+// than the average, 1 / consumed(P) for consumed = (1 - (1-a')^n) / a', n = P/2
+// positions a round, a' = a + min(a, 0.12), times what a warp's round costs at
+// the warps a scheduler holds.  Measured (1,024 sites, a = 0.12, times of a
+// generation kernel relative to one warp a scheduler): 1.44 at two, 2.0 at three,
+// beyond that in proportion (whole blocks of four warps, so the steps are at
+// multiples of the SM count).  Narrow groups stage more rows a lane: 1.12 at 4
+// lanes (1.35 when rows stream from memory), 2.2 at 2 lanes; on VQ codes, whose
+// table reads conflict more in a wide group, 1.15 at 32.  The widths this picks,
+// against 8 and 16 lanes: 256 samples 32 lanes 0.36 ms (0.56, 0.40), 1,000
+// samples 16 lanes 0.43 (0.56, 0.43; 32 lanes 0.52), 2,000 x 8,192 from a panel 16
+// lanes 4.25 (5.15, 4.25; 32 lanes 6.07), 10,000 samples 8 lanes 1.67 (1.67, 2.03).
+constexpr double kLaneRoundCost[6] = {0.0, 2.2, 1.12, 1.0, 1.0, 1.0};
 
 template <class FnOf>
-uint32_t pick_lanes(double a, uint64_t N, int sms, FnOf kernel_for, double *cache = nullptr,
-                    bool *known = nullptr) {
+uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
+                    double *cache = nullptr, bool *known = nullptr) {
   double local[6] = {};
   double *res = cache ? cache : local;
   if (!known || !*known) {
@@ -465,23 +471,28 @@ uint32_t pick_lanes(double a, uint64_t N, int sms, FnOf kernel_for, double *cach
     if (known)
       *known = true;
   }
-  double most = 0;
-  for (int i = 1; i < 6; ++i)
-    most = std::max(most, res[i]);
-  if (most <= 0)
-    return 8;
-  uint32_t best = 2;
-  double best_score = 0;
+  const double as = std::min(a + std::min(a, 0.12), 1.0);
+  uint32_t best = 8;
+  double best_time = 0;
   for (int i = 1; i < 6; ++i) {
+    if (res[i] <= 0)
+      continue;
     const uint32_t P = 1u << i;
     const double n = P / 2;
-    const double eff = (1.0 - std::pow(1.0 - a, n)) / (a * n);
-    const double u = std::min((double)N * P, res[i]) / most;
-    constexpr double h = 0.08;
-    const double rate = u * (1.0 + h) / (u + h);
-    const double score = eff * rate / kLaneRoundCost[i];
-    if (score > best_score * 1.02) {
-      best_score = score;
+    const double consumed = (1.0 - std::pow(1.0 - as, n)) / as;
+    const uint64_t per_block = (uint64_t)glp::kThreads / P;
+    const uint64_t blocks = (N + per_block - 1) / per_block;
+    // blocks an SM holds at a time, and for one warp a scheduler in each
+    const double most = std::max(1.0, res[i] / ((double)glp::kThreads * sms));
+    const double held = (double)((blocks + sms - 1) / sms);
+    auto warps_cost = [](double w) { return w <= 1 ? 1.0 : w <= 2 ? 1.44 : w * (2.0 / 3.0); };
+    const double warps = held <= most
+                             ? warps_cost(held * glp::kWarps / 4.0)
+                             : warps_cost(most * glp::kWarps / 4.0) * ((double)blocks / sms) / most;
+    const double cost = kLaneRoundCost[i] * (vq && P == 32 ? 1.15 : 1.0);
+    const double time = warps * cost / consumed;
+    if (best_time == 0 || time < best_time * 0.98) {
+      best_time = time;
       best = P;
     }
   }
@@ -495,7 +506,7 @@ uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen) {
                        ? 0.12
                        : std::max(c->last_accept, 1e-3);
   return pick_lanes(
-      a, N, c->sms,
+      a, N, c->sms, vq,
       [&](uint32_t P) {
         Shape sh;
         sh.P = P;
@@ -634,12 +645,34 @@ unsigned grid_for(glp_ctx *c, Fn fn, uint64_t samples, uint32_t P, int *rc) {
   return (unsigned)std::max<uint64_t>(1, std::min(want, cap));
 }
 
+// Emission rows that the rounds of a generation read again and again.
+uint64_t emission_bytes(const glp::GenParams &p) {
+  return p.emit_mode == GLP_EMIT_FLOAT ? (uint64_t)p.N * p.S * sizeof(float4) : 0;
+}
+
+// Whether the rows are asked for ahead (GenParams::stream): when they exceed L2
+// and the launch leaves few warps to wait for them -- one chunk of at most two
+// 8-lane warps a scheduler, or chunks of different lengths, whose longest ends
+// alone (2,000 x 8,192: 6.30 -> 5.64 ms a generation, eight uneven chunks 14.4 ->
+// 14.1; with the GPU full, 10,000 x 4,096, 7.39 -> 7.43).
+void mark_stream(const glp_ctx *c, glp::GenParams *chunks, uint32_t count) {
+  uint64_t bytes = 0, samples = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    bytes += emission_bytes(chunks[i]);
+    samples += chunks[i].N;
+  }
+  const bool few = count > 1 || samples * 8 <= (uint64_t)2 * 128 * c->sms;
+  for (uint32_t i = 0; i < count; ++i)
+    chunks[i].stream = bytes > c->l2_bytes && few ? 1u : 0u;
+}
+
 int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
   glp::GenParams p;
   int rc = make_params(c, pb, a, &p);
   if (rc)
     return rc;
   const bool vq = (a->flags & GLP_GEN_VQ) != 0;
+  mark_stream(c, &p, 1);
   const Shape sh = choose_shape(c, a->num_samples, false, vq, a->pen);
   const uint32_t P = sh.P;
   SingleFn fn = single_kernel(sh, vq);
@@ -851,6 +884,7 @@ int glp_create(int device, glp_ctx **out) {
         return GLP_ERR_CUDA;
       }
   c->sms = prop.multiProcessorCount;
+  c->l2_bytes = (size_t)prop.l2CacheSize;
   c->stream = c->own_stream;
   *out = c;
   return GLP_OK;
@@ -1052,6 +1086,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     if (total > 0xffffffffull)
       return fail(c, GLP_ERR_ARG, "a batch holds at most 2^32-1 samples");
   }
+  mark_stream(c, c->h_table, count);
   const WorkGrids work = batch_tables(c->h_table, count, c->h_offsets);
   if ((rc = ensure(c, c->d_table, c->table_cap, count)) ||
       (rc = ensure(c, c->d_offsets, c->offsets_cap, glp::batch_words(count))))
@@ -1173,6 +1208,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   glp_batch *b = new glp_batch();
   b->c = c;
   b->count = count;
+  mark_stream(c, table.data(), count);
   b->work = batch_tables(table.data(), count, offsets.data());
   b->chain_cycles = chain_cycles;
   cudaStream_t cs = nullptr;
@@ -2064,7 +2100,7 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   // measured at set-up
   bool known = true;
   const uint32_t P = pick_lanes(
-      0.12, N, sms,
+      0.12, N, sms, false,
       [](uint32_t w) {
         Shape s1;
         s1.P = w;
