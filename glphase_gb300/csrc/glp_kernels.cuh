@@ -542,18 +542,6 @@ __device__ __forceinline__ double eval_pair(const GenParams &p, const E &em, uin
   FState x;
   fstate_fill(x, 0x1p60f, bwd ? -60 : -62);
   uint32_t eacc = 0;  // OR of the blocks' range codes (fwd_norm)
-  if (bwd && (S & 63u)) {
-    const Parents pw = load_parents(p.haps, wn, q, nw);
-#pragma unroll 1
-    for (int m = (int)S - 1; m >= (int)(nw * 64); --m) {
-      const uint32_t j = (uint32_t)m & 63u;
-      float s00, s01, s10, s11;
-      select4(em.get1((uint32_t)m), (pw.f0 >> j) & 1, (pw.f1 >> j) & 1, (pw.m0 >> j) & 1,
-              (pw.m1 >> j) & 1, s00, s01, s10, s11);
-      fwd_step(x, __ldg(tran4 + m + 1), s00, s01, s10, s11);
-    }
-    fwd_renorm(x);
-  }
   float4 *const stF = stage, *const stB = stage + kBwdOffF4;
   const StageRows rows = stage_rows<kMaxRows>(li, P);
   // block t0 + d of both directions into slot (t0 + d) mod 4: forward sites
@@ -576,6 +564,43 @@ __device__ __forceinline__ double eval_pair(const GenParams &p, const E &em, uin
   };
   issue(0, 0);
   issue(0, 1);
+  if (bwd && (S & 63u)) {
+    // the sites of the partial top word, four at a time with the next four's
+    // rows already on their way
+    const Parents pw = load_parents(p.haps, wn, q, nw);
+    const int lo = (int)(nw * 64);
+    float4 e[4], t[4];
+    auto load = [&](int m0) {  // sites m0, m0 - 1, ...
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t m = (uint32_t)max(m0 - k, lo);
+        e[k] = em.get1(m);
+        t[k] = __ldg(tran4 + m + 1);
+      }
+    };
+    load((int)S - 1);
+#pragma unroll 1
+    for (int m0 = (int)S - 1; m0 >= lo; m0 -= 4) {
+      float4 ce[4], ct[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        ce[k] = e[k];
+        ct[k] = t[k];
+      }
+      load(m0 - 4);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (m0 - k < lo)
+          break;
+        const uint32_t j = (uint32_t)(m0 - k) & 63u;
+        float s00, s01, s10, s11;
+        select4(ce[k], (pw.f0 >> j) & 1, (pw.f1 >> j) & 1, (pw.m0 >> j) & 1, (pw.m1 >> j) & 1,
+                s00, s01, s10, s11);
+        fwd_step(x, ct[k], s00, s01, s10, s11);
+      }
+    }
+    fwd_renorm(x);
+  }
   float4 *const mine = bwd ? stB : stF;
 #pragma unroll 1
   for (uint32_t i = 0; i < wf; ++i) {
@@ -1079,6 +1104,33 @@ __device__ __forceinline__ void set_slot(uint4 &q, uint32_t r, uint32_t v) {
     q.w = v;
 }
 
+// One cycle's draws: the accept uniform, the proposed haplotype and the slot that
+// it replaces.
+struct __align__(16) Draw {
+  double u;
+  uint32_t hap, slot;
+};
+constexpr uint32_t kDraws = 64;  // a warp's windows: two per lane of each group
+
+// L1 prefetch of the words of haplotype h that an evaluation starts with: word 0
+// (forward), the top whole word and the partial one (backward).
+__device__ __forceinline__ void prefetch_first(const GenParams &p, uint32_t h, bool fwd) {
+  const uint64_t *const row = p.haps + (size_t)h * p.wn;
+  if (fwd) {
+    prefetch_l1(row);
+  } else {
+    const uint32_t nw = p.S >> 6;
+    prefetch_l1(row + (nw ? nw - 1 : 0));
+    prefetch_l1(row + p.wn - 1);
+  }
+}
+__device__ __forceinline__ void prefetch_first(const GenParams &p, uint4 q, bool fwd) {
+  prefetch_first(p, q.x, fwd);
+  prefetch_first(p, q.y, fwd);
+  prefetch_first(p, q.z, fwd);
+  prefetch_first(p, q.w, fwd);
+}
+
 // Work sources.  One chunk: the kernel parameter.  Many chunks: a descriptor
 // table in global memory; the samples of all chunks form one queue, chunk by
 // chunk, so a group's neighbours in the queue usually share its chunk.
@@ -1230,7 +1282,11 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
   // current partition of the warp's lanes
   uint32_t Pc = P, gbase = lane - lane % P, gidx = lane / P, ngroups = G0;
   uint32_t li = lane - gbase;
-  extern __shared__ float4 glp_stage[];  // kWarps * (32/P) * kGroupStrideF4 float4
+  // kWarps * (32/P) * kGroupStrideF4 float4 of rings, then the warps' draws
+  extern __shared__ float4 glp_stage[];
+  Draw *const draws = reinterpret_cast<Draw *>(glp_stage + (size_t)kWarps * G0 * kGroupStrideF4) +
+                      warp * kDraws;
+  uint32_t drawn = 0;  // cycles of the sample whose draws the window has reached
 
   const uint32_t total = src.total();
   // The first sample of group slot g of global warp w is g * W + w, which
@@ -1266,6 +1322,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       if (ns < total) {
         src.locate(ns, c, s);
         e = 0;
+        drawn = 0;
         const GenParams &p = src.chunk(c);
         const uint32_t N = p.N;
         if (p.quad_in) {
@@ -1316,6 +1373,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       ngroups = ng.count;
       li = lane - gbase;
       exhausted = true;
+      drawn = max(e, 1u) - 1;  // the window lies elsewhere now
     }
     const bool active = s != kNone;
     const unsigned amask = __ballot_sync(FULL, active);
@@ -1332,28 +1390,56 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
     const uint32_t npos = Pc >> 1, r = li >> 1, ev = e + r;
     const bool lead_lane = (li & 1u) == 0;
     const uint32_t k = active ? min(npos, C + 1 - e) : 0u;
+    const bool scores = r < k && ev > 0;
+    // The words that the evaluation starts with, for the parents known so far.
+    if (active)
+      prefetch_first(p, q, lead_lane);
+    // Draws of cycle i at entry i mod 2 Pc of the group's window, made Pc cycles
+    // at a time, one a lane, when the window does not reach this round's last one
+    // (or another group of the warp draws and there is room): a chain makes each
+    // draw once, and the other rounds only read them.  The generators' chain of
+    // integer products stood in front of every round (with it and without the
+    // prefetches above: 3 x 3 0.241 and 0.214 ms, 3,001 x 4,000 from codes 4.52
+    // and 4.45, 2,000 x 8,192 5.72 and 5.58).
+    Draw *const window = draws + 2 * gbase;
+    const uint32_t wmask = 2 * Pc - 1, next = max(e, 1u) - 1;  // the round's first cycle
+    if (__any_sync(FULL, active && drawn < min(C, e + k - 1))) {
+      if (active && drawn < C && drawn + Pc - next <= 2 * Pc) {
+        const uint32_t cyc = drawn + li;
+        if (cyc < C) {
+          Draw d;
+          if (p.tr_slot) {
+            d.slot = p.tr_slot[(size_t)s * C + cyc] & 3u;
+            d.u = p.tr_u[(size_t)s * C + cyc];
+          } else {
+            glp_mh_draw(p.seed, p.generation, s, cyc, &d.slot, &d.u);
+          }
+          d.hap = p.props ? __ldg(p.props + (size_t)cyc * N + s)
+                  : (p.kick_first && cyc == 0)
+                      ? glp_surrogate_ref(p.seed, p.generation, s, cyc, GLP_TAG_PROP, 2u * N, H,
+                                          p.nbr, p.klen)
+                      : glp_surrogate(p.seed, p.generation, s, cyc, GLP_TAG_PROP, p.samp_lo,
+                                      p.samp_hi, p.nbr, p.klen);
+          if (d.hap >= H) {
+            atomicOr(error, 1);
+            d.hap = 0;
+          }
+          window[cyc & wmask] = d;
+        }
+        drawn += Pc;
+      }
+      __syncwarp();
+    }
     uint32_t slot = 0, phap = 0;
     double u = 0.0;
     uint4 myq = q;
-    if (r < k && ev > 0) {
-      const uint32_t cyc = ev - 1;
-      if (p.tr_slot) {
-        slot = p.tr_slot[(size_t)s * C + cyc] & 3u;
-        u = p.tr_u[(size_t)s * C + cyc];
-      } else {
-        glp_mh_draw(p.seed, p.generation, s, cyc, &slot, &u);
-      }
-      phap = p.props ? __ldg(p.props + (size_t)cyc * N + s)
-             : (p.kick_first && cyc == 0)
-                 ? glp_surrogate_ref(p.seed, p.generation, s, cyc, GLP_TAG_PROP, 2u * N, H,
-                                     p.nbr, p.klen)
-                 : glp_surrogate(p.seed, p.generation, s, cyc, GLP_TAG_PROP, p.samp_lo,
-                                 p.samp_hi, p.nbr, p.klen);
-      if (phap >= H) {
-        atomicOr(error, 1);
-        phap = 0;
-      }
+    if (scores) {
+      const Draw d = window[(ev - 1) & wmask];
+      slot = d.slot;
+      phap = d.hap;
+      u = d.u;
       set_slot(myq, slot, phap);
+      prefetch_first(p, phap, lead_lane);
     }
     double L = 0.0;
     // When every lane of the warp scores a chunk of the same length, all
@@ -1470,9 +1556,10 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
 }
 
 // Dynamic shared memory of a generation kernel with P lanes per sample: one
-// staging ring (both directions) per group.
+// staging ring (both directions) per group, and the warps' draws.
 __host__ __device__ constexpr size_t stage_bytes(int P) {
-  return sizeof(float4) * (size_t)kWarps * (32 / P) * kGroupStrideF4;
+  return sizeof(float4) * (size_t)kWarps * (32 / P) * kGroupStrideF4 +
+         sizeof(Draw) * (size_t)kWarps * kDraws;
 }
 
 // One chunk per launch (the reference's RunHMMOnDevice granularity).  P lanes

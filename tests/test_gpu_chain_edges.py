@@ -1,0 +1,99 @@
+"""The generation kernel where its chains' bookkeeping and the sites above the
+last whole word can go wrong: cycle counts around the windows of draws (2 P
+cycles of a chain, made P at a time), groups of a warp that leave it at different
+times, every remainder of a word, and rescaling inside the remainder.
+
+Decisions, quadruples and words against the oracle, and against the narrowest
+speculation, exactly; log-likelihoods within 1e-5 of the oracle's (the
+reference's binary32 arithmetic, impute.cpp:327-376, rounds a site's products
+and sums about ten times, 6e-8 each; over S sites that grows as sqrt(S) against a
+log-likelihood that grows as S).
+"""
+import numpy as np
+import pytest
+
+from glphase_gb300 import native as nat
+from glphase_gb300.glpack import GLPack
+from glphase_gb300.hmmlike import HMMLikeCUDA
+from test_gpu_parity import REL_TOL, check_against_oracle, make_problem, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    d = HMMLikeCUDA(0)
+    yield d
+    d.cleanup()
+
+
+def at_width(dev, lanes, *args, **kw):
+    dev.set_lanes_per_sample(lanes)
+    try:
+        return run_gpu(dev, *args, **kw)
+    finally:
+        dev.set_lanes_per_sample(0)
+
+
+@pytest.mark.parametrize("C", [0, 1, 2, 7, 8, 9, 31, 32, 33, 65, 130])
+def test_windows_of_draws(dev, oracle_lib, C):
+    m, haps, quad, props = make_problem(N=37, S=70, C=C, seed=C + 1)
+    ref = at_width(dev, 1, m, haps, quad, props, 0.5, seed=9, gen=3)
+    check_against_oracle(oracle_lib, m, haps, quad, props, 0.5, ref, 9, 3, check_work=False)
+    for lanes in (2, 4, 8, 16, 32):
+        out = at_width(dev, lanes, m, haps, quad, props, 0.5, seed=9, gen=3)
+        for key in ("quad", "acc", "hnew", "like"):
+            assert np.array_equal(out[key], ref[key]), (lanes, key)
+        assert np.array_equal(out["evals"], ref["evals"], equal_nan=True), lanes
+
+
+@pytest.mark.parametrize("vq", [False, True])
+@pytest.mark.parametrize("first", [0, 64, 192])
+def test_every_remainder_of_a_word(dev, oracle_lib, first, vq):
+    O = oracle_lib
+    for left in [1, 2, 3, 4, 5, 7, 8, 9, 12, 31, 33, 40, 61, 62, 63]:
+        S = first + left
+        m, haps, quad, props = make_problem(N=9, S=S, C=9, seed=S)
+        if not vq:
+            out = run_gpu(dev, m, haps, quad, props, 1.0, seed=5, gen=2)
+            check_against_oracle(O, m, haps, quad, props, 1.0, out, 5, 2, check_work=False)
+            continue
+        gp = GLPack(m.t, np.random.default_rng(left))
+        packed, cb = gp.packed_gls(), gp.code_book()
+        dev.copy_code_book_to_device(cb)
+        dev.copy_packed_gls_to_device(packed)
+        out = run_gpu(dev, m, haps, quad, props, 1.0, seed=5, flags=nat.GLP_GEN_VQ)
+        pb = O.OracleProblem(haps, m.emit, m.t, m.tran, m.pc, 9, packed=packed, codebook=cb,
+                             emit_mode=O.EMIT_VQ)
+        tr = pb.trace(seed=5, generation=0)
+        for s in range(m.N):
+            like32, _, own, qf = O.replay_sample(pb, tr, s, quad, props, 1.0, out["acc"][s])
+            rel = np.abs(out["evals"][s] - like32) / np.abs(like32)
+            assert rel.max() <= REL_TOL, (S, s, rel.max())
+            assert np.array_equal(qf, out["quad"][:, s])
+
+
+@pytest.mark.parametrize("scale", [1e-3, 1e-8, 1e-12])
+def test_rescaling_inside_the_remainder(dev, oracle_lib, scale):
+    """Emissions that take the state below 2^-64 within a site, within four, and
+    over several fours, in some samples and not in others."""
+    m, haps, quad, props = make_problem(N=12, S=64 + 47, C=10, seed=21)
+    m.emit = m.emit.copy()
+    m.emit[::2, 70:100] *= np.float32(scale)
+    m.emit[1::4, 101] *= np.float32(scale)
+    pb = oracle_lib.OracleProblem(haps, m.emit, m.t, m.tran, m.pc, 10)
+    tr = pb.trace(seed=6, generation=1)
+    for lanes in (2, 8, 32):
+        out = at_width(dev, lanes, m, haps, quad, props, 1.0, seed=6, gen=1)
+        for s in range(m.N):
+            like32, like64, _, qf = oracle_lib.replay_sample(pb, tr, s, quad, props, 1.0,
+                                                             out["acc"][s])
+            # at 1e-12 the binary32 reference leaves its own range for some quadruples
+            # (0 times infinity: NaN); the binary64 one stands for it there
+            ok = np.isfinite(like32)
+            assert scale < 1e-8 or np.all(ok)
+            assert np.all(np.isfinite(like64))
+            for want, at in ((like64, slice(None)), (like32.astype(np.float64), ok)):
+                rel = np.abs(out["evals"][s][at] - want[at]) / np.abs(want[at])
+                assert rel.max() <= REL_TOL, (lanes, s, rel.max())
+            assert np.array_equal(qf, out["quad"][:, s])
