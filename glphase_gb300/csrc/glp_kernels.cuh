@@ -218,6 +218,12 @@ struct EmitF32 {
   __device__ __forceinline__ void ahead(uint32_t m) const {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(row + m));
   }
+  // the sites m .. m + 3, m a multiple of 4, from global memory
+  __device__ __forceinline__ void get4(uint32_t m, float4 (&e)[4]) const {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      e[j] = __ldg(row + m + j);
+  }
   // copy block t (sites 8t .. 8t+7) into a forward / backward slot
   template <int kMaxRows>
   __device__ __forceinline__ void stage(float4 *dst, uint32_t t, StageRows r) const {
@@ -247,6 +253,12 @@ struct EmitVQ {
     table = tab;
   }
   __device__ __forceinline__ void ahead(uint32_t) const {}
+  __device__ __forceinline__ void get4(uint32_t m, float4 (&e)[4]) const {
+    const uint32_t w = __ldg(col + (size_t)(m >> 3) * stride) << (4u * (m & 4u));
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+      e[j] = table[(w >> (28u - 4u * j)) & 15u];
+  }
   __device__ __forceinline__ float4 get1(uint32_t m) const {
     const uint32_t w = __ldg(col + (size_t)(m >> 3) * stride);
     return table[(w >> (28u - 4u * (m & 7u))) & 15u];
@@ -330,6 +342,19 @@ __device__ __forceinline__ void fwd_step(FState &f, const float4 t, float s00, f
     fstate_scale(f, kHuge);
     f.k -= 64;
   }
+}
+
+// fwd_step's products and sums in its order, two at a time, without its
+// rescaling; returns the state's sum.
+__device__ __forceinline__ float fwd_step_free(FState &f, const float4 t, float2 sx, float2 sy) {
+  const float2 tx = make_float2(t.x, t.x), ty = make_float2(t.y, t.y),
+               tz = make_float2(t.z, t.z), c = make_float2(f.P.y, f.P.x);
+  const float2 bx = __ffma2_rn(f.Y, tz, __ffma2_rn(c, ty, __fmul2_rn(f.X, tx)));
+  const float2 by = __ffma2_rn(f.X, tz, __ffma2_rn(c, ty, __fmul2_rn(f.Y, tx)));
+  f.X = __fmul2_rn(bx, sx);
+  f.Y = __fmul2_rn(by, sy);
+  f.P = __fadd2_rn(f.X, f.Y);
+  return f.P.x + f.P.y;
 }
 
 // The same step without rescaling, in a shared-term form of T: with
@@ -565,38 +590,45 @@ __device__ __forceinline__ double eval_pair(const GenParams &p, const E &em, uin
   issue(0, 0);
   issue(0, 1);
   if (bwd && (S & 63u)) {
-    // the sites of the partial top word, four at a time with the next four's
-    // rows already on their way
+    // the sites of the partial top word: four at a time, their rows loaded
+    // together and the test for the rescaling of fwd_step made once for the four;
+    // where it would have rescaled, and for the sites above the last whole four,
+    // site by site.  A lone warp takes 83 cycles a site, and 49 in a whole word
+    // (site by site 120; a generation of 60 x 1,000 0.654 and 0.617 ms).  Two
+    // fours in registers at once were slower: 168 registers, with spills.
     const Parents pw = load_parents(p.haps, wn, q, nw);
-    const int lo = (int)(nw * 64);
-    float4 e[4], t[4];
-    auto load = [&](int m0) {  // sites m0, m0 - 1, ...
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t m = (uint32_t)max(m0 - k, lo);
-        e[k] = em.get1(m);
-        t[k] = __ldg(tran4 + m + 1);
-      }
-    };
-    load((int)S - 1);
 #pragma unroll 1
-    for (int m0 = (int)S - 1; m0 >= lo; m0 -= 4) {
-      float4 ce[4], ct[4];
+    for (int lo = (int)((S - 1) & ~3u), n = (int)S - lo; lo >= (int)(nw * 64); lo -= 4, n = 4) {
+      const uint32_t sh = (uint32_t)lo & 63u;
+      float low = 0.0f;
+      FState y = x;
+      if (n == 4) {
+        const Bits32 bw = {(uint32_t)(pw.f0 >> sh), (uint32_t)(pw.f1 >> sh),
+                           (uint32_t)(pw.m0 >> sh), (uint32_t)(pw.m1 >> sh)};
+        float4 e[4], t[4];
+        em.get4((uint32_t)lo, e);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        ce[k] = e[k];
-        ct[k] = t[k];
+        for (int j = 0; j < 4; ++j)
+          t[j] = __ldg(tran4 + lo + 1 + j);
+        low = kHuge;
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+          float2 sx, sy;
+          site_emission(e[j], bw, j, sx, sy);
+          low = fminf(low, fwd_step_free(y, t[j], sx, sy));
+        }
       }
-      load(m0 - 4);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (m0 - k < lo)
-          break;
-        const uint32_t j = (uint32_t)(m0 - k) & 63u;
-        float s00, s01, s10, s11;
-        select4(ce[k], (pw.f0 >> j) & 1, (pw.f1 >> j) & 1, (pw.m0 >> j) & 1, (pw.m1 >> j) & 1,
-                s00, s01, s10, s11);
-        fwd_step(x, ct[k], s00, s01, s10, s11);
+      if (low >= kTiny) {
+        x = y;
+      } else {
+#pragma unroll 1
+        for (int j = n - 1; j >= 0; --j) {
+          const uint32_t i = sh + (uint32_t)j;
+          float s00, s01, s10, s11;
+          select4(em.get1((uint32_t)(lo + j)), (pw.f0 >> i) & 1, (pw.f1 >> i) & 1,
+                  (pw.m0 >> i) & 1, (pw.m1 >> i) & 1, s00, s01, s10, s11);
+          fwd_step(x, __ldg(tran4 + lo + j + 1), s00, s01, s10, s11);
+        }
       }
     }
     fwd_renorm(x);
