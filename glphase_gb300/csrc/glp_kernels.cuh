@@ -517,19 +517,50 @@ __device__ __noinline__ double like_forward(const uint64_t *__restrict__ haps, u
   return log(sum) + (double)f.k * 0.69314718055994530942;
 }
 
-// ln(dot) + k ln 2 for a positive dot product: the binary64 exponent of dot
-// joins k exactly, and the logarithm of its mantissa m in [1, 2) is taken in
-// binary32 (absolute error below 3e-7, against log-likelihoods of order
-// -S), so the FP64 pipe only adds the two parts.  Dots far below the block
-// range (never in the blocked pass) take the binary64 logarithm.
-__device__ __forceinline__ double log_scaled(double dot, int k) {
+// a + b = s + err exactly.
+__device__ __forceinline__ float two_sum(float a, float b, float &err) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+  return s;
+}
+
+// ln(x . y) + k ln 2 over the four states, in natural log and binary64.  The
+// exponent of the product joins k exactly, and the logarithm of its mantissa in
+// [1, 2) is taken in binary32 (absolute error below 3e-7, against
+// log-likelihoods of order -S), so binary64 only adds the two parts: its pipe
+// takes an instruction of a warp in 16 cycles.  For the same reason the product
+// itself is a pair of floats: the four products exact as a float and an error,
+// their sums too, so that the mantissa is rounded once, from a value good to 46
+// bits (in binary64 the products, sums and conversions took 820 cycles of a round
+// that has 3,600 beside its sites, now 70; a lone warp's round over 64 sites, with
+// the accept rule in binary32 as well, 3.64 and 3.18 us, over 1,024 15.7 and 15.3).
+// Products outside the range where the errors are floats (a blocked pass's never
+// are) and invalid ones go through binary64.
+__device__ __forceinline__ double log_dot(float2 xX, float2 xY, float2 yX, float2 yY, int k) {
   constexpr double kLn2 = 0.69314718055994530942;
-  if (!(dot > 0x1p-1000))
-    return log(dot) + (double)k * kLn2;
-  const long long bits = __double_as_longlong(dot);
-  const int e = (int)((bits >> 52) & 0x7ff) - 1023;
-  const double m = __longlong_as_double((bits & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
-  return (double)logf((float)m) + (double)(e + k) * kLn2;
+  const float p0 = __fmul_rn(xX.x, yX.x), p1 = __fmul_rn(xX.y, yX.y),
+              p2 = __fmul_rn(xY.y, yY.y), p3 = __fmul_rn(xY.x, yY.x);
+  float d0, d1, d2;
+  const float s0 = two_sum(p0, p1, d0), s1 = two_sum(p2, p3, d1), s = two_sum(s0, s1, d2);
+  const float r0 = __fadd_rn(fmaf(xX.x, yX.x, -p0), fmaf(xX.y, yX.y, -p1));
+  const float r1 = __fadd_rn(fmaf(xY.y, yY.y, -p2), fmaf(xY.x, yY.x, -p3));
+  const float hi = __fadd_rn(s, __fadd_rn(__fadd_rn(d0, d1), __fadd_rn(d2, __fadd_rn(r0, r1))));
+  float m;
+  int e;
+  if (hi >= 0x1p-60f && hi < 0x1p127f) {
+    const uint32_t bits = __float_as_uint(hi);
+    e = (int)(bits >> 23) - 127;
+    m = __uint_as_float((bits & 0x007fffffu) | 0x3f800000u);
+  } else {
+    const double dot = (double)xX.x * (double)yX.x + (double)xX.y * (double)yX.y +
+                       (double)xY.y * (double)yY.y + (double)xY.x * (double)yY.x;
+    if (!(dot > 0x1p-1000))
+      return log(dot) + (double)k * kLn2;
+    const long long bits = __double_as_longlong(dot);
+    e = (int)((bits >> 52) & 0x7ff) - 1023;
+    m = (float)__longlong_as_double((bits & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
+  }
+  return (double)logf(m) + (double)(e + k) * kLn2;
 }
 
 // Log-likelihood (natural log, binary64) of quadruple q, scored by a lane
@@ -685,14 +716,14 @@ __device__ __forceinline__ double eval_pair(const GenParams &p, const E &em, uin
   }
   if (bwd)  // beta_{64 wf - 1} = T_{64 wf} v_{64 wf} (row S is the identity)
     apply_tran(x, __ldg(tran4 + 64 * (size_t)wf));
-  const float y00 = __shfl_xor_sync(gmask, x.X.x, 1), y01 = __shfl_xor_sync(gmask, x.X.y, 1),
-              y10 = __shfl_xor_sync(gmask, x.Y.y, 1), y11 = __shfl_xor_sync(gmask, x.Y.x, 1);
+  // alpha . beta on both lanes: the same products, and sums of the same pairs
+  const float2 yX = make_float2(__shfl_xor_sync(gmask, x.X.x, 1),
+                                __shfl_xor_sync(gmask, x.X.y, 1)),
+               yY = make_float2(__shfl_xor_sync(gmask, x.Y.x, 1),
+                                __shfl_xor_sync(gmask, x.Y.y, 1));
   const int yk = __shfl_xor_sync(gmask, x.k, 1);
   const uint32_t bad = (eacc | __shfl_xor_sync(gmask, eacc, 1)) & ~127u;
-  // alpha . beta on both lanes: the same exact products in the same order
-  const double dot = (double)x.X.x * (double)y00 + (double)x.X.y * (double)y01 +
-                     (double)x.Y.y * (double)y10 + (double)x.Y.x * (double)y11;
-  double L = log_scaled(dot, x.k + yk);
+  double L = log_dot(x.X, x.Y, yX, yY, x.k + yk);
   if (__any_sync(gmask, bad != 0u)) {
     double Lf = L;
     if (bad && !bwd) {
@@ -1139,8 +1170,8 @@ __device__ __forceinline__ void set_slot(uint4 &q, uint32_t r, uint32_t v) {
 // One cycle's draws: the accept uniform, the proposed haplotype and the slot that
 // it replaces.
 struct __align__(16) Draw {
-  double u;
-  uint32_t hap, slot;
+  float u;  // accept_bound
+  uint32_t hap, slot, unused;
 };
 constexpr uint32_t kDraws = 64;  // a warp's windows: two per lane of each group
 
@@ -1294,13 +1325,18 @@ __device__ __forceinline__ LaneGroups regroup(uint32_t lane, uint32_t na) {
 // exponential is taken in binary32 (relative error below 3e-6: a decision can
 // differ from the binary64 one only where |d - ln u| < 3e-6); below -37 it
 // is under 2^-53, so only u = 0 accepts, as in binary64.
-__device__ __forceinline__ bool mh_accept(double prop, double curr, float pen, double u) {
+// u comes as accept_bound(u), made once with the draw: f > u for a float f exactly
+// when f > bound, and u = 0 is the bound -0.
+__device__ __forceinline__ float accept_bound(double u) {
+  return u == 0.0 ? -0.0f : __double2float_rd(u);
+}
+__device__ __forceinline__ bool mh_accept(double prop, double curr, double pen, float bound) {
   if (prop >= curr)
     return true;
-  const double d = (prop - curr) * (double)pen;
+  const double d = (prop - curr) * pen;
   if (d > -37.0)
-    return u < (double)expf((float)d);
-  return u == 0.0 && u < exp(d);
+    return expf((float)d) > bound;
+  return __float_as_uint(bound) == 0x80000000u && exp(d) > 0.0;
 }
 
 template <int P, class E, class Src, int kSub = 1>
@@ -1440,12 +1476,14 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
         const uint32_t cyc = drawn + li;
         if (cyc < C) {
           Draw d;
+          double u;
           if (p.tr_slot) {
             d.slot = p.tr_slot[(size_t)s * C + cyc] & 3u;
-            d.u = p.tr_u[(size_t)s * C + cyc];
+            u = p.tr_u[(size_t)s * C + cyc];
           } else {
-            glp_mh_draw(p.seed, p.generation, s, cyc, &d.slot, &d.u);
+            glp_mh_draw(p.seed, p.generation, s, cyc, &d.slot, &u);
           }
+          d.u = accept_bound(u);
           d.hap = p.props ? __ldg(p.props + (size_t)cyc * N + s)
                   : (p.kick_first && cyc == 0)
                       ? glp_surrogate_ref(p.seed, p.generation, s, cyc, GLP_TAG_PROP, 2u * N, H,
@@ -1463,7 +1501,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       __syncwarp();
     }
     uint32_t slot = 0, phap = 0;
-    double u = 0.0;
+    float u = 0.0f;
     uint4 myq = q;
     if (scores) {
       const Draw d = window[(ev - 1) & wmask];
@@ -1502,9 +1540,10 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
     // starting one, so each position tests its own proposal against it in
     // parallel and the first accepting position (in chain order) wins: the
     // same decisions as the sequential loop.  The even lanes vote.
+    const double pen = (double)p.pen;
     const double L0 = __shfl_sync(FULL, L, gbase);
     const double curr0 = (e == 0) ? L0 : curr;
-    const bool acc = lead_lane && r < k && ev > 0 && mh_accept(L, curr0, p.pen, u);
+    const bool acc = lead_lane && r < k && ev > 0 && mh_accept(L, curr0, pen, u);
     const unsigned gmask = (Pc == 32) ? FULL : (((1u << Pc) - 1u) << gbase);
     const unsigned abal = __ballot_sync(FULL, acc) & gmask;
     const uint32_t srcl = abal ? (uint32_t)(__ffs(abal) - 1) : gbase;
@@ -1520,20 +1559,20 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
     uint32_t last = first_acc, hap = pha;
     uint32_t more = 0;  // accepted positions after first_acc
     double cur = La;
-    bool go = active && abal != 0;
-    for (uint32_t d = 1; d < 16u; ++d) {
-      const uint32_t r2 = first_acc + d;
-      go = go && r2 < k;
-      const uint32_t from = gbase + 2u * (go ? r2 : 0u);
-      const uint32_t sl_r = __shfl_sync(FULL, slot, from);
-      go = go && sl_r == sla;
-      if (!__any_sync(FULL, go))
-        break;
-      const double L_r = __shfl_sync(FULL, L, from), u_r = __shfl_sync(FULL, u, from);
+    const unsigned others = __ballot_sync(FULL, !(scores && lead_lane && slot == sla)) &
+                            0x55555555u & gmask;
+    // pairs after the first accepting one up to the next that replaces another slot
+    const unsigned after = others & ~((2u << srcl) - 1u);
+    const uint32_t stop =
+        !abal ? 0u : after ? ((uint32_t)__ffs(after) - 1 - gbase) >> 1 : npos;
+    for (uint32_t r2 = first_acc + 1; __any_sync(FULL, r2 < stop); ++r2) {
+      const uint32_t from = gbase + 2u * (r2 < stop ? r2 : 0u);
+      const double L_r = __shfl_sync(FULL, L, from);
+      const float u_r = __shfl_sync(FULL, u, from);
       const uint32_t ph_r = __shfl_sync(FULL, phap, from);
-      if (go) {
+      if (r2 < stop) {
         last = r2;
-        if (mh_accept(L_r, cur, p.pen, u_r)) {
+        if (mh_accept(L_r, cur, pen, u_r)) {
           cur = L_r;
           hap = ph_r;
           more |= 1u << r2;

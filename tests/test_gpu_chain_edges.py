@@ -97,3 +97,31 @@ def test_rescaling_inside_the_remainder(dev, oracle_lib, scale):
                 rel = np.abs(out["evals"][s][at] - want[at]) / np.abs(want[at])
                 assert rel.max() <= REL_TOL, (lanes, s, rel.max())
             assert np.array_equal(qf, out["quad"][:, s])
+
+
+def test_uniforms_at_the_ends_of_their_range(dev):
+    """The accept test takes the uniform rounded down to a float: traced uniforms
+    that are 0, that lie between floats, that no float of the rule's range reaches,
+    and next to 1, against the rule in binary64 (prop >= curr, or u < exp(d) for d =
+    (prop - curr) pen above -37, or u = 0 below it), on either side of -37."""
+    m, haps, quad, props = make_problem(N=16, S=150, C=24, seed=33)
+    rng = np.random.default_rng(5)
+    ends = np.array([0.0, 2.0**-53, 1e-300, 2.0**-40 + 2.0**-53, 0.5 - 2.0**-53, 0.5,
+                     0.5 + 2.0**-53, 1 - 2.0**-53])
+    u = ends[rng.integers(0, len(ends), (16, 24))]
+    trace = (rng.integers(0, 4, (16, 24)).astype(np.uint8), u,
+             rng.random((16, 150)).astype(np.float32))
+    accepted = []
+    for pen in (0.01, 1.0, 30.0):
+        out = run_gpu(dev, m, haps, quad, props, pen, trace=trace)
+        for s in range(16):
+            curr = out["evals"][s, 0]
+            for c in range(24):
+                prop = out["evals"][s, c + 1]
+                d = (prop - curr) * pen
+                bound = 1.0 if d >= 0 else np.exp(d) if d > -37 or u[s, c] == 0 else 0.0
+                if abs(bound - u[s, c]) > 3e-6 * bound:  # the exponential is binary32
+                    assert out["acc"][s, c] == (d >= 0 or u[s, c] < bound), (pen, s, c)
+                curr = prop if out["acc"][s, c] else curr
+        accepted.append(out["acc"][u == 0.0].mean())
+    assert accepted[0] == 1.0 and accepted[2] < 1.0
