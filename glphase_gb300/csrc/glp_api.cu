@@ -443,21 +443,39 @@ double resident_threads(Fn fn, uint32_t P, int sms) {
   return (double)occ * glp::kThreads * sms;
 }
 
+// Acceptance rate of a generation that nothing is known of.
+constexpr double kUsualRate = 0.12;
+
+// The positions that a chain goes on a round, on average: the chances that the
+// scored nodes of its speculation tree are reached.
+double steps_a_round(double a, uint32_t P) {
+  static constexpr glp::SpecTrees trees = glp::make_spec_trees();
+  const int rate = glp::kSpecTree((int)P) ? (int)(a * 16.0 + 0.5) : 0;
+  const glp::SpecNode *t = trees.node[std::min(rate, glp::kSpecRates - 1)];
+  double sum = 0.0;
+  for (uint32_t i = 0; i < P / 2; ++i) {
+    const int accepted = __builtin_popcount(t[i].accept),
+              refused = __builtin_popcount(t[i].path) - accepted;
+    sum += std::pow(a, accepted) * std::pow(1.0 - a, refused);
+  }
+  return sum;
+}
+
 // Speculation width for N samples at acceptance rate a.  A generation lasts as
 // long as its longest chain while every sample has a group of its own, so the
-// rule compares, for each width, the rounds of a chain that accepts more often
-// than the average, 1 / consumed(P) for consumed = (1 - (1-a')^n) / a', n = P/2
-// positions a round, a' = a + min(a, 0.12), times what a warp's round costs at
-// the warps a scheduler holds.  Measured (1,024 sites, a = 0.12, times of a
-// generation kernel relative to one warp a scheduler): 1.44 at two, 2.0 at three,
-// beyond that in proportion (whole blocks of four warps, so the steps are at
-// multiples of the SM count).  Narrow groups stage more rows a lane: 1.12 at 4
-// lanes (1.35 when rows stream from memory), 2.2 at 2 lanes; on VQ codes, whose
-// table reads conflict more in a wide group, 1.15 at 32.  The widths this picks,
-// against 8 and 16 lanes: 256 samples 32 lanes 0.36 ms (0.56, 0.40), 1,000
-// samples 16 lanes 0.43 (0.56, 0.43; 32 lanes 0.52), 2,000 x 8,192 from a panel 16
-// lanes 4.25 (5.15, 4.25; 32 lanes 6.07), 10,000 samples 8 lanes 1.67 (1.67, 2.03).
-constexpr double kLaneRoundCost[6] = {0.0, 2.2, 1.12, 1.0, 1.0, 1.0};
+// rule compares, for each width, the rounds of a chain whose rate is off the
+// average, a or a' = a + min(a, 0.12), whichever goes on fewer positions a round,
+// times what a warp's round costs at the warps a scheduler holds.  Measured
+// (1,024 sites, a = 0.12, times of a generation kernel relative to one warp a
+// scheduler): 1.44 at two, 2.0 at three, beyond that in proportion (whole blocks of
+// four warps, so the steps are at multiples of the SM count).  Narrow groups stage
+// more rows a lane: 1.16 at 4 lanes, 2.2 at 2 lanes; at 8 lanes 1.05; on VQ codes,
+// whose table reads conflict more in a wide group, 1.15 at 32.  The widths this
+// picks, against others: 256 samples 32 lanes 0.36 ms (8: 0.55, 16: 0.42), 1,000
+// samples 16 lanes 0.55 (0.76; 32: 0.64), 1,500 x 2,048 8 lanes 1.07 (16: 1.14),
+// 2,500 x 2,048 16 lanes 1.42 (8: 1.51), 3,001 x 4,000 from codes 16 lanes 3.47 (8:
+// 3.68; 32: 4.52), 10,000 samples 8 lanes 2.05 (16: 2.49).
+constexpr double kLaneRoundCost[6] = {0.0, 2.2, 1.16, 1.05, 1.0, 1.0};
 
 template <class FnOf>
 uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
@@ -478,8 +496,7 @@ uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
     if (res[i] <= 0)
       continue;
     const uint32_t P = 1u << i;
-    const double n = P / 2;
-    const double consumed = (1.0 - std::pow(1.0 - as, n)) / as;
+    const double consumed = std::min(steps_a_round(a, P), steps_a_round(as, P));
     const uint64_t per_block = (uint64_t)glp::kThreads / P;
     const uint64_t blocks = (N + per_block - 1) / per_block;
     // blocks an SM holds at a time, and for one warp a scheduler in each
@@ -499,14 +516,18 @@ uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
   return best;
 }
 
+// The acceptance rate that a launch with penalty pen is expected to have: the last
+// generation's at that penalty.
+double expected_rate(const glp_ctx *c, float pen) {
+  return (c->last_accept < 0 || pen != c->accept_pen) ? kUsualRate
+                                                      : std::max(c->last_accept, 1e-3);
+}
+
 uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen) {
   if (c->lanes)
     return c->lanes;
-  const double a = (c->last_accept < 0 || pen != c->accept_pen)
-                       ? 0.12
-                       : std::max(c->last_accept, 1e-3);
   return pick_lanes(
-      a, N, c->sms, vq,
+      expected_rate(c, pen), N, c->sms, vq,
       [&](uint32_t P) {
         Shape sh;
         sh.P = P;
@@ -623,6 +644,7 @@ int make_params(glp_ctx *c, glp_problem *pb, const glp_generation_args *a,
   p->burnin = a->burnin;
   p->kick = a->kick_start ? 1u : 0u;
   p->kick_first = kick_first ? 1u : 0u;
+  p->rate = (float)expected_rate(c, a->pen);
   return GLP_OK;
 }
 
@@ -2094,13 +2116,14 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   p.seed = a->seed;
   p.generation = a->generation;
   p.do_work = work ? 1u : 0u;
+  p.rate = (float)kUsualRate;
 
   // speculation width for an acceptance rate of about 0.12 (the rule of
   // choose_lanes without a context's history), from the resident threads
   // measured at set-up
   bool known = true;
   const uint32_t P = pick_lanes(
-      0.12, N, sms, false,
+      kUsualRate, N, sms, false,
       [](uint32_t w) {
         Shape s1;
         s1.P = w;

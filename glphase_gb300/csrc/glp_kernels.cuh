@@ -105,6 +105,7 @@ struct GenParams {
   uint32_t generation;
   uint32_t do_work;
   uint32_t stream;  // 1: emission rows are asked for ahead (mark_stream)
+  float rate;       // acceptance rate that a chain's speculation starts from
 };
 
 // ---------------------------------------------------------------------------
@@ -1167,6 +1168,73 @@ __device__ __forceinline__ void set_slot(uint4 &q, uint32_t r, uint32_t v) {
     q.w = v;
 }
 
+// Speculation trees.  A round of n evaluations scores n nodes of the tree of a
+// chain's possible decisions: the root is the chain's next position, a node's two
+// children the position after it with the node's proposal refused or accepted.  At
+// an acceptance rate a the n nodes most likely to be reached -- a node's chance is
+// the product of a or 1 - a along its path -- are a line of refusals for a small
+// a, a line of acceptances for a near 1, and branched between: with 16 nodes the
+// chain goes on 7.3 positions a round at a = 0.12, 4.3 at 0.35 (2.9 on a line of
+// refusals), 12 at 0.96 (1.0).  The nodes are numbered in the order in which a
+// greedy search takes them, so that a tree's first n nodes are the tree for n.
+// Which nodes are scored changes no result: each is the evaluation that the chain
+// would make there, and the chain takes those on its way.  A generation of few
+// chains lasts as long as the chain that accepts most often: 3 x 3 0.183 and 0.108
+// ms, 256 x 1,024 0.559 and 0.532, 30 generations of 60 x 1,000 17.6 and 16.7.
+struct SpecNode {
+  uint32_t path;    // its ancestors: bit 2 i for node i
+  uint32_t accept;  // those of them whose proposal it has accepted
+  uint32_t desc;    // [0, 4) depth, [4, 8) the last of those, [8, 24) their depths
+};
+constexpr int kSpecNodes = 16;  // a warp's lane pairs
+constexpr int kSpecRates = 17;  // tree i is made for a = i / 16
+struct SpecTrees {
+  SpecNode node[kSpecRates][kSpecNodes];
+};
+constexpr SpecTrees make_spec_trees() {
+  SpecTrees t{};
+  for (int i = 0; i < kSpecRates; ++i) {
+    const double a = i == 0 ? 0.02 : i == 16 ? 0.98 : i / 16.0;
+    double prob[kSpecNodes] = {};
+    bool child[kSpecNodes][2] = {};
+    prob[0] = 1.0;
+    for (int n = 1; n < kSpecNodes; ++n) {
+      int from = 0, dec = 0;
+      double best = -1.0;
+      for (int v = 0; v < n; ++v)
+        for (int d = 0; d < 2; ++d) {
+          // beside a refusal's child a quarter of an acceptance's is not needed: the
+          // next position replaces the same slot (generation_body)
+          const double pr = prob[v] * (d ? a : 1 - a) * (d && child[v][0] ? 0.75 : 1.0);
+          if (!child[v][d] && pr > best) {
+            best = pr;
+            from = v;
+            dec = d;
+          }
+        }
+      child[from][dec] = true;
+      prob[n] = prob[from] * (dec ? a : 1 - a);
+      const SpecNode &pa = t.node[i][from];
+      const uint32_t depth = pa.desc & 15u;
+      SpecNode &nd = t.node[i][n];
+      nd.path = pa.path | (1u << (2 * from));
+      nd.accept = pa.accept | (dec ? 1u << (2 * from) : 0u);
+      nd.desc = (depth + 1) | (dec ? (uint32_t)from << 4 : pa.desc & 0xf0u) |
+                (pa.desc & 0xffff00u) | (dec ? 0x100u << depth : 0u);
+    }
+  }
+  return t;
+}
+static __device__ const SpecTrees kSpecTrees = make_spec_trees();
+// A chain's rate moves with weight 1 / 24 a cycle from the generation's (with 1 / 6,
+// chains of 10,000 samples took 0.8 % more rounds, 3 x 3 sites 1 % fewer).
+constexpr float kRateWeight = 24.0f;
+// Kernels that start with 16 lanes a sample or more take trees.  Below, four nodes
+// or fewer differ from the line of refusals only where a chain accepts more than 40
+// % of its proposals, and the kernel without them is the faster one (3,001 x 4,000
+// from codes at 8 lanes 4.39 and 4.46 ms, 10,000 x 4,096 7.36 and 7.40).
+constexpr bool kSpecTree(int P) { return P >= 16; }
+
 // One cycle's draws: the accept uniform, the proposed haplotype and the slot that
 // it replaces.
 struct __align__(16) Draw {
@@ -1346,6 +1414,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
   static_assert(P == 2 || P == 4 || P == 8 || P == 16 || P == 32, "P");
   constexpr unsigned FULL = 0xffffffffu;
   constexpr uint32_t G0 = 32u / P;  // group slots (staging rings) per warp
+  constexpr bool kTree = kSpecTree(P);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // current partition of the warp's lanes
   uint32_t Pc = P, gbase = lane - lane % P, gidx = lane / P, ngroups = G0;
@@ -1368,6 +1437,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
   uint32_t c = 0, s = kNone, e = 0;
   uint4 q = make_uint4(0, 0, 0, 0);
   double curr = 0.0;
+  float rate = 0.0f;  // the chain's acceptance rate so far
   bool exhausted = false;
   unsigned long long n_evals = 0, n_rounds = 0, n_acc = 0;
   unsigned long long n_warp_rounds = 0, n_active_lanes = 0;
@@ -1393,6 +1463,8 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
         drawn = 0;
         const GenParams &p = src.chunk(c);
         const uint32_t N = p.N;
+        if (kTree)
+          rate = p.rate;
         if (p.quad_in) {
           q = make_uint4(__ldg(p.quad_in + s), __ldg(p.quad_in + N + s),
                          __ldg(p.quad_in + 2 * (size_t)N + s),
@@ -1435,6 +1507,8 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       q.z = __shfl_sync(FULL, q.z, from);
       q.w = __shfl_sync(FULL, q.w, from);
       curr = __shfl_sync(FULL, curr, from);
+      if (kTree)
+        rate = __shfl_sync(FULL, rate, from);
       Pc = ng.size;
       gbase = ng.base;
       gidx = ng.index;
@@ -1452,13 +1526,25 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
 
     const GenParams &p = src.chunk(c);
     const uint32_t N = p.N, C = p.C, H = p.H;
-    // One speculative round: the group's Pc/2 lane pairs score the next Pc/2
-    // positions of the chain, pair r = li/2 position e + r (its even lane the
-    // forward half, its odd lane the backward half of the evaluation).
-    const uint32_t npos = Pc >> 1, r = li >> 1, ev = e + r;
+    // One speculative round: the group's Pc/2 lane pairs score the first Pc/2
+    // nodes of the speculation tree for the chain's rate, pair r = li/2 node r, at
+    // position e + depth (its even lane the forward half, its odd lane the
+    // backward half of the evaluation).  Position 0 is the quadruple that the
+    // chain starts with, neither accepted nor refused: the round that begins there
+    // takes the line of refusals, as every round of a narrow kernel does.
+    const uint32_t npos = Pc >> 1, r = li >> 1;
+    uint32_t path = 0, wants = 0, desc = r;
+    if (kTree) {
+      const uint32_t tree = e == 0 ? 0u : (uint32_t)(rate * 16.0f + 0.5f);
+      const SpecNode *const node = &kSpecTrees.node[min(tree, kSpecRates - 1u)][r];
+      path = __ldg(&node->path);
+      wants = __ldg(&node->accept);
+      desc = __ldg(&node->desc);
+    }
+    const uint32_t depth = desc & 15u, taken = desc >> 8, ev = e + depth;
     const bool lead_lane = (li & 1u) == 0;
-    const uint32_t k = active ? min(npos, C + 1 - e) : 0u;
-    const bool scores = r < k && ev > 0;
+    const uint32_t k = active ? min(npos, C + 1 - e) : 0u;  // positions, at most
+    const bool valid = depth < k, scores = valid && ev > 0;
     // The words that the evaluation starts with, for the parents known so far.
     if (active)
       prefetch_first(p, q, lead_lane);
@@ -1504,6 +1590,12 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
     float u = 0.0f;
     uint4 myq = q;
     if (scores) {
+      if (kTree)
+        for (uint32_t m = taken; m != 0u; m &= m - 1u) {  // accepted on its path
+          const Draw d = window[(e + (uint32_t)__ffs(m) - 2) & wmask];
+          set_slot(myq, d.slot, d.hap);
+          prefetch_first(p, d.hap, lead_lane);
+        }
       const Draw d = window[(ev - 1) & wmask];
       slot = d.slot;
       phap = d.hap;
@@ -1531,74 +1623,155 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
                                                                        gm)
               : eval_pair<(P >= 8 ? 1 : 8 / P), E, kSub, false, P == 8>(p, em, myq, ring, li,
                                                                         Pc, gm);
-      if (r >= k)
+      if (!valid)
         L = 0.0;
     }
-    // The accept rule of MHSampler.hpp:86-93 in chain order.  Every
-    // evaluation of the round was built on the round's starting state, and
-    // until the first acceptance the chain's current likelihood is the
-    // starting one, so each position tests its own proposal against it in
-    // parallel and the first accepting position (in chain order) wins: the
-    // same decisions as the sequential loop.  The even lanes vote.
     const double pen = (double)p.pen;
     const double L0 = __shfl_sync(FULL, L, gbase);
     const double curr0 = (e == 0) ? L0 : curr;
-    const bool acc = lead_lane && r < k && ev > 0 && mh_accept(L, curr0, pen, u);
-    const unsigned gmask = (Pc == 32) ? FULL : (((1u << Pc) - 1u) << gbase);
-    const unsigned abal = __ballot_sync(FULL, acc) & gmask;
-    const uint32_t srcl = abal ? (uint32_t)(__ffs(abal) - 1) : gbase;
-    const uint32_t first_acc = abal ? (srcl - gbase) >> 1 : npos;
-    const double La = __shfl_sync(FULL, L, srcl);
-    const uint32_t sla = __shfl_sync(FULL, slot, srcl);
-    const uint32_t pha = __shfl_sync(FULL, phap, srcl);
-    // The positions after the first acceptance that replace the same slot
-    // scored exactly the quadruple the sequential chain builds there (it
-    // differs from the round's start only in that slot), so the chain goes on
-    // through them -- each tested against the likelihood accepted last --
-    // up to the first position that replaces another slot.
-    uint32_t last = first_acc, hap = pha;
-    uint32_t more = 0;  // accepted positions after first_acc
-    double cur = La;
-    const unsigned others = __ballot_sync(FULL, !(scores && lead_lane && slot == sla)) &
-                            0x55555555u & gmask;
-    // pairs after the first accepting one up to the next that replaces another slot
-    const unsigned after = others & ~((2u << srcl) - 1u);
-    const uint32_t stop =
-        !abal ? 0u : after ? ((uint32_t)__ffs(after) - 1 - gbase) >> 1 : npos;
-    for (uint32_t r2 = first_acc + 1; __any_sync(FULL, r2 < stop); ++r2) {
-      const uint32_t from = gbase + 2u * (r2 < stop ? r2 : 0u);
-      const double L_r = __shfl_sync(FULL, L, from);
-      const float u_r = __shfl_sync(FULL, u, from);
-      const uint32_t ph_r = __shfl_sync(FULL, phap, from);
-      if (r2 < stop) {
-        last = r2;
-        if (mh_accept(L_r, cur, pen, u_r)) {
-          cur = L_r;
-          hap = ph_r;
-          more |= 1u << r2;
+    if constexpr (kTree) {
+      // The accept rule of MHSampler.hpp:86-93.  Every node's test is made at once,
+      // against the likelihood that is current on its path: that of the last node
+      // accepted there, or the round's first.  The chain reaches the nodes whose
+      // ancestors decided as their paths say, the deepest of them the last in number:
+      // the same decisions as the sequential loop.  The even lanes vote.
+      const double Lup = __shfl_sync(FULL, L, gbase + 2u * ((desc >> 4) & 15u));
+      const bool acc = lead_lane && scores && mh_accept(L, taken ? Lup : curr0, pen, u);
+      const uint32_t gones = Pc == 32 ? FULL : (1u << Pc) - 1u;
+      const unsigned abal = (__ballot_sync(FULL, acc) >> gbase) & gones;
+      const bool hit = lead_lane && valid && ((abal ^ wants) & path) == 0u;
+      unsigned reached = (__ballot_sync(FULL, hit) >> gbase) & gones;
+      const unsigned accepted = abal & reached;
+      const uint32_t end = active ? 31u - __clz(reached) : 0u;  // twice the last node
+      const uint32_t la = accepted ? 31u - __clz(accepted) : 0u;
+      double cur = __shfl_sync(FULL, L, gbase + la);
+      const uint4 qa = make_uint4(
+          __shfl_sync(FULL, myq.x, gbase + la), __shfl_sync(FULL, myq.y, gbase + la),
+          __shfl_sync(FULL, myq.z, gbase + la), __shfl_sync(FULL, myq.w, gbase + la));
+      // Where the chain accepts at its last node, the nodes on that one's line of
+      // refusals that replace the same slot scored exactly the quadruple that the
+      // chain builds there, so the chain goes on through them -- each tested against
+      // the likelihood accepted last -- up to the first that replaces another slot.
+      const uint32_t desc_e = __shfl_sync(FULL, desc, gbase + end);
+      const uint32_t slot_e = __shfl_sync(FULL, slot, gbase + end);
+      const bool line = lead_lane && valid && taken == desc_e >> 8 && depth > (desc_e & 15u);
+      unsigned run = (__ballot_sync(FULL, line) >> gbase) & gones;
+      const unsigned other = (__ballot_sync(FULL, line && slot != slot_e) >> gbase) & gones;
+      if (!accepted || la != end)
+        run = 0;
+      else if (other)
+        run &= (other & (0u - other)) - 1u;
+      uint32_t hap = 0;
+      unsigned more = 0;  // accepted nodes of the run
+      reached |= run;
+      while (__any_sync(FULL, run != 0u)) {
+        const uint32_t from = gbase + (run ? (uint32_t)__ffs(run) - 1u : 0u);
+        const double L_r = __shfl_sync(FULL, L, from);
+        const float u_r = __shfl_sync(FULL, u, from);
+        const uint32_t ph_r = __shfl_sync(FULL, phap, from);
+        if (run) {
+          if (mh_accept(L_r, cur, pen, u_r)) {
+            cur = L_r;
+            hap = ph_r;
+            more |= run & (0u - run);
+          }
+          run &= run - 1u;
         }
       }
-    }
-    if (active) {
-      curr = curr0;
-      if (abal) {
-        set_slot(q, sla, hap);
-        curr = cur;
+      if (active) {
+        curr = curr0;
+        if (accepted) {
+          curr = cur;
+          q = qa;
+          if (more)
+            set_slot(q, slot_e, hap);
+        }
       }
-    }
-    if (lead_lane && r < k && r <= last) {
-      if (p.eval_trace)
-        p.eval_trace[(size_t)s * (C + 1) + ev] = L;
-      if (ev > 0 && p.accept_trace)
-        p.accept_trace[(size_t)s * C + ev - 1] =
-            (uint8_t)(r == first_acc || ((more >> r) & 1u));
-    }
-    if (active) {
-      e = (first_acc < npos) ? e + last + 1 : e + k;
-      if (li == 0) {
-        n_evals += k;
-        ++n_rounds;
-        n_acc += first_acc < npos ? 1u + (uint32_t)__popc(more) : 0u;
+      const unsigned mine = 1u << (lane - gbase);
+      if (lead_lane && (reached & mine)) {
+        if (p.eval_trace)
+          p.eval_trace[(size_t)s * (C + 1) + ev] = L;
+        if (ev > 0 && p.accept_trace)
+          p.accept_trace[(size_t)s * C + ev - 1] = (uint8_t)(((accepted | more) & mine) != 0u);
+      }
+      const uint32_t scored =
+          (uint32_t)__popc((__ballot_sync(FULL, lead_lane && valid) >> gbase) & gones);
+      if (active) {
+        const uint32_t steps = (uint32_t)__popc(reached),
+                       na = (uint32_t)(__popc(accepted) + __popc(more));
+        rate = __fdividef(kRateWeight * rate + (float)na,
+                          kRateWeight + (float)(steps - (e == 0 ? 1u : 0u)));
+        e += steps;
+        if (li == 0) {
+          n_evals += scored;
+          ++n_rounds;
+          n_acc += na;
+        }
+      }
+    } else {
+      // The accept rule of MHSampler.hpp:86-93 in chain order.  Every
+      // evaluation of the round was built on the round's starting state, and
+      // until the first acceptance the chain's current likelihood is the
+      // starting one, so each position tests its own proposal against it in
+      // parallel and the first accepting position (in chain order) wins: the
+      // same decisions as the sequential loop.  The even lanes vote.
+      const bool acc = lead_lane && r < k && ev > 0 && mh_accept(L, curr0, pen, u);
+      const unsigned gmask = (Pc == 32) ? FULL : (((1u << Pc) - 1u) << gbase);
+      const unsigned abal = __ballot_sync(FULL, acc) & gmask;
+      const uint32_t srcl = abal ? (uint32_t)(__ffs(abal) - 1) : gbase;
+      const uint32_t first_acc = abal ? (srcl - gbase) >> 1 : npos;
+      const double La = __shfl_sync(FULL, L, srcl);
+      const uint32_t sla = __shfl_sync(FULL, slot, srcl);
+      const uint32_t pha = __shfl_sync(FULL, phap, srcl);
+      // The positions after the first acceptance that replace the same slot
+      // scored exactly the quadruple the sequential chain builds there (it
+      // differs from the round's start only in that slot), so the chain goes on
+      // through them -- each tested against the likelihood accepted last --
+      // up to the first position that replaces another slot.
+      uint32_t last = first_acc, hap = pha;
+      uint32_t more = 0;  // accepted positions after first_acc
+      double cur = La;
+      const unsigned others = __ballot_sync(FULL, !(scores && lead_lane && slot == sla)) &
+                              0x55555555u & gmask;
+      // pairs after the first accepting one up to the next that replaces another slot
+      const unsigned after = others & ~((2u << srcl) - 1u);
+      const uint32_t stop =
+          !abal ? 0u : after ? ((uint32_t)__ffs(after) - 1 - gbase) >> 1 : npos;
+      for (uint32_t r2 = first_acc + 1; __any_sync(FULL, r2 < stop); ++r2) {
+        const uint32_t from = gbase + 2u * (r2 < stop ? r2 : 0u);
+        const double L_r = __shfl_sync(FULL, L, from);
+        const float u_r = __shfl_sync(FULL, u, from);
+        const uint32_t ph_r = __shfl_sync(FULL, phap, from);
+        if (r2 < stop) {
+          last = r2;
+          if (mh_accept(L_r, cur, pen, u_r)) {
+            cur = L_r;
+            hap = ph_r;
+            more |= 1u << r2;
+          }
+        }
+      }
+      if (active) {
+        curr = curr0;
+        if (abal) {
+          set_slot(q, sla, hap);
+          curr = cur;
+        }
+      }
+      if (lead_lane && r < k && r <= last) {
+        if (p.eval_trace)
+          p.eval_trace[(size_t)s * (C + 1) + ev] = L;
+        if (ev > 0 && p.accept_trace)
+          p.accept_trace[(size_t)s * C + ev - 1] =
+              (uint8_t)(r == first_acc || ((more >> r) & 1u));
+      }
+      if (active) {
+        e = (first_acc < npos) ? e + last + 1 : e + k;
+        if (li == 0) {
+          n_evals += k;
+          ++n_rounds;
+          n_acc += first_acc < npos ? 1u + (uint32_t)__popc(more) : 0u;
+        }
       }
     }
 

@@ -47,6 +47,24 @@ def test_windows_of_draws(dev, oracle_lib, C):
         assert np.array_equal(out["evals"], ref["evals"], equal_nan=True), lanes
 
 
+@pytest.mark.parametrize("pen", [1e-9, 0.003, 0.02, 0.08, 0.25, 1.0])
+def test_trees_of_every_shape(dev, oracle_lib, pen):
+    """Penalties from chains that accept everything to ones that accept little, so
+    that the wide groups' trees go from a line of acceptances over branched ones to
+    a line of refusals, at cycle counts that end a round early; the rate that the
+    kernel starts from is the generation before's."""
+    for N, C in ((3, 100), (37, 47)):
+        m, haps, quad, props = make_problem(N=N, S=130, C=C, seed=C)
+        ref = at_width(dev, 1, m, haps, quad, props, pen, seed=4, gen=1)
+        check_against_oracle(oracle_lib, m, haps, quad, props, pen, ref, 4, 1, check_work=False)
+        for lanes in (16, 32, 16, 32):
+            out = at_width(dev, lanes, m, haps, quad, props, pen, seed=4, gen=1)
+            for key in ("quad", "acc", "hnew", "like"):
+                assert np.array_equal(out[key], ref[key]), (lanes, key)
+            assert np.array_equal(out["evals"], ref["evals"], equal_nan=True), lanes
+            assert dev.counters()[2] == ref["acc"].sum()
+
+
 @pytest.mark.parametrize("vq", [False, True])
 @pytest.mark.parametrize("first", [0, 64, 192])
 def test_every_remainder_of_a_word(dev, oracle_lib, first, vq):
