@@ -128,7 +128,7 @@ struct glp_ctx {
   int knn_metric = GLP_KNN_HAMMING;  // glp_set_knn_metric
   bool short_blocks = false;
   // resident threads per lane width (1 .. 32), per [multi-chunk][VQ] kernel
-  double resident[2][2][6] = {};
+  double resident[2][2][8] = {};  // by the logarithm of the lanes
   bool resident_known[2][2] = {};
   uint32_t lanes_used = 4;
   double last_accept = -1.0;  // acceptance rate of the last generation
@@ -450,13 +450,23 @@ constexpr double kUsualRate = 0.12;
 // scored nodes of its speculation tree are reached.
 double steps_a_round(double a, uint32_t P) {
   static constexpr glp::SpecTrees trees = glp::make_spec_trees();
-  const int rate = glp::kSpecTree((int)P) ? (int)(a * 16.0 + 0.5) : 0;
-  const glp::SpecNode *t = trees.node[std::min(rate, glp::kSpecRates - 1)];
+  static constexpr glp::TeamTrees teams = glp::make_team_trees();
+  int rate = std::min((int)(a * 16.0 + 0.5), glp::kSpecRates - 1);
+  if (!glp::kSpecTree((int)P))
+    rate = 0;
   double sum = 0.0;
   for (uint32_t i = 0; i < P / 2; ++i) {
-    const int accepted = __builtin_popcount(t[i].accept),
-              refused = __builtin_popcount(t[i].path) - accepted;
-    sum += std::pow(a, accepted) * std::pow(1.0 - a, refused);
+    int accepted, depth;
+    if (P > 32) {
+      const glp::TeamNode &t = teams.node[rate][i];
+      accepted = __builtin_popcount(t.taken[0]) + __builtin_popcount(t.taken[1]);
+      depth = (int)(t.desc & 255u);
+    } else {
+      const glp::SpecNode &t = trees.node[rate][i];
+      accepted = __builtin_popcount(t.accept);
+      depth = __builtin_popcount(t.path);
+    }
+    sum += std::pow(a, accepted) * std::pow(1.0 - a, depth - accepted);
   }
   return sum;
 }
@@ -475,16 +485,20 @@ double steps_a_round(double a, uint32_t P) {
 // samples 16 lanes 0.55 (0.76; 32: 0.64), 1,500 x 2,048 8 lanes 1.07 (16: 1.14),
 // 2,500 x 2,048 16 lanes 1.42 (8: 1.51), 3,001 x 4,000 from codes 16 lanes 3.47 (8:
 // 3.68; 32: 4.52), 10,000 samples 8 lanes 2.05 (16: 2.49).
-constexpr double kLaneRoundCost[6] = {0.0, 2.2, 1.16, 1.05, 1.0, 1.0};
+// 64 and 128 lanes are teams of two and four warps, for one chunk alone.  They are
+// picked while every warp has a scheduler of its own: 152 x 1,024 128 lanes 0.237 ms
+// (32: 0.369), 300 64 lanes 0.281 (0.355), 400 32 lanes 0.353.
+constexpr int kWidths = 8;  // 1 << 0 .. 1 << 7 lanes
+constexpr double kLaneRoundCost[kWidths] = {0.0, 2.2, 1.16, 1.05, 1.0, 1.0, 1.0, 1.0};
 
 template <class FnOf>
-uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
+uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, uint32_t widest, FnOf kernel_for,
                     double *cache = nullptr, bool *known = nullptr) {
-  double local[6] = {};
+  double local[kWidths] = {};
   double *res = cache ? cache : local;
   if (!known || !*known) {
     res[0] = 0.0;
-    for (int i = 1; i < 6; ++i)
+    for (int i = 1; 1u << i <= widest; ++i)
       res[i] = resident_threads(kernel_for(1u << i), 1u << i, sms);
     if (known)
       *known = true;
@@ -492,7 +506,7 @@ uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
   const double as = std::min(a + std::min(a, 0.12), 1.0);
   uint32_t best = 8;
   double best_time = 0;
-  for (int i = 1; i < 6; ++i) {
+  for (int i = 1; 1u << i <= widest; ++i) {
     if (res[i] <= 0)
       continue;
     const uint32_t P = 1u << i;
@@ -506,7 +520,7 @@ uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, FnOf kernel_for,
     const double warps = held <= most
                              ? warps_cost(held * glp::kWarps / 4.0)
                              : warps_cost(most * glp::kWarps / 4.0) * ((double)blocks / sms) / most;
-    const double cost = kLaneRoundCost[i] * (vq && P == 32 ? 1.15 : 1.0);
+    const double cost = kLaneRoundCost[i] * (vq && P >= 32 ? 1.15 : 1.0);
     const double time = warps * cost / consumed;
     if (best_time == 0 || time < best_time * 0.98) {
       best_time = time;
@@ -527,7 +541,7 @@ uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen) {
   if (c->lanes)
     return c->lanes;
   return pick_lanes(
-      expected_rate(c, pen), N, c->sms, vq,
+      expected_rate(c, pen), N, c->sms, vq, multi ? 32u : 128u,
       [&](uint32_t P) {
         Shape sh;
         sh.P = P;
@@ -1935,7 +1949,7 @@ struct NoallocSetup {
   unsigned long long ctx_id = 0;  // 0: slot unused
   unsigned char *base = nullptr;
   int sms = 0;
-  double resident[6] = {};
+  double resident[kWidths] = {};
 };
 constexpr int kNoallocContexts = 16;
 std::mutex g_noalloc_mutex;
@@ -1997,7 +2011,7 @@ int noalloc_setup(NoallocSetup *out) {
       cudaDeviceGetAttribute(&e.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       allow_chain_smem() != cudaSuccess)
     return GLP_ERR_CUDA;
-  for (int i = 1; i < 6; ++i) {  // also sets each kernel's shared-memory attribute
+  for (int i = 1; i < kWidths; ++i) {  // also sets each kernel's shared-memory attribute
     Shape sh;
     sh.P = 1u << i;
     e.resident[i] = resident_threads(single_kernel(sh, false), sh.P, e.sms);
@@ -2123,7 +2137,7 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   // measured at set-up
   bool known = true;
   const uint32_t P = pick_lanes(
-      kUsualRate, N, sms, false,
+      kUsualRate, N, sms, false, 128u,
       [](uint32_t w) {
         Shape s1;
         s1.P = w;

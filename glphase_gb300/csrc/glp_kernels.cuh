@@ -1187,33 +1187,52 @@ struct SpecNode {
   uint32_t desc;    // [0, 4) depth, [4, 8) the last of those, [8, 24) their depths
 };
 constexpr int kSpecNodes = 16;  // a warp's lane pairs
+constexpr int kTeamNodes = 64;  // a team's of four warps
 constexpr int kSpecRates = 17;  // tree i is made for a = i / 16
+// Node n of a tree hangs from node parent[n], by acceptance or refusal.
+struct SpecShape {
+  int parent[kTeamNodes];
+  bool accept[kTeamNodes];
+};
+constexpr SpecShape make_spec_shape(int i) {
+  const double a = i == 0 ? 0.02 : i == 16 ? 0.98 : i / 16.0;
+  SpecShape t{};
+  double prob[kTeamNodes] = {};
+  double weight[kTeamNodes][2] = {};  // of the two children, 0 once they are there
+  prob[0] = 1.0;
+  weight[0][0] = 1 - a;
+  weight[0][1] = a;
+  for (int n = 1; n < kTeamNodes; ++n) {
+    int from = 0, dec = 0;
+    for (int v = 0; v < n; ++v)
+      for (int d = 0; d < 2; ++d)
+        if (weight[v][d] > weight[from][dec]) {
+          from = v;
+          dec = d;
+        }
+    t.parent[n] = from;
+    t.accept[n] = dec != 0;
+    prob[n] = prob[from] * (dec ? a : 1 - a);
+    weight[n][0] = prob[n] * (1 - a);
+    weight[n][1] = prob[n] * a;
+    // beside a refusal's child a quarter of an acceptance's is not needed: the next
+    // position replaces the same slot (generation_body)
+    if (!dec && weight[from][1] > 0.0)
+      weight[from][1] *= 0.75;
+    weight[from][dec] = 0.0;
+  }
+  return t;
+}
 struct SpecTrees {
   SpecNode node[kSpecRates][kSpecNodes];
 };
 constexpr SpecTrees make_spec_trees() {
   SpecTrees t{};
   for (int i = 0; i < kSpecRates; ++i) {
-    const double a = i == 0 ? 0.02 : i == 16 ? 0.98 : i / 16.0;
-    double prob[kSpecNodes] = {};
-    bool child[kSpecNodes][2] = {};
-    prob[0] = 1.0;
+    const SpecShape sh = make_spec_shape(i);
     for (int n = 1; n < kSpecNodes; ++n) {
-      int from = 0, dec = 0;
-      double best = -1.0;
-      for (int v = 0; v < n; ++v)
-        for (int d = 0; d < 2; ++d) {
-          // beside a refusal's child a quarter of an acceptance's is not needed: the
-          // next position replaces the same slot (generation_body)
-          const double pr = prob[v] * (d ? a : 1 - a) * (d && child[v][0] ? 0.75 : 1.0);
-          if (!child[v][d] && pr > best) {
-            best = pr;
-            from = v;
-            dec = d;
-          }
-        }
-      child[from][dec] = true;
-      prob[n] = prob[from] * (dec ? a : 1 - a);
+      const int from = sh.parent[n];
+      const bool dec = sh.accept[n];
       const SpecNode &pa = t.node[i][from];
       const uint32_t depth = pa.desc & 15u;
       SpecNode &nd = t.node[i][n];
@@ -1226,6 +1245,38 @@ constexpr SpecTrees make_spec_trees() {
   return t;
 }
 static __device__ const SpecTrees kSpecTrees = make_spec_trees();
+// The same for the nodes of a team: node 16 w + i is bit 2 i of word w.
+struct __align__(16) TeamNode {
+  uint32_t path[4], accept[4];
+  uint32_t taken[2];  // the accepted ancestors' depths
+  uint32_t desc;      // [0, 8) depth, [8, 16) the last of those
+  uint32_t unused;
+};
+struct TeamTrees {
+  TeamNode node[kSpecRates][kTeamNodes];
+};
+constexpr TeamTrees make_team_trees() {
+  TeamTrees t{};
+  for (int i = 0; i < kSpecRates; ++i) {
+    const SpecShape sh = make_spec_shape(i);
+    for (int n = 1; n < kTeamNodes; ++n) {
+      const int from = sh.parent[n];
+      const bool dec = sh.accept[n];
+      TeamNode &nd = t.node[i][n];
+      nd = t.node[i][from];
+      const uint32_t depth = nd.desc & 255u, bit = 1u << (2 * (from % kSpecNodes));
+      nd.path[from / kSpecNodes] |= bit;
+      if (dec) {
+        nd.accept[from / kSpecNodes] |= bit;
+        nd.taken[depth / 32] |= 1u << (depth % 32);
+        nd.desc = (uint32_t)from << 8;
+      }
+      nd.desc = (nd.desc & 0xff00u) | (depth + 1);
+    }
+  }
+  return t;
+}
+static __device__ const TeamTrees kTeamTrees = make_team_trees();
 // A chain's rate moves with weight 1 / 24 a cycle from the generation's (with 1 / 6,
 // chains of 10,000 samples took 0.8 % more rounds, 3 x 3 sites 1 % fewer).
 constexpr float kRateWeight = 24.0f;
@@ -1235,6 +1286,12 @@ constexpr float kRateWeight = 24.0f;
 // from codes at 8 lanes 4.39 and 4.46 ms, 10,000 x 4,096 7.36 and 7.40).
 constexpr bool kSpecTree(int P) { return P >= 16; }
 
+// The accept rule compares a uniform u with a float f: f > u for a float f exactly
+// when f > bound, and u = 0 has the bound -0.
+__device__ __forceinline__ float accept_bound(double u) {
+  return u == 0.0 ? -0.0f : __double2float_rd(u);
+}
+
 // One cycle's draws: the accept uniform, the proposed haplotype and the slot that
 // it replaces.
 struct __align__(16) Draw {
@@ -1242,6 +1299,46 @@ struct __align__(16) Draw {
   uint32_t hap, slot, unused;
 };
 constexpr uint32_t kDraws = 64;  // a warp's windows: two per lane of each group
+
+__device__ __forceinline__ Draw make_draw(const GenParams &p, uint32_t s, uint32_t cyc,
+                                          int *error) {
+  Draw d;
+  double u;
+  if (p.tr_slot) {
+    d.slot = p.tr_slot[(size_t)s * p.C + cyc] & 3u;
+    u = p.tr_u[(size_t)s * p.C + cyc];
+  } else {
+    glp_mh_draw(p.seed, p.generation, s, cyc, &d.slot, &u);
+  }
+  d.u = accept_bound(u);
+  d.hap = p.props ? __ldg(p.props + (size_t)cyc * p.N + s)
+          : (p.kick_first && cyc == 0)
+              ? glp_surrogate_ref(p.seed, p.generation, s, cyc, GLP_TAG_PROP, 2u * p.N, p.H,
+                                  p.nbr, p.klen)
+              : glp_surrogate(p.seed, p.generation, s, cyc, GLP_TAG_PROP, p.samp_lo, p.samp_hi,
+                              p.nbr, p.klen);
+  if (d.hap >= p.H) {
+    atomicOr(error, 1);
+    d.hap = 0;
+  }
+  return d;
+}
+
+// The accepted ancestors' haplotypes into q, whose slots in `have` are set: from
+// the last, at the highest of the bits of m (the draws of the cycles from `first`
+// on), to the first that still finds its slot open.
+__device__ __forceinline__ void place_path(uint4 &q, const Draw *window, uint32_t wmask,
+                                           uint32_t first, uint32_t m, uint32_t &have) {
+  while (m != 0u && have != 15u) {
+    const uint32_t top = 31u - __clz(m);
+    const Draw d = window[(first + top) & wmask];
+    if (!((have >> d.slot) & 1u)) {
+      set_slot(q, d.slot, d.hap);
+      have |= 1u << d.slot;
+    }
+    m ^= 1u << top;
+  }
+}
 
 // L1 prefetch of the words of haplotype h that an evaluation starts with: word 0
 // (forward), the top whole word and the partial one (backward).
@@ -1393,11 +1490,7 @@ __device__ __forceinline__ LaneGroups regroup(uint32_t lane, uint32_t na) {
 // exponential is taken in binary32 (relative error below 3e-6: a decision can
 // differ from the binary64 one only where |d - ln u| < 3e-6); below -37 it
 // is under 2^-53, so only u = 0 accepts, as in binary64.
-// u comes as accept_bound(u), made once with the draw: f > u for a float f exactly
-// when f > bound, and u = 0 is the bound -0.
-__device__ __forceinline__ float accept_bound(double u) {
-  return u == 0.0 ? -0.0f : __double2float_rd(u);
-}
+// u comes as accept_bound(u).
 __device__ __forceinline__ bool mh_accept(double prop, double curr, double pen, float bound) {
   if (prop >= curr)
     return true;
@@ -1405,6 +1498,32 @@ __device__ __forceinline__ bool mh_accept(double prop, double curr, double pen, 
   if (d > -37.0)
     return expf((float)d) > bound;
   return __float_as_uint(bound) == 0x80000000u && exp(d) > 0.0;
+}
+
+// The quadruple that sample s starts a generation with.
+__device__ __forceinline__ uint4 first_quad(const GenParams &p, uint32_t s, int *error) {
+  const uint32_t N = p.N, H = p.H;
+  uint4 q;
+  if (p.quad_in) {
+    q = make_uint4(__ldg(p.quad_in + s), __ldg(p.quad_in + N + s),
+                   __ldg(p.quad_in + 2 * (size_t)N + s), __ldg(p.quad_in + 3 * (size_t)N + s));
+  } else {
+    // fresh quadruple from the sampler, as RunHMMOnSamples draws one
+    // every generation (hmmLike.cpp:90-95)
+    q.x = glp_surrogate(p.seed, p.generation, s, 0, GLP_TAG_INIT, p.samp_lo, p.samp_hi, p.nbr,
+                        p.klen);
+    q.y = glp_surrogate(p.seed, p.generation, s, 1, GLP_TAG_INIT, p.samp_lo, p.samp_hi, p.nbr,
+                        p.klen);
+    q.z = glp_surrogate(p.seed, p.generation, s, 2, GLP_TAG_INIT, p.samp_lo, p.samp_hi, p.nbr,
+                        p.klen);
+    q.w = glp_surrogate(p.seed, p.generation, s, 3, GLP_TAG_INIT, p.samp_lo, p.samp_hi, p.nbr,
+                        p.klen);
+  }
+  if (q.x >= H || q.y >= H || q.z >= H || q.w >= H) {
+    atomicOr(error, 1);
+    q = make_uint4(0, 0, 0, 0);
+  }
+  return q;
 }
 
 template <int P, class E, class Src, int kSub = 1>
@@ -1462,30 +1581,9 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
         e = 0;
         drawn = 0;
         const GenParams &p = src.chunk(c);
-        const uint32_t N = p.N;
         if (kTree)
           rate = p.rate;
-        if (p.quad_in) {
-          q = make_uint4(__ldg(p.quad_in + s), __ldg(p.quad_in + N + s),
-                         __ldg(p.quad_in + 2 * (size_t)N + s),
-                         __ldg(p.quad_in + 3 * (size_t)N + s));
-        } else {
-          // fresh quadruple from the sampler, as RunHMMOnSamples draws one
-          // every generation (hmmLike.cpp:90-95)
-          q.x = glp_surrogate(p.seed, p.generation, s, 0, GLP_TAG_INIT, p.samp_lo, p.samp_hi,
-                              p.nbr, p.klen);
-          q.y = glp_surrogate(p.seed, p.generation, s, 1, GLP_TAG_INIT, p.samp_lo, p.samp_hi,
-                              p.nbr, p.klen);
-          q.z = glp_surrogate(p.seed, p.generation, s, 2, GLP_TAG_INIT, p.samp_lo, p.samp_hi,
-                              p.nbr, p.klen);
-          q.w = glp_surrogate(p.seed, p.generation, s, 3, GLP_TAG_INIT, p.samp_lo, p.samp_hi,
-                              p.nbr, p.klen);
-        }
-        const uint32_t H = p.H;
-        if (q.x >= H || q.y >= H || q.z >= H || q.w >= H) {
-          atomicOr(error, 1);
-          q = make_uint4(0, 0, 0, 0);
-        }
+        q = first_quad(p, s, error);
       } else {
         exhausted = true;
       }
@@ -1561,25 +1659,7 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       if (active && drawn < C && drawn + Pc - next <= 2 * Pc) {
         const uint32_t cyc = drawn + li;
         if (cyc < C) {
-          Draw d;
-          double u;
-          if (p.tr_slot) {
-            d.slot = p.tr_slot[(size_t)s * C + cyc] & 3u;
-            u = p.tr_u[(size_t)s * C + cyc];
-          } else {
-            glp_mh_draw(p.seed, p.generation, s, cyc, &d.slot, &u);
-          }
-          d.u = accept_bound(u);
-          d.hap = p.props ? __ldg(p.props + (size_t)cyc * N + s)
-                  : (p.kick_first && cyc == 0)
-                      ? glp_surrogate_ref(p.seed, p.generation, s, cyc, GLP_TAG_PROP, 2u * N, H,
-                                          p.nbr, p.klen)
-                      : glp_surrogate(p.seed, p.generation, s, cyc, GLP_TAG_PROP, p.samp_lo,
-                                      p.samp_hi, p.nbr, p.klen);
-          if (d.hap >= H) {
-            atomicOr(error, 1);
-            d.hap = 0;
-          }
+          const Draw d = make_draw(p, s, cyc, error);
           window[cyc & wmask] = d;
         }
         drawn += Pc;
@@ -1590,18 +1670,17 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
     float u = 0.0f;
     uint4 myq = q;
     if (scores) {
-      if (kTree)
-        for (uint32_t m = taken; m != 0u; m &= m - 1u) {  // accepted on its path
-          const Draw d = window[(e + (uint32_t)__ffs(m) - 2) & wmask];
-          set_slot(myq, d.slot, d.hap);
-          prefetch_first(p, d.hap, lead_lane);
-        }
       const Draw d = window[(ev - 1) & wmask];
       slot = d.slot;
       phap = d.hap;
       u = d.u;
       set_slot(myq, slot, phap);
       prefetch_first(p, phap, lead_lane);
+      if (kTree && taken) {
+        uint32_t have = 1u << slot;
+        place_path(myq, window, wmask, e - 1, taken, have);
+        prefetch_first(p, myq, lead_lane);
+      }
     }
     double L = 0.0;
     // When every lane of the warp scores a chunk of the same length, all
@@ -1799,11 +1878,165 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
   }
 }
 
+// What the warps of a team show one another in a round, a warp's part.
+struct __align__(16) TeamShare {
+  uint4 q[kSpecNodes];
+  double L[kSpecNodes];
+  uint32_t accepts, reached, next, unused;
+};
+
+// Generations of few samples: W warps of a block score 16 W nodes of a chain's
+// tree.  The chains are as long as before in evaluations and shorter in rounds (at
+// a = 0.12 a round goes on 7.3, 8.8 and 10.6 positions with 16, 32 and 64 nodes), and
+// the added warps run on schedulers that would stand idle.  Each warp stages the
+// sample's rows for itself; the warps meet at three barriers a round, for the
+// likelihoods, the votes and the nodes reached.  Where a round ends with an
+// acceptance the chain starts its next one there: the tree has that child mostly.
+// Measured, a team against one warp a chain: 60 x 1,024 0.351 and 0.234 ms (four
+// warps), 256 x 1,024 0.356 and 0.265 (two), 100 x 8,192 2.55 and 1.47, 3 x 3 0.056
+// and 0.041, 60 x 1,000 from codes 0.553 and 0.345.  Bound now: the chain of a site,
+// by the rounds of the longest chain.
+template <int W, class E, int kSub>
+__device__ __forceinline__ void generation_team(const GenParams &p, const float4 *vq_smem) {
+  static_assert(W == 2 || W == 4, "W");
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr uint32_t kNodes = (uint32_t)(kSpecNodes * W), kLanes = 32u * W;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, wt = warp % W,
+                 team = warp / W;
+  const uint32_t tl = 32 * wt + lane, r = tl >> 1;
+  const bool lead_lane = (lane & 1u) == 0;
+  extern __shared__ float4 glp_stage[];
+  float4 *const ring = glp_stage + (size_t)warp * kGroupStrideF4;
+  Draw *const window = reinterpret_cast<Draw *>(glp_stage + (size_t)kWarps * kGroupStrideF4) +
+                       team * W * kDraws;
+  TeamShare *const share =
+      reinterpret_cast<TeamShare *>(glp_stage + (size_t)kWarps * (kGroupStrideF4 + kDraws)) +
+      team * W;
+  static_assert(kDraws * W == 2 * kLanes && sizeof(Draw) == sizeof(float4), "window");
+  auto meet = [&]() {
+    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kLanes) : "memory");
+  };
+  const uint32_t N = p.N, C = p.C, teams = gridDim.x * (uint32_t)(kWarps / W);
+  const double pen = (double)p.pen;
+  unsigned long long n_evals = 0, n_rounds = 0, n_acc = 0, n_warp_rounds = 0;
+
+  for (uint32_t s = blockIdx.x * (uint32_t)(kWarps / W) + team; s < N;) {
+    uint4 q = first_quad(p, s, p.error);
+    double curr = 0.0;
+    float rate = p.rate;
+    uint32_t drawn = 0;
+    E em;
+    em.init(p, s, vq_smem);
+    for (uint32_t e = 0; e <= C;) {
+      const uint32_t tree = e == 0 ? 0u : (uint32_t)(rate * 16.0f + 0.5f);
+      const TeamNode *const node = &kTeamTrees.node[min(tree, kSpecRates - 1u)][r];
+      const uint32_t desc = __ldg(&node->desc), t0 = __ldg(&node->taken[0]),
+                     t1 = __ldg(&node->taken[1]);
+      const uint32_t depth = desc & 255u, ev = e + depth, k = min(kNodes, C + 1 - e);
+      const bool valid = depth < k, scores = valid && ev > 0;
+      prefetch_first(p, q, lead_lane);
+      // draws as in generation_body, for the team
+      constexpr uint32_t wmask = 2 * kLanes - 1;
+      if (drawn < min(C, e + k - 1)) {
+        const uint32_t cyc = drawn + tl;
+        if (cyc < C)
+          window[cyc & wmask] = make_draw(p, s, cyc, p.error);
+        drawn += kLanes;
+      }
+      meet();  // the draws are there, and what the last round shared is read
+      uint4 myq = q;
+      float u = 0.0f;
+      if (scores) {
+        const Draw d = window[(ev - 1) & wmask];
+        u = d.u;
+        set_slot(myq, d.slot, d.hap);
+        prefetch_first(p, d.hap, lead_lane);
+        if (t0 | t1) {
+          uint32_t have = 1u << d.slot;
+          place_path(myq, window, wmask, e + 31, t1, have);
+          place_path(myq, window, wmask, e - 1, t0, have);
+          prefetch_first(p, myq, lead_lane);
+        }
+      }
+      const double L = eval_pair<1, E, kSub, true, false>(p, em, myq, ring, lane, 32, FULL);
+      if (lead_lane) {
+        share[wt].L[lane >> 1] = L;
+        share[wt].q[lane >> 1] = myq;
+      }
+      meet();
+      if (e == 0)
+        curr = share[0].L[0];
+      const uint32_t up = (desc >> 8) & 255u;
+      const double at = (t0 | t1) ? share[up / kSpecNodes].L[up % kSpecNodes] : curr;
+      const unsigned votes =
+          __ballot_sync(FULL, lead_lane && scores && mh_accept(L, at, pen, u));
+      if (lane == 0)
+        share[wt].accepts = votes;
+      meet();
+      bool hit = lead_lane && valid;
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        hit = hit && ((share[w].accepts ^ __ldg(&node->accept[w])) & __ldg(&node->path[w])) == 0u;
+      const unsigned mine = __ballot_sync(FULL, hit);
+      if (lane == 0)
+        share[wt].reached = mine;
+      meet();
+      uint32_t steps = 0, na = 0, la = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        const unsigned reached = share[w].reached, accepted = reached & share[w].accepts;
+        steps += (uint32_t)__popc(reached);
+        na += (uint32_t)__popc(accepted);
+        if (accepted)
+          la = (uint32_t)(kSpecNodes * w) + ((31u - __clz(accepted)) >> 1);
+      }
+      if (na) {
+        curr = share[la / kSpecNodes].L[la % kSpecNodes];
+        q = share[la / kSpecNodes].q[la % kSpecNodes];
+      }
+      if (hit) {
+        if (p.eval_trace)
+          p.eval_trace[(size_t)s * (C + 1) + ev] = L;
+        if (ev > 0 && p.accept_trace)
+          p.accept_trace[(size_t)s * C + ev - 1] = (uint8_t)((votes >> lane) & 1u);
+      }
+      rate = __fdividef(kRateWeight * rate + (float)na,
+                        kRateWeight + (float)(steps - (e == 0 ? 1u : 0u)));
+      e += steps;
+      n_evals += (unsigned)__popc(__ballot_sync(FULL, lead_lane && valid));
+      n_acc += na;
+      ++n_rounds;
+      ++n_warp_rounds;
+    }
+    if (tl == 0) {
+      p.quad_out[s] = q.x;
+      p.quad_out[N + s] = q.y;
+      p.quad_out[2 * (size_t)N + s] = q.z;
+      p.quad_out[3 * (size_t)N + s] = q.w;
+      if (p.like_out)
+        p.like_out[s] = curr;
+      share[0].next = min(N, teams) + atomicAdd(p.counter, 1u);
+    }
+    meet();
+    s = share[0].next;
+  }
+  if (p.stats && n_warp_rounds && lane == 0) {
+    atomicAdd(p.stats, n_evals);
+    if (wt == 0) {
+      atomicAdd(p.stats + 1, n_rounds);
+      atomicAdd(p.stats + 2, n_acc);
+    }
+    atomicAdd(p.stats + 4, n_warp_rounds);
+    atomicAdd(p.stats + 5, 32 * n_warp_rounds);
+  }
+}
+
 // Dynamic shared memory of a generation kernel with P lanes per sample: one
-// staging ring (both directions) per group, and the warps' draws.
+// staging ring (both directions) per group or warp, the warps' draws, and what
+// teams share.
 __host__ __device__ constexpr size_t stage_bytes(int P) {
-  return sizeof(float4) * (size_t)kWarps * (32 / P) * kGroupStrideF4 +
-         sizeof(Draw) * (size_t)kWarps * kDraws;
+  return sizeof(float4) * (size_t)kWarps * (P < 32 ? 32 / P : 1) * kGroupStrideF4 +
+         sizeof(Draw) * (size_t)kWarps * kDraws + (P > 32 ? sizeof(TeamShare) * kWarps : 0);
 }
 
 // One chunk per launch (the reference's RunHMMOnDevice granularity).  P lanes
@@ -1816,8 +2049,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) generation_kernel(const 
   if (threadIdx.x < 16 && p.vq_table)
     s_vq[threadIdx.x] = p.vq_table[threadIdx.x];
   __syncthreads();
-  const OneChunk src{p};
-  generation_body<P, E, OneChunk, kSub>(src, p.counter, p.stats, p.error, s_vq);
+  if constexpr (P > 32) {
+    generation_team<P / 32, E, kSub>(p, s_vq);
+  } else {
+    const OneChunk src{p};
+    generation_body<P, E, OneChunk, kSub>(src, p.counter, p.stats, p.error, s_vq);
+  }
 }
 
 // Many chunks of uneven size in one persistent launch: one queue over all

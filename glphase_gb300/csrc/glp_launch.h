@@ -3,7 +3,8 @@
 // Each (entry kind, emission source, normalisation block) triple is
 // instantiated in its own translation unit (glp_gen_*.cu) so the
 // instantiations compile in parallel; the host code picks a kernel by its
-// speculation width: P lanes per sample (P/2 evaluations a round).
+// speculation width: P lanes per sample (P/2 evaluations a round); for one chunk
+// also the teams of two and four warps.
 #pragma once
 
 #include "glp_kernels.cuh"
@@ -26,16 +27,21 @@ MultiFn multi_kernel_vq_sub4(uint32_t P);
 }  // namespace glp
 
 // Body of one table: KERNEL<P, EMIT, SUB> for P = 2, 4, 8, 16, 32 (narrower
-// requests get two lanes: one evaluation a round, the sequential chain).
-#define GLP_GEN_TABLE(NAME, FNTYPE, KERNEL, EMIT, SUB) \
-  FNTYPE NAME(uint32_t P) {                            \
-    switch (P) {                                       \
-      case 0:                                          \
-      case 1:                                          \
-      case 2: return KERNEL<2, EMIT, SUB>;             \
-      case 4: return KERNEL<4, EMIT, SUB>;             \
-      case 8: return KERNEL<8, EMIT, SUB>;             \
-      case 16: return KERNEL<16, EMIT, SUB>;           \
-      default: return KERNEL<32, EMIT, SUB>;           \
-    }                                                  \
+// requests get two lanes: one evaluation a round, the sequential chain) and MORE.
+#define GLP_GEN_TABLE(NAME, FNTYPE, KERNEL, EMIT, SUB, MORE) \
+  FNTYPE NAME(uint32_t P) {                                  \
+    switch (P) {                                             \
+      case 0:                                                \
+      case 1:                                                \
+      case 2: return KERNEL<2, EMIT, SUB>;                   \
+      case 4: return KERNEL<4, EMIT, SUB>;                   \
+      case 8: return KERNEL<8, EMIT, SUB>;                   \
+      case 16: return KERNEL<16, EMIT, SUB>;                 \
+        MORE(KERNEL, EMIT, SUB)                              \
+      default: return KERNEL<32, EMIT, SUB>;                 \
+    }                                                        \
   }
+#define GLP_GEN_TEAMS(KERNEL, EMIT, SUB)   \
+  case 64: return KERNEL<64, EMIT, SUB>;   \
+  case 128: return KERNEL<128, EMIT, SUB>;
+#define GLP_GEN_NO_TEAMS(KERNEL, EMIT, SUB)

@@ -179,7 +179,8 @@ int glp_finish(glp_ctx *ctx);
  * lane pairs that each score one chain position a round (one lane the
  * forward half of the sites, the other the backward half); 1 is taken as 2
  * (one position a round: the sequential chain); 0 = choose from the last
- * generation's acceptance rate. */
+ * generation's acceptance rate, for one chunk of few samples also 64 or 128
+ * lanes (two or four warps a sample).  Results are the same at every width. */
 int glp_set_lanes_per_sample(glp_ctx *ctx, uint32_t lanes);
 
 /* Evaluations each lane pair scores per speculative round: 1 (or 0, the

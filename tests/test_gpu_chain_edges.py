@@ -40,7 +40,7 @@ def test_windows_of_draws(dev, oracle_lib, C):
     m, haps, quad, props = make_problem(N=37, S=70, C=C, seed=C + 1)
     ref = at_width(dev, 1, m, haps, quad, props, 0.5, seed=9, gen=3)
     check_against_oracle(oracle_lib, m, haps, quad, props, 0.5, ref, 9, 3, check_work=False)
-    for lanes in (2, 4, 8, 16, 32):
+    for lanes in (2, 4, 8, 16, 32, 0):  # 0: teams of warps
         out = at_width(dev, lanes, m, haps, quad, props, 0.5, seed=9, gen=3)
         for key in ("quad", "acc", "hnew", "like"):
             assert np.array_equal(out[key], ref[key]), (lanes, key)
@@ -57,7 +57,7 @@ def test_trees_of_every_shape(dev, oracle_lib, pen):
         m, haps, quad, props = make_problem(N=N, S=130, C=C, seed=C)
         ref = at_width(dev, 1, m, haps, quad, props, pen, seed=4, gen=1)
         check_against_oracle(oracle_lib, m, haps, quad, props, pen, ref, 4, 1, check_work=False)
-        for lanes in (16, 32, 16, 32):
+        for lanes in (16, 32, 0, 16, 32, 0):  # 0: teams of warps
             out = at_width(dev, lanes, m, haps, quad, props, pen, seed=4, gen=1)
             for key in ("quad", "acc", "hnew", "like"):
                 assert np.array_equal(out[key], ref[key]), (lanes, key)
