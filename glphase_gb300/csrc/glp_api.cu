@@ -404,18 +404,16 @@ void launch_work(const glp::MultiParams &mp, WorkGrids g, cudaStream_t st) {
 WorkGrids batch_tables(const glp::GenParams *chunks, uint32_t count, uint32_t *out) {
   uint32_t *offsets = out, *order = out + count + 1, *blocks = order + count,
            *warps = blocks + count + 1;
-  uint32_t total = 0;
-  for (uint32_t i = 0; i < count; ++i) {
-    offsets[i] = total;
-    total += chunks[i].N;
+  for (uint32_t i = 0; i < count; ++i)
     order[i] = i;
-  }
-  offsets[count] = total;
   std::stable_sort(order, order + count,
                    [&](uint32_t a, uint32_t b) { return chunks[a].S > chunks[b].S; });
   WorkGrids g;
+  uint32_t total = 0;
   for (uint32_t i = 0; i < count; ++i) {
     const glp::GenParams &p = chunks[order[i]];
+    offsets[i] = total;
+    total += p.N;
     blocks[i] = g.chains;
     warps[i] = g.samples;
     if (p.do_work) {
@@ -423,6 +421,7 @@ WorkGrids batch_tables(const glp::GenParams *chunks, uint32_t count, uint32_t *o
       g.samples += p.N * glp::sample_parts(p.wn);
     }
   }
+  offsets[count] = total;
   blocks[count] = g.chains;
   warps[count] = g.samples;
   return g;

@@ -143,3 +143,39 @@ def test_uniforms_at_the_ends_of_their_range(dev):
                 curr = prop if out["acc"][s, c] else curr
         accepted.append(out["acc"][u == 0.0].mean())
     assert accepted[0] == 1.0 and accepted[2] < 1.0
+
+
+@pytest.mark.parametrize("lanes", [2, 8, 32])
+def test_queue_of_uneven_chunks(dev, lanes):
+    """More samples than the GPU holds groups (at 32 lanes), chunks not in the
+    order of their sites: every sample is run once, in its own chunk."""
+    import ctypes
+
+    import torch
+    from test_gpu_batch import Chunk
+    chunks = [Chunk(dev, N, S, 3, seed=i + 1)
+              for i, (N, S) in enumerate([(700, 40), (1101, 130), (3, 200), (997, 70)])]
+    dev.set_lanes_per_sample(lanes)
+    try:
+        torch.cuda.synchronize()
+        args = (nat.GenerationArgs * 4)(*[ch.args(0.5, 2) for ch in chunks])
+        pbs = (ctypes.c_void_p * 4)(*[ch.pb for ch in chunks])
+        dev._c(dev.L.glp_run_batch(dev.ctx, 4, pbs, args))
+        dev._c(dev.L.glp_finish(dev.ctx))
+        batched = [ch.outputs() for ch in chunks]
+        for ch, out in zip(chunks, batched):
+            ch.reset()
+            dev.copy_tran_to_device(ch.m.tran)
+            dev.copy_mutation_mat_to_device(ch.m.pc)
+            dev.copy_emission_to_device(ch.m.emit, ch.m.t)
+            torch.cuda.synchronize()
+            a = ch.args(0.5, 2)
+            dev._c(dev.L.glp_run_generation(dev.ctx, ctypes.byref(a)))
+            dev._c(dev.L.glp_finish(dev.ctx))
+            alone = ch.outputs()
+            for k in ("quad", "like", "acc", "evals", "hnew"):
+                assert np.array_equal(out[k], alone[k]), k
+    finally:
+        dev.set_lanes_per_sample(0)
+        for ch in chunks:
+            dev.L.glp_problem_destroy(ch.pb)
