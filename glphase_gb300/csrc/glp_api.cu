@@ -478,21 +478,33 @@ double steps_a_round(double a, uint32_t P) {
 // (1,024 sites, a = 0.12, times of a generation kernel relative to one warp a
 // scheduler): 1.44 at two, 2.0 at three, beyond that in proportion (whole blocks of
 // four warps, so the steps are at multiples of the SM count).  Narrow groups stage
-// more rows a lane: 1.16 at 4 lanes, 2.2 at 2 lanes; at 8 lanes 1.05; on VQ codes,
-// whose table reads conflict more in a wide group, 1.15 at 32.  The widths this
-// picks, against others: 256 samples 32 lanes 0.36 ms (8: 0.55, 16: 0.42), 1,000
-// samples 16 lanes 0.55 (0.76; 32: 0.64), 1,500 x 2,048 8 lanes 1.07 (16: 1.14),
-// 2,500 x 2,048 16 lanes 1.42 (8: 1.51), 3,001 x 4,000 from codes 16 lanes 3.47 (8:
-// 3.68; 32: 4.52), 10,000 samples 8 lanes 2.05 (16: 2.49).
+// more rows a lane and read a row for fewer evaluations: at 4 lanes 1.25, on VQ
+// codes 1.5, and where the rows exceed half of L2 1.9 (measured against 8 lanes 1.5
+// to 2.2: 20,000 x 512 at 8 lanes 1.65 ms, 4: 2.37; 15,000 x 2,048 4.66 and 8.28;
+// 40,000 x 100, whose rows stay, 2.36 and 2.02); at 2 lanes, one block an SM, 2.7;
+// at 8 lanes 1.05, and 1.1 for such rows (2,000 x 4,096 2.65 ms, 16: 2.35); on VQ
+// codes, whose table reads conflict more in a wide group, 1.15 from 32.  The widths
+// this picks, against others: 256 samples 64 lanes 0.27 ms (32: 0.36, 8: 0.55),
+// 1,000 samples 16 lanes 0.55 (0.76; 32: 0.64), 1,500 x 2,048 8 lanes 1.07 (16:
+// 1.14), 2,500 x 2,048 16 lanes 1.42 (8: 1.51), 3,001 x 4,000 from codes 16 lanes
+// 3.47 (8: 3.68; 32: 4.52), 10,000 samples 8 lanes 2.05 (16: 2.49).
 // 64 and 128 lanes are teams of two and four warps, for one chunk alone.  They are
 // picked while every warp has a scheduler of its own: 152 x 1,024 128 lanes 0.237 ms
 // (32: 0.369), 300 64 lanes 0.281 (0.355), 400 32 lanes 0.353.
 constexpr int kWidths = 8;  // 1 << 0 .. 1 << 7 lanes
-constexpr double kLaneRoundCost[kWidths] = {0.0, 2.2, 1.16, 1.05, 1.0, 1.0, 1.0, 1.0};
+double lane_round_cost(uint32_t P, bool vq, bool streams) {
+  switch (P) {
+    case 2: return 2.7;
+    case 4: return vq ? 1.5 : streams ? 1.9 : 1.25;
+    case 8: return streams ? 1.1 : 1.05;
+    case 16: return 1.0;
+    default: return vq ? 1.15 : 1.0;
+  }
+}
 
 template <class FnOf>
-uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, uint32_t widest, FnOf kernel_for,
-                    double *cache = nullptr, bool *known = nullptr) {
+uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, bool streams, uint32_t widest,
+                    FnOf kernel_for, double *cache = nullptr, bool *known = nullptr) {
   double local[kWidths] = {};
   double *res = cache ? cache : local;
   if (!known || !*known) {
@@ -519,7 +531,7 @@ uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, uint32_t widest, FnO
     const double warps = held <= most
                              ? warps_cost(held * glp::kWarps / 4.0)
                              : warps_cost(most * glp::kWarps / 4.0) * ((double)blocks / sms) / most;
-    const double cost = kLaneRoundCost[i] * (vq && P >= 32 ? 1.15 : 1.0);
+    const double cost = lane_round_cost(P, vq, streams);
     const double time = warps * cost / consumed;
     if (best_time == 0 || time < best_time * 0.98) {
       best_time = time;
@@ -536,11 +548,11 @@ double expected_rate(const glp_ctx *c, float pen) {
                                                       : std::max(c->last_accept, 1e-3);
 }
 
-uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen) {
+uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bool streams) {
   if (c->lanes)
     return c->lanes;
   return pick_lanes(
-      expected_rate(c, pen), N, c->sms, vq, multi ? 32u : 128u,
+      expected_rate(c, pen), N, c->sms, vq, streams, multi ? 32u : 128u,
       [&](uint32_t P) {
         Shape sh;
         sh.P = P;
@@ -551,9 +563,9 @@ uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen) {
 
 // Lanes from choose_lanes (a request below two lanes gets two: one
 // evaluation a round), normalisation block from the context's rule.
-Shape choose_shape(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen) {
+Shape choose_shape(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bool streams) {
   Shape sh;
-  sh.P = std::max<uint32_t>(2u, choose_lanes(c, N, multi, vq, pen));
+  sh.P = std::max<uint32_t>(2u, choose_lanes(c, N, multi, vq, pen, streams));
   c->launch_pen = pen;
   if (c->block_sites == 4 || (c->block_sites == 0 && c->short_blocks))
     sh.sub = 2;
@@ -690,7 +702,8 @@ uint64_t emission_bytes(const glp::GenParams &p) {
 // 8-lane warps a scheduler, or chunks of different lengths, whose longest ends
 // alone (2,000 x 8,192: 6.30 -> 5.64 ms a generation, eight uneven chunks 14.4 ->
 // 14.1; with the GPU full, 10,000 x 4,096, 7.39 -> 7.43).
-void mark_stream(const glp_ctx *c, glp::GenParams *chunks, uint32_t count) {
+// Returns whether they exceed half of L2 (a half serves the SMs beside it).
+bool mark_stream(const glp_ctx *c, glp::GenParams *chunks, uint32_t count) {
   uint64_t bytes = 0, samples = 0;
   for (uint32_t i = 0; i < count; ++i) {
     bytes += emission_bytes(chunks[i]);
@@ -699,6 +712,7 @@ void mark_stream(const glp_ctx *c, glp::GenParams *chunks, uint32_t count) {
   const bool few = count > 1 || samples * 8 <= (uint64_t)2 * 128 * c->sms;
   for (uint32_t i = 0; i < count; ++i)
     chunks[i].stream = bytes > c->l2_bytes && few ? 1u : 0u;
+  return 2 * bytes > c->l2_bytes;
 }
 
 int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
@@ -707,8 +721,8 @@ int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
   if (rc)
     return rc;
   const bool vq = (a->flags & GLP_GEN_VQ) != 0;
-  mark_stream(c, &p, 1);
-  const Shape sh = choose_shape(c, a->num_samples, false, vq, a->pen);
+  const bool streams = mark_stream(c, &p, 1);
+  const Shape sh = choose_shape(c, a->num_samples, false, vq, a->pen, streams);
   const uint32_t P = sh.P;
   SingleFn fn = single_kernel(sh, vq);
   const unsigned grid = grid_for(c, fn, a->num_samples, P, &rc);
@@ -1121,7 +1135,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     if (total > 0xffffffffull)
       return fail(c, GLP_ERR_ARG, "a batch holds at most 2^32-1 samples");
   }
-  mark_stream(c, c->h_table, count);
+  const bool streams = mark_stream(c, c->h_table, count);
   const WorkGrids work = batch_tables(c->h_table, count, c->h_offsets);
   if ((rc = ensure(c, c->d_table, c->table_cap, count)) ||
       (rc = ensure(c, c->d_offsets, c->offsets_cap, glp::batch_words(count))))
@@ -1138,7 +1152,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   mp.counter = c->d_counter;
   mp.stats = c->d_stats;
   mp.error = c->d_error;
-  const Shape sh = choose_shape(c, total, true, vq, c->h_table[0].pen);
+  const Shape sh = choose_shape(c, total, true, vq, c->h_table[0].pen, streams);
   const uint32_t P = sh.P;
   MultiFn fn = multi_kernel(sh, vq);
   const unsigned grid = grid_for(c, fn, total, P, &rc);
@@ -1243,7 +1257,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   glp_batch *b = new glp_batch();
   b->c = c;
   b->count = count;
-  mark_stream(c, table.data(), count);
+  const bool streams = mark_stream(c, table.data(), count);
   b->work = batch_tables(table.data(), count, offsets.data());
   b->chain_cycles = chain_cycles;
   cudaStream_t cs = nullptr;
@@ -1267,7 +1281,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   b->mp.counter = c->d_counter;
   b->mp.stats = c->d_stats;
   b->mp.error = c->d_error;
-  const Shape sh = choose_shape(c, total, true, vq, table[0].pen);
+  const Shape sh = choose_shape(c, total, true, vq, table[0].pen, streams);
   b->P = sh.P;
   b->fn = multi_kernel(sh, vq);
   b->grid = grid_for(c, b->fn, total, b->P, &rc);
@@ -2136,7 +2150,7 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   // measured at set-up
   bool known = true;
   const uint32_t P = pick_lanes(
-      kUsualRate, N, sms, false, 128u,
+      kUsualRate, N, sms, false, false, 128u,
       [](uint32_t w) {
         Shape s1;
         s1.P = w;

@@ -53,11 +53,11 @@ namespace glp {
 #endif
 constexpr int kWarps = GLP_GEN_WARPS;  // warps per generation block
 constexpr int kThreads = 32 * kWarps;
-// Resident blocks per SM the generation kernels are compiled for (the
-// launch bound's minimum): with 3 the compiler may use up to 168 registers
-// a thread and schedules the loop in 119-127, so 4 blocks (16 warps) still
-// fit; measured 1.2 % faster than the bound of 4 (a cap of 128) on 10,000
-// samples x 4,096 sites.  5 (a cap of 96) was 16 % slower.
+// Resident blocks per SM the generation kernels are compiled for (the launch
+// bound's minimum): with 3 the compiler may use up to 168 registers a thread and
+// takes 120-136, so 3 blocks of the 8- and 16-lane kernels fit.  A bound of 4 (a cap
+// of 128) was 2.4 % slower on 10,000 samples x 4,096 sites and 5 % on 2,000 x 8,192,
+// 5 (a cap of 96) 16 %; of 2 the same.
 #ifndef GLP_MIN_BLOCKS
 #define GLP_MIN_BLOCKS 3
 #endif
@@ -567,8 +567,8 @@ __device__ __forceinline__ double log_dot(float2 xX, float2 xY, float2 yX, float
 // Log-likelihood (natural log, binary64) of quadruple q, scored by a lane
 // pair of a P-lane group.  Of the nw = floor(S/64) full 64-site words, the
 // even lane runs the forward half over words [0, wf), wf = ceil(nw/2); the
-// odd lane first runs the sites of the partial top word site by site
-// (straight from global memory), then the backward half over words
+// odd lane first runs the sites of the partial top word (straight from
+// global memory), then the backward half over words
 // [wf, nw) from the top.  Each word is eight 8-site blocks, run four at a
 // time so that ring slots and parent-bit positions are constants: step t
 // stages forward block t and backward block 8 nw - 1 - t of every pair into
