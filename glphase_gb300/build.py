@@ -1,6 +1,6 @@
 """In-tree build of the CUDA library ``glphase_gb300/libglphase_gpu.so``.
 
-Five translation units (the host side and four tables of generation-kernel
+Nine translation units (the host side and eight tables of generation-kernel
 instantiations) compiled in parallel with nvcc, one ``-gencode`` (sm_103a),
 then linked; host code with ``-ffp-contract=off`` so host-side float
 arithmetic rounds identically on x86-64 and aarch64.
