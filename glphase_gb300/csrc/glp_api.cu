@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -80,6 +81,15 @@ struct glp_problem {
   size_t beta_cap = 0;
 };
 
+// What a context's launches write beside their outputs, together so that one
+// memset clears a launch's part and one copy brings all of it back (a generation of
+// 3 x 3 sites, launched and finished: 97 us with two of each, 88 so).
+struct LaunchRecord {
+  unsigned long long stats[glp::kStats];
+  uint32_t counter;  // the sample queue
+  int error;         // kept until glp_finish reports it
+};
+
 struct glp_ctx {
   int device = 0;
   int sms = 0;
@@ -89,9 +99,7 @@ struct glp_ctx {
   std::string err;
   glp_problem def;  // the model set by glp_set_* (HMMLikeCUDA semantics)
   // work buffers
-  uint32_t *d_counter = nullptr;
-  unsigned long long *d_stats = nullptr;
-  int *d_error = nullptr;
+  LaunchRecord *d_record = nullptr;
   glp::GenParams *d_table = nullptr;  // batch descriptors
   uint32_t *d_offsets = nullptr;
   size_t table_cap = 0, offsets_cap = 0;
@@ -654,9 +662,9 @@ int make_params(glp_ctx *c, glp_problem *pb, const glp_generation_args *a,
   p->eval_trace = a->eval_trace;
   p->accept_trace = a->accept_trace;
   p->beta = pb->d_beta;
-  p->counter = c->d_counter;
-  p->stats = c->d_stats;
-  p->error = c->d_error;
+  p->counter = &c->d_record->counter;
+  p->stats = c->d_record->stats;
+  p->error = &c->d_record->error;
   p->nbr = a->neighbors;
   p->klen = a->neighbors_per_sample;
   p->samp_lo = lo;
@@ -690,6 +698,11 @@ unsigned grid_for(glp_ctx *c, Fn fn, uint64_t samples, uint32_t P, int *rc) {
   const uint64_t cap = (uint64_t)occ * c->sms;
   *rc = GLP_OK;
   return (unsigned)std::max<uint64_t>(1, std::min(want, cap));
+}
+
+// Clears a launch's part of the record.
+cudaError_t clear_record(const glp_ctx *c, cudaStream_t st) {
+  return cudaMemsetAsync(c->d_record, 0, offsetof(LaunchRecord, error), st);
 }
 
 // Emission rows that the rounds of a generation read again and again.
@@ -728,8 +741,7 @@ int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
   const unsigned grid = grid_for(c, fn, a->num_samples, P, &rc);
   if (rc)
     return rc;
-  GLP_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(uint32_t), c->stream));
-  GLP_CUDA(c, cudaMemsetAsync(c->d_stats, 0, glp::kStats * sizeof(unsigned long long), c->stream));
+  GLP_CUDA(c, clear_record(c, c->stream));
   cudaEvent_t *ev = c->ev[c->ev_count++ % glp_ctx::kTimed];
   GLP_CUDA(c, cudaEventRecord(ev[0], c->stream));
   fn<<<grid, glp::kThreads, glp::stage_bytes((int)P), c->stream>>>(p);
@@ -847,7 +859,7 @@ int knn_products(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t H,
     auto fn = p.sym ? glp::knn_gemm_kernel<true> : glp::knn_gemm_kernel<false>;
     fn<<<grid, glp::kGemmThreads, glp::kGemmSmem, c->stream>>>(
         am, am, q0, 0, nq, H, q0, 0, H, steps, c->d_knn_sites, p.pitch, c->d_knn_dist,
-        c->d_error);
+        &c->d_record->error);
     GLP_CUDA(c, cudaGetLastError());
     return GLP_OK;
   }
@@ -865,7 +877,7 @@ int knn_products(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t H,
       const dim3 grid(tiles(na, glp::kGemmM), tiles(nb, glp::kGemmN));
       glp::knn_gemm_kernel<false><<<grid, glp::kGemmThreads, glp::kGemmSmem, c->stream>>>(
           am, bm, 0, 0, na, nb, q0 + i, h, H, steps, c->d_knn_sites, p.pitch,
-          c->d_knn_dist + (size_t)i * p.pitch, c->d_error);
+          c->d_knn_dist + (size_t)i * p.pitch, &c->d_record->error);
       GLP_CUDA(c, cudaGetLastError());
     }
   }
@@ -918,10 +930,8 @@ int glp_create(int device, glp_ctx **out) {
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc((void **)&c->d_counter, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc((void **)&c->d_stats, glp::kStats * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc((void **)&c->d_error, sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->d_error, 0, sizeof(int)) != cudaSuccess ||
+      cudaMalloc((void **)&c->d_record, sizeof(LaunchRecord)) != cudaSuccess ||
+      cudaMemset(c->d_record, 0, sizeof(LaunchRecord)) != cudaSuccess ||
       allow_chain_smem() != cudaSuccess) {
     glp_destroy(c);
     return GLP_ERR_CUDA;
@@ -946,9 +956,7 @@ void glp_destroy(glp_ctx *c) {
   if (c->stream)
     cudaStreamSynchronize(c->stream);
   release_problem(&c->def);
-  release(c->d_counter);
-  release(c->d_stats);
-  release(c->d_error);
+  release(c->d_record);
   release(c->d_table);
   release(c->d_offsets);
   if (c->h_table)
@@ -1149,17 +1157,16 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   mp.chunks = c->d_table;
   mp.offsets = c->d_offsets;
   mp.nchunks = count;
-  mp.counter = c->d_counter;
-  mp.stats = c->d_stats;
-  mp.error = c->d_error;
+  mp.counter = &c->d_record->counter;
+  mp.stats = c->d_record->stats;
+  mp.error = &c->d_record->error;
   const Shape sh = choose_shape(c, total, true, vq, c->h_table[0].pen, streams);
   const uint32_t P = sh.P;
   MultiFn fn = multi_kernel(sh, vq);
   const unsigned grid = grid_for(c, fn, total, P, &rc);
   if (rc)
     return rc;
-  GLP_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(uint32_t), c->stream));
-  GLP_CUDA(c, cudaMemsetAsync(c->d_stats, 0, glp::kStats * sizeof(unsigned long long), c->stream));
+  GLP_CUDA(c, clear_record(c, c->stream));
   cudaEvent_t *ev = c->ev[c->ev_count++ % glp_ctx::kTimed];
   GLP_CUDA(c, cudaEventRecord(ev[0], c->stream));
   fn<<<grid, glp::kThreads, glp::stage_bytes((int)P), c->stream>>>(mp);
@@ -1194,8 +1201,7 @@ namespace {
 
 int batch_enqueue(glp_batch *b, cudaStream_t st) {
   glp_ctx *c = b->c;
-  GLP_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(uint32_t), st));
-  GLP_CUDA(c, cudaMemsetAsync(c->d_stats, 0, glp::kStats * sizeof(unsigned long long), st));
+  GLP_CUDA(c, clear_record(c, st));
   b->fn<<<b->grid, glp::kThreads, glp::stage_bytes((int)b->P), st>>>(b->mp);
   GLP_CUDA(c, cudaGetLastError());
   launch_work(b->mp, b->work, st);
@@ -1278,9 +1284,9 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   b->mp.chunks = b->d_table;
   b->mp.offsets = b->d_offsets;
   b->mp.nchunks = count;
-  b->mp.counter = c->d_counter;
-  b->mp.stats = c->d_stats;
-  b->mp.error = c->d_error;
+  b->mp.counter = &c->d_record->counter;
+  b->mp.stats = c->d_record->stats;
+  b->mp.error = &c->d_record->error;
   const Shape sh = choose_shape(c, total, true, vq, table[0].pen, streams);
   b->P = sh.P;
   b->fn = multi_kernel(sh, vq);
@@ -1337,10 +1343,10 @@ int glp_finish(glp_ctx *c) {
     return rc;
   GLP_CUDA(c, cudaStreamSynchronize(c->stream));
   GLP_CUDA(c, cudaGetLastError());
-  int h_err = 0;
-  GLP_CUDA(c, cudaMemcpy(&h_err, c->d_error, sizeof(int), cudaMemcpyDeviceToHost));
-  GLP_CUDA(c, cudaMemcpy(c->last_stats, c->d_stats, sizeof(c->last_stats),
-                         cudaMemcpyDeviceToHost));
+  LaunchRecord record;
+  GLP_CUDA(c, cudaMemcpy(&record, c->d_record, sizeof(record), cudaMemcpyDeviceToHost));
+  const int h_err = record.error;
+  std::memcpy(c->last_stats, record.stats, sizeof(record.stats));
   if (c->last_chain_cycles) {
     c->last_accept = (double)c->last_stats[2] / (double)c->last_chain_cycles;
     c->accept_pen = c->launch_pen;
@@ -1348,7 +1354,7 @@ int glp_finish(glp_ctx *c) {
   if (c->block_sites == 0 && c->last_stats[0] && c->last_stats[3] * 1000ull > c->last_stats[0])
     c->short_blocks = true;
   if (h_err) {
-    GLP_CUDA(c, cudaMemset(c->d_error, 0, sizeof(int)));
+    GLP_CUDA(c, cudaMemset(&c->d_record->error, 0, sizeof(int)));
     if (h_err & ~1)
       return fail(c, GLP_ERR_INDEX, "device self-check failed: flag 0x%x", (unsigned)h_err);
     return fail(c, GLP_ERR_INDEX, "a haplotype index >= num_haps reached the device");
