@@ -1872,7 +1872,7 @@ int glp_knn_neighbors(glp_ctx *c, const uint64_t *haps, uint32_t H, uint32_t S, 
       return rc;
     }
     select<<<n, glp::kKnnThreads, 0, c->stream>>>(c->d_knn_dist, pitch, H, s0, half, S,
-                                                  neighbors);
+                                                  &c->d_record->error, neighbors);
     GLP_CUDA(c, cudaGetLastError());
   }
   return GLP_OK;

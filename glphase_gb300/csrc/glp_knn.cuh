@@ -31,6 +31,8 @@ constexpr int kKnnThreads = 512;
 constexpr uint32_t kKnnMaxHaps = 50000;
 constexpr uint32_t kKnnMaxHalf = 1024;
 constexpr uint16_t kKnnExcluded = 0xffffu;
+constexpr uint32_t kKnnNoHap = 0xffffffffu;  // a list without distances behind it
+constexpr int kGemmTimeout = 2;  // error flag bit: a wait of knn_gemm_kernel ran out
 
 // The bits of 32 lanes transposed: lane l gets bit l of every lane's x (in some
 // order, which a population count does not see).
@@ -138,7 +140,8 @@ constexpr uint32_t kSelectMost = 1024;
 
 // The general path: the `half` smallest (d, index) of the entries of row d that
 // are not kKnnExcluded and not in `taken` (may be null), written sorted to
-// out[0 .. half).  keys: 2 * kKnnMaxHalf words.
+// out[0 .. half); 0xffff, which no haplotype has, where the row holds fewer.
+// keys: kKnnMaxHalf words.
 __device__ __noinline__ void select_general(const uint16_t *__restrict__ d, uint32_t H,
                                             uint32_t half, uint32_t dmax, const uint32_t *taken,
                                             uint32_t *keys, uint32_t *red, uint32_t *out) {
@@ -172,6 +175,12 @@ __device__ __noinline__ void select_general(const uint16_t *__restrict__ d, uint
   uint32_t rank = block_exclusive(ties, red, &total);
   uint32_t pos = block_exclusive(nless, red, &below);
   const uint32_t need = half - below;  // ties at t, taken in index order
+  uint32_t n2 = 1;  // the next power of two
+  while (n2 < half)
+    n2 <<= 1;
+  for (uint32_t i = tid; i < n2; i += kKnnThreads)
+    keys[i] = 0xffffffffu;
+  __syncthreads();
   // entries below the threshold first (positions [0, below)), then ties
   for (uint32_t h = b0; h < b1; ++h) {
     const uint32_t v = at(h);
@@ -183,13 +192,8 @@ __device__ __noinline__ void select_general(const uint16_t *__restrict__ d, uint
       ++rank;
     }
   }
-  // bitonic sort of (distance, index) over the next power of two
-  uint32_t n2 = 1;
-  while (n2 < half)
-    n2 <<= 1;
-  for (uint32_t i = half + tid; i < n2; i += kKnnThreads)
-    keys[i] = 0xffffffffu;
   __syncthreads();
+  // bitonic sort of (distance, index)
   for (uint32_t k = 2; k <= n2; k <<= 1) {
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
       for (uint32_t i = tid; i < n2; i += kKnnThreads) {
@@ -257,7 +261,7 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
         const uint32_t dist = (x[j >> 1] >> (16 * (j & 1))) & 0xffffu;
         if (dist <= u) {
           const uint32_t h = 8 * (i * kKnnThreads + tid) + j;
-          if (!(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
+          if (h < H && !(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
             const uint32_t n = atomicAdd(&found, 1u);
             if (n < kSelectMost)
               keys[n] = (dist << 16) | h;
@@ -422,11 +426,14 @@ __global__ void __launch_bounds__(kDistThreads)
 // distances (rows 2 i and 2 i + 1 of the chunk's i-th sample, `pitch` entries
 // apart, those past H excluded): the `half` nearest to its first haplotype, then
 // the `half` nearest to the second among those not taken, interleaved
-// (KNN::ClusterHaps, kNN.cpp:170-206).
+// (KNN::ClusterHaps, kNN.cpp:170-206).  Where a wait of the distances' kernel ran
+// out (kGemmTimeout in *error) they are not all there: the lists are filled with
+// kKnnNoHap, which a generation refuses, and glp_finish reports the flag.
 template <int kV>
 __global__ void __launch_bounds__(kKnnThreads)
     knn_select_kernel(const uint16_t *__restrict__ dist, uint32_t pitch, uint32_t H, uint32_t s0,
-                      uint32_t half, uint32_t dmax, uint32_t *__restrict__ neighbors) {
+                      uint32_t half, uint32_t dmax, const int *__restrict__ error,
+                      uint32_t *__restrict__ neighbors) {
   __shared__ __align__(16) uint32_t keys[kKnnMaxHalf];
   __shared__ uint32_t chosen[2 * kKnnMaxHalf];
   __shared__ uint32_t taken[kKnnMaxHaps / 32 + 1];
@@ -434,16 +441,22 @@ __global__ void __launch_bounds__(kKnnThreads)
   static_assert(kSelectMost <= kKnnMaxHalf, "keys");
   const uint32_t tid = threadIdx.x;
   const uint16_t *const row = dist + (size_t)2 * blockIdx.x * pitch;
+  uint32_t *const out = neighbors + (size_t)(s0 + blockIdx.x) * 2 * half;
+  if (*error & kGemmTimeout) {
+    for (uint32_t i = tid; i < 2 * half; i += kKnnThreads)
+      out[i] = kKnnNoHap;
+    return;
+  }
   for (uint32_t i = tid; i < (H + 31) / 32; i += kKnnThreads)
     taken[i] = 0;
   select_nearest<kV>(row, H, half, dmax, nullptr, half, keys, red, chosen);
   for (uint32_t i = tid; i < half; i += kKnnThreads)
-    atomicOr(&taken[chosen[i] >> 5], 1u << (chosen[i] & 31u));
+    if (chosen[i] < H)
+      atomicOr(&taken[chosen[i] >> 5], 1u << (chosen[i] & 31u));
   __syncthreads();
   // at most `half` of the second row's nearest are taken
   select_nearest<kV>(row + pitch, H, half, dmax, taken, 2 * half, keys, red,
                      chosen + kKnnMaxHalf);
-  uint32_t *const out = neighbors + (size_t)(s0 + blockIdx.x) * 2 * half;
   for (uint32_t i = tid; i < half; i += kKnnThreads) {
     out[2 * i] = chosen[i];
     out[2 * i + 1] = chosen[kKnnMaxHalf + i];

@@ -33,7 +33,7 @@ constexpr uint32_t kGemmABytes = kGemmM * kGemmK, kGemmBBytes = kGemmN * kGemmK;
 constexpr uint32_t kGemmStageBytes = kGemmABytes + kGemmBBytes;
 constexpr int kGemmThreads = 192;  // producer, product and four epilogue warps
 constexpr size_t kGemmSmem = 1024 + (size_t)kGemmStages * kGemmStageBytes;
-constexpr int kGemmTimeout = 2;  // error flag bit: a wait ran out
+constexpr uint64_t kGemmWaitNs = 2000000000ull;  // after which a wait gives up
 
 // Operand row length in bytes: whole steps of K.
 inline uint32_t knn_operand_pitch(uint32_t S) { return (S + kGemmK - 1) / kGemmK * kGemmK; }
@@ -92,8 +92,9 @@ __device__ __forceinline__ uint64_t global_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-// Waits for the phase of parity `parity`; false once two seconds have passed.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
+// Waits for the phase of parity `parity`; false once `limit` nanoseconds have passed.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
+                                          uint64_t limit = kGemmWaitNs) {
   uint64_t until = 0;
   for (uint32_t n = 0;; ++n) {
     uint32_t done;
@@ -109,7 +110,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     if ((n & 63u) == 63u) {
       const uint64_t now = global_ns();
       if (!until)
-        until = now + 2000000000ull;
+        until = now + limit;
       else if (now > until)
         return false;
     }
