@@ -44,6 +44,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "glp_join.h"
 #include "glp_rng.h"
 
 namespace glp {
@@ -518,41 +519,21 @@ __device__ __noinline__ double like_forward(const uint64_t *__restrict__ haps, u
   return log(sum) + (double)f.k * 0.69314718055994530942;
 }
 
-// a + b = s + err exactly.
-__device__ __forceinline__ float two_sum(float a, float b, float &err) {
-  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
-  return s;
-}
-
 // ln(x . y) + k ln 2 over the four states, in natural log and binary64.  The
 // exponent of the product joins k exactly, and the logarithm of its mantissa in
 // [1, 2) is taken in binary32 (absolute error below 3e-7, against
 // log-likelihoods of order -S), so binary64 only adds the two parts: its pipe
-// takes an instruction of a warp in 16 cycles.  For the same reason the product
-// itself is a pair of floats: the four products exact as a float and an error,
-// their sums too, so that the mantissa is rounded once, from a value good to 46
-// bits (in binary64 the products, sums and conversions took 820 cycles of a round
-// that has 3,600 beside its sites, now 70; a lone warp's round over 64 sites, with
-// the accept rule in binary32 as well, 3.64 and 3.18 us, over 1,024 15.7 and 15.3).
-// Products outside the range where the errors are floats (a blocked pass's never
-// are) and invalid ones go through binary64.
+// takes an instruction of a warp in 16 cycles.  For the same reason the mantissa
+// comes from pairs of floats where those give the same float as the binary64
+// product, and else from that (glp_join.h).  In binary64 alone the products, sums
+// and conversions took 820 cycles of a round that has 3,600 beside its sites, as
+// pairs 70; the test for the other case adds 0.1 us a round (a generation of 3 x 3
+// sites 83.4 and 84.5 us, larger ones within 0.2 %).
 __device__ __forceinline__ double log_dot(float2 xX, float2 xY, float2 yX, float2 yY, int k) {
   constexpr double kLn2 = 0.69314718055994530942;
-  const float p0 = __fmul_rn(xX.x, yX.x), p1 = __fmul_rn(xX.y, yX.y),
-              p2 = __fmul_rn(xY.y, yY.y), p3 = __fmul_rn(xY.x, yY.x);
-  float d0, d1, d2;
-  const float s0 = two_sum(p0, p1, d0), s1 = two_sum(p2, p3, d1), s = two_sum(s0, s1, d2);
-  const float r0 = __fadd_rn(fmaf(xX.x, yX.x, -p0), fmaf(xX.y, yX.y, -p1));
-  const float r1 = __fadd_rn(fmaf(xY.y, yY.y, -p2), fmaf(xY.x, yY.x, -p3));
-  const float hi = __fadd_rn(s, __fadd_rn(__fadd_rn(d0, d1), __fadd_rn(d2, __fadd_rn(r0, r1))));
   float m;
   int e;
-  if (hi >= 0x1p-60f && hi < 0x1p127f) {
-    const uint32_t bits = __float_as_uint(hi);
-    e = (int)(bits >> 23) - 127;
-    m = __uint_as_float((bits & 0x007fffffu) | 0x3f800000u);
-  } else {
+  if (!join_product(xX.x, xX.y, xY.y, xY.x, yX.x, yX.y, yY.y, yY.x, m, e)) {
     const double dot = (double)xX.x * (double)yX.x + (double)xX.y * (double)yX.y +
                        (double)xY.y * (double)yY.y + (double)xY.x * (double)yY.x;
     if (!(dot > 0x1p-1000))
