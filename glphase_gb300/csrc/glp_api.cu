@@ -716,16 +716,16 @@ uint64_t emission_bytes(const glp::GenParams &p) {
 // alone (2,000 x 8,192: 6.30 -> 5.64 ms a generation, eight uneven chunks 14.4 ->
 // 14.1; with the GPU full, 10,000 x 4,096, 7.39 -> 7.43).
 // Returns whether they exceed half of L2 (a half serves the SMs beside it).
-bool mark_stream(const glp_ctx *c, glp::GenParams *chunks, uint32_t count) {
+bool mark_stream(size_t l2_bytes, int sms, glp::GenParams *chunks, uint32_t count) {
   uint64_t bytes = 0, samples = 0;
   for (uint32_t i = 0; i < count; ++i) {
     bytes += emission_bytes(chunks[i]);
     samples += chunks[i].N;
   }
-  const bool few = count > 1 || samples * 8 <= (uint64_t)2 * 128 * c->sms;
+  const bool few = count > 1 || samples * 8 <= (uint64_t)2 * 128 * sms;
   for (uint32_t i = 0; i < count; ++i)
-    chunks[i].stream = bytes > c->l2_bytes && few ? 1u : 0u;
-  return 2 * bytes > c->l2_bytes;
+    chunks[i].stream = bytes > l2_bytes && few ? 1u : 0u;
+  return 2 * bytes > l2_bytes;
 }
 
 int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
@@ -734,7 +734,7 @@ int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
   if (rc)
     return rc;
   const bool vq = (a->flags & GLP_GEN_VQ) != 0;
-  const bool streams = mark_stream(c, &p, 1);
+  const bool streams = mark_stream(c->l2_bytes, c->sms, &p, 1);
   const Shape sh = choose_shape(c, a->num_samples, false, vq, a->pen, streams);
   const uint32_t P = sh.P;
   SingleFn fn = single_kernel(sh, vq);
@@ -1143,7 +1143,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     if (total > 0xffffffffull)
       return fail(c, GLP_ERR_ARG, "a batch holds at most 2^32-1 samples");
   }
-  const bool streams = mark_stream(c, c->h_table, count);
+  const bool streams = mark_stream(c->l2_bytes, c->sms, c->h_table, count);
   const WorkGrids work = batch_tables(c->h_table, count, c->h_offsets);
   if ((rc = ensure(c, c->d_table, c->table_cap, count)) ||
       (rc = ensure(c, c->d_offsets, c->offsets_cap, glp::batch_words(count))))
@@ -1263,7 +1263,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   glp_batch *b = new glp_batch();
   b->c = c;
   b->count = count;
-  const bool streams = mark_stream(c, table.data(), count);
+  const bool streams = mark_stream(c->l2_bytes, c->sms, table.data(), count);
   b->work = batch_tables(table.data(), count, offsets.data());
   b->chain_cycles = chain_cycles;
   cudaStream_t cs = nullptr;
@@ -1968,6 +1968,7 @@ struct NoallocSetup {
   unsigned long long ctx_id = 0;  // 0: slot unused
   unsigned char *base = nullptr;
   int sms = 0;
+  size_t l2_bytes = 0;
   double resident[kWidths] = {};
 };
 constexpr int kNoallocContexts = 16;
@@ -2025,11 +2026,13 @@ int noalloc_setup(NoallocSetup *out) {
   if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p)
     return GLP_ERR_CUDA;
   e.base = static_cast<unsigned char *>(p);
-  int dev = 0;
+  int dev = 0, l2 = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&e.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
       allow_chain_smem() != cudaSuccess)
     return GLP_ERR_CUDA;
+  e.l2_bytes = (size_t)l2;
   for (int i = 1; i < kWidths; ++i) {  // also sets each kernel's shared-memory attribute
     Shape sh;
     sh.P = 1u << i;
@@ -2153,10 +2156,12 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
 
   // speculation width for an acceptance rate of about 0.12 (the rule of
   // choose_lanes without a context's history), from the resident threads
-  // measured at set-up
+  // measured at set-up.  Without hmm_work the scratch bounds no rows: they may
+  // exceed L2 (20,000 x 512 at 8 lanes 1.70 ms; as for rows in L2, at 4, 2.33).
   bool known = true;
+  const bool streams = mark_stream(su.l2_bytes, sms, &p, 1);
   const uint32_t P = pick_lanes(
-      kUsualRate, N, sms, false, false, 128u,
+      kUsualRate, N, sms, false, streams, 128u,
       [](uint32_t w) {
         Shape s1;
         s1.P = w;
