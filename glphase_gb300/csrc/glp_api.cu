@@ -1867,7 +1867,9 @@ int glp_knn_neighbors(glp_ctx *c, const uint64_t *haps, uint32_t H, uint32_t S, 
                       (2 * n + glp::kTractQ - 1) / glp::kTractQ);
       auto fn = plan.sym ? glp::knn_tract_dist_kernel<true> : glp::knn_tract_dist_kernel<false>;
       fn<<<grid, glp::kDistThreads, 0, c->stream>>>(
-          haps, H, wn, c->d_mask, 2 * s0, 2 * n, pitch, c->d_knn_dist);
+          haps, H, wn, c->d_mask, 2 * s0, 2 * n, pitch,
+          glp::tract_exact_chunks(wn, plan.sym, (uint64_t)grid.x * grid.y / 2, c->sms),
+          c->d_knn_dist);
     } else if ((rc = knn_products(c, plan, haps, H, wn, 2 * s0, 2 * n))) {
       return rc;
     }

@@ -302,17 +302,20 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
 // sites minus the longest run.  A CTA takes 32 queries x 64 haplotypes, each
 // thread 2 x 4 pairs.  kSym: the queries are the whole panel; tiles below the
 // diagonal are not computed, their distances are written transposed.
+// Words go in two passes (see below), or, the first `exact` chunks of 8, in one with
+// each word's longest run found on its own, whose cost is the same for all
+// haplotypes (tract_exact_chunks).
 // Bound: the ALU instructions of a pair's word (89 % of that pipe).  4,990
-// haplotypes x 1,024 sites: 1.82 ms with all tiles and each 64-bit word's longest
-// run found on its own, 0.92 with the tiles of one half, 0.85 with `best` raised
-// inside one pass (it rises mostly in the first words, and every lane waits), 0.63
-// ms in two passes; 20,000 x 4,096 the table 119 -> 33 ms.
+// haplotypes x 1,024 sites, a table: 2.14 ms with all tiles in one pass, 0.76 with
+// the tiles of one half in two, 0.87 with the first chunk exact; of haplotypes that
+// agree at half of the sites at random (no long runs: `best` rises for longer, and
+// every lane waits) 2.14, 1.17 and 1.06.  20,000 x 4,096 119 -> 33 ms.
 constexpr uint32_t kTractQ = 32, kTractH = 64, kDistW = 8, kDistThreads = 256;
 template <bool kSym>
 __global__ void __launch_bounds__(kDistThreads)
     knn_tract_dist_kernel(const uint64_t *__restrict__ haps, uint32_t H, uint32_t wn,
                           const uint64_t *__restrict__ mask, uint32_t q0, uint32_t nq,
-                          uint32_t pitch, uint16_t *__restrict__ dist) {
+                          uint32_t pitch, uint32_t exact, uint16_t *__restrict__ dist) {
   const uint32_t hb = blockIdx.x * kTractH, qb = blockIdx.y * kTractQ;
   if (kSym && hb + kTractH <= qb)
     return;
@@ -321,20 +324,23 @@ __global__ void __launch_bounds__(kDistThreads)
   __shared__ uint64_t smask[kDistW];
   __shared__ uint16_t st[kSym ? kTractH : 1][kTractQ + 2];  // the tile transposed
   const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
+  const uint32_t chunks = (wn + kDistW - 1) / kDistW;
+  const bool all_exact = chunks <= exact;
   uint32_t common = 0;
+  int form = 0;  // of the runs inside: tract_inside32, _mid, _long
   OpenRun run[2][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      run[i][j] = OpenRun{0, kRunFloor};
-  // twice over the words: the runs that cross 32-site boundaries (and the words
-  // with sites that are not common), which leave `best` near the longest; then the
-  // runs inside, which seldom exceed it
+      run[i][j] = OpenRun{0, all_exact ? 0u : kRunFloor};
+  // twice over the words: the runs that cross 32-site boundaries (and all of the
+  // runs of exact words, and of words with sites that are not common), which leave
+  // `best` near the longest; then the runs inside, which seldom exceed it
 #pragma unroll 1
-  for (uint32_t chunk = 0, chunks = (wn + kDistW - 1) / kDistW; chunk < 2 * chunks; ++chunk) {
+  for (uint32_t chunk = 0; chunk < 2 * chunks - exact; ++chunk) {
     const bool inside = chunk >= chunks;
-    const uint32_t w0 = (inside ? chunk - chunks : chunk) * kDistW;
+    const uint32_t w0 = (inside ? chunk - chunks + exact : chunk) * kDistW;
     for (uint32_t i = tid; i < kTractQ * kDistW; i += kDistThreads) {
       const uint32_t r = i / kDistW, k = i % kDistW, w = w0 + k;
       sq[k][r] = (qb + r < nq && w < wn) ? __ldg(haps + (size_t)(q0 + qb + r) * wn + w) : 0ull;
@@ -358,18 +364,40 @@ __global__ void __launch_bounds__(kDistThreads)
         hv[j] = sh[k][tx + 16 * j];
       if (inside) {
         if (m == ~0ull) {
+          // the form of the test that all of the warp's pairs may use
+          if (form != 2) {
+            uint32_t least = run[0][0].best, most = least;
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              tract_inside32(run[i][j].best, (uint32_t)(qv[i] ^ hv[j]));
-              tract_inside32(run[i][j].best, (uint32_t)((qv[i] ^ hv[j]) >> 32));
-            }
+              for (int j = 0; j < 4; ++j) {
+                least = min(least, run[i][j].best);
+                most = max(most, run[i][j].best);
+              }
+            form = __all_sync(0xffffffffu, least >= kRunLong)                        ? 2
+                   : __all_sync(0xffffffffu, least >= kRunMid && most <= kRunMost) ? 1
+                                                                                   : 0;
+          }
+          auto inside_word = [&](auto test) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                test(run[i][j].best, (uint32_t)(qv[i] ^ hv[j]));
+                test(run[i][j].best, (uint32_t)((qv[i] ^ hv[j]) >> 32));
+              }
+          };
+          if (form == 2)
+            inside_word([](uint32_t &best, uint32_t x) { tract_inside32_long(best, x); });
+          else if (form == 1)
+            inside_word([](uint32_t &best, uint32_t x) { tract_inside32_mid(best, x); });
+          else
+            inside_word([](uint32_t &best, uint32_t x) { tract_inside32(best, x); });
         }
         continue;
       }
       common += tract_popc(m);
-      if (m == ~0ull) {
+      if (m == ~0ull && chunk >= exact) {
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -394,7 +422,7 @@ __global__ void __launch_bounds__(kDistThreads)
     for (int j = 0; j < 4; ++j) {
       const uint32_t h = hb + tx + 16 * j;
       uint32_t best = run[i][j].best;
-      if (best == kRunFloor && q < nq && h < H) {  // no longer run: its exact length
+      if (!all_exact && best == kRunFloor && q < nq && h < H) {  // no longer run: its exact length
         const uint64_t *const x = haps + (size_t)(q0 + q) * wn, *const y = haps + (size_t)h * wn;
         Tract t{0, 0, 0, 0};
         for (uint32_t w = 0; w < wn; ++w) {
@@ -420,6 +448,19 @@ __global__ void __launch_bounds__(kDistThreads)
         dist[(size_t)h * pitch + q] = st[r][tid & 31u];
     }
   }
+}
+
+// The chunks of 8 words that knn_tract_dist_kernel takes exactly: the first where
+// it is all of the words (`best` would rise inside most of them), where all tiles are
+// computed, or where fewer tiles than SMs leave a pair's chain of words to wait for;
+// none where tiles of one half fill the GPU.  Tables in ms with none / one, typical
+// haplotypes and (random ones): 14,000 x 64 2.13 / 0.84 (1.67 / 0.85), 14,000 x 512
+// 3.57 / 3.88 (5.82 / 3.90), 14,000 x 1,024 5.24 / 6.17 (8.38 / 7.80); all tiles,
+// 24,000 x 1,024 29.7 / 35.4 (48.2 / 44.5); few, 200 x 1,000 0.086 / 0.078 (0.114 /
+// 0.091), 600 x 1,024 0.100 / 0.095 (0.123 / 0.110).  In one pass over all tiles, as
+// before either: 2.29, 9.05, 15.9, 45.4, 0.097 and 0.120.
+inline uint32_t tract_exact_chunks(uint32_t wn, bool sym, uint64_t tiles, int sms) {
+  return wn <= kDistW || !sym || tiles <= (uint64_t)sms ? 1 : 0;
 }
 
 // The neighbour lists of the samples s0 + blockIdx.x from their rows of
