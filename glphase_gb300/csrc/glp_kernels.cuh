@@ -796,10 +796,13 @@ struct ChainTiles {  // of one recursion
   float4 t[kChainRing][kChainTile];  // transition rows
 };
 
-// 1.0f / x correctly rounded, for x in [2^-126, 2^126): one Newton step from
-// the approximate reciprocal.  Equal to __frcp_rn for every float of that
-// range (checked exhaustively), without its range test and branch in the
-// dependent chain.  Outside it: NaN below, 0 above.
+// 1 / x correctly rounded, for x in [2^-126, 2^126]: one Newton step y + y (1 - x y),
+// each product and sum fused, from the approximate reciprocal y.  Where y is within
+// a unit of its last place, 1 - x y is exact and the step's result correctly rounded
+// but for a mantissa of ones (P. Markstein, IA-64 and Elementary Functions, 2000,
+// chapter 8); that it is for every x of the range, those too, is what
+// test_gpu_reciprocal.py compares, float by float.  Outside: NaN below, 0 above, NaN
+// for infinity.
 __device__ __forceinline__ float recip_newton(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
