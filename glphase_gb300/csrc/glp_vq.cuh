@@ -36,13 +36,15 @@ constexpr uint32_t kVQBlock = kVQRun * kVQThreads;  // points per block
 // product a y, which can be two units off, within one.  The operands' range keeps
 // every remainder exact.  One reciprocal serves both quotients, and a zero
 // numerator (frequent: probabilities clamped at 0) takes the same path.
+// test_gpu_vq_quotient.py compares 10^10 quotients with the compiler's.
 __device__ __forceinline__ float vq_quotient(float a, float s, float y) {
   const float q0 = __fmul_rn(a, y);
   const float q1 = __fmaf_rn(__fmaf_rn(-s, q0, a), y, q0);
   return __fmaf_rn(__fmaf_rn(-s, q1, a), y, q1);
 }
 __device__ __forceinline__ bool vq_quotient_ok(float a) {
-  return a == 0.0f || (fabsf(a) >= 0x1p-80f && fabsf(a) <= 0x1p40f);
+  // +0, or of that range; the corrections would make -0 a +0
+  return __float_as_uint(a) == 0u || (fabsf(a) >= 0x1p-80f && fabsf(a) <= 0x1p40f);
 }
 __device__ __forceinline__ void vq_normalise(float g0, float g1, float g2, float &rr,
                                              float &het) {
