@@ -809,13 +809,21 @@ __device__ __forceinline__ float recip_newton(float x) {
   return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
 }
 
+// The same for any x: below 2^-126 by way of x 2^64 (both scalings are exact, or
+// overflow as the reciprocal does), 0 and above 2^126 by __frcp_rn.
+__device__ __forceinline__ float recip_any(float x) {
+  const float a = fabsf(x), scale = a < 0x1p-126f ? 0x1p64f : 1.0f;
+  const float r = recip_newton(x * scale) * scale;
+  return a == 0.0f || a > 0x1p126f ? __frcp_rn(x) : r;
+}
+
 // The normalisation of a step (impute.cpp:404-409, 441-446): the sum in the
-// reference's order, its reciprocal (kSafe: the division for any sum) and the
-// four products.  seen turns NaN with the reciprocal.
+// reference's order, its reciprocal (kSafe: for any sum) and the four products.
+// seen turns NaN with the reciprocal.
 template <bool kSafe>
 __device__ __forceinline__ States work_normalise(const States n, float &seen) {
   const float sum = __fadd_rn(__fadd_rn(__fadd_rn(n.P.x, n.P.y), n.Q.y), n.Q.x);
-  const float inv = kSafe ? __frcp_rn(sum) : recip_newton(sum);
+  const float inv = kSafe ? recip_any(sum) : recip_newton(sum);
   seen = fmaf(inv, 0.0f, seen);
   return States{__fmul2_rn(n.P, dup2(inv)), __fmul2_rn(n.Q, dup2(inv))};
 }
@@ -875,8 +883,8 @@ __device__ __forceinline__ void cp_async16_cg(void *smem, const void *gmem) {
 // descending.  kComb: the other recursion's vectors are staged with the
 // emissions and the products p are stored; else the vectors are.  Lane l has
 // sample s0 + l with the final quadruple q (lanes past the chunk's end repeat its
-// last sample and store nothing).
-template <bool kFwd, bool kComb>
+// last sample and store nothing).  kSafe: reciprocals for any sum.
+template <bool kFwd, bool kComb, bool kSafe>
 __device__ __forceinline__ void chain_run(const GenParams &p, ChainTiles &sm, uint32_t lane,
                                           uint32_t s0, uint4 q, States &v, float &seen, int base0,
                                           int n) {
@@ -948,10 +956,10 @@ __device__ __forceinline__ void chain_run(const GenParams &p, ChainTiles &sm, ui
       const uint32_t bit = 1u << o;
       const States s = pick_states(e, A0 & bit, A1 & bit, C0 & bit, C1 & bit);
       if (kFwd)
-        v = work_fwd_step<false>(v, s, t, seen);
+        v = work_fwd_step<kSafe>(v, s, t, seen);
       out[o] = f4_of(kComb ? mul_states(v, states_of(other)) : v);
       if (!kFwd)
-        v = work_bwd_step<false>(v, s, t, seen);
+        v = work_bwd_step<kSafe>(v, s, t, seen);
     };
     auto four = [&](const Rows &r, int half) {
 #pragma unroll
@@ -992,58 +1000,48 @@ __device__ __forceinline__ void chain_run(const GenParams &p, ChainTiles &sm, ui
   __syncwarp();
 }
 
-// The recursions of 32 samples by one warp, one after the other, with the
-// reference's division: for sums outside the fast reciprocal's range.
-inline __device__ __noinline__ void chains_any_sum(const GenParams &p, uint32_t s, uint4 q,
-                                                   bool valid) {
-  const float4 *e = p.emit + (size_t)s * p.S;
-  float4 *const beta = p.beta + (size_t)s * p.S;
-  float seen = 0.f;
-  auto picked = [&](uint32_t m) {
-    const Parents w = load_parents(p.haps, p.wn, q, m >> 6);
-    const uint32_t j = m & 63u;
-    return pick_states(__ldg(e + m), (w.f0 >> j) & 1, (w.f1 >> j) & 1, (w.m0 >> j) & 1,
-                       (w.m1 >> j) & 1);
-  };
-  States v = States{dup2(1.f), dup2(1.f)};
-  for (int m = (int)p.S - 1; m >= 0; --m) {
-    if (valid)
-      beta[m] = f4_of(v);
-    v = work_bwd_step<true>(v, picked((uint32_t)m), __ldg(p.tran4 + m), seen);
-  }
-  v = States{dup2(0.25f), dup2(0.25f)};
-  for (uint32_t m = 0; m < p.S; ++m) {
-    v = work_fwd_step<true>(v, picked(m), __ldg(p.tran4 + m), seen);
-    if (valid)
-      beta[m] = f4_of(mul_states(v, states_of(beta[m])));
-  }
-}
-
-// A block's samples s0 .. s0 + 31 of one chunk; tiles[0] backward, tiles[1]
-// forward.
-__device__ __forceinline__ void work_chains(const GenParams &p, uint32_t s0, ChainTiles *tiles) {
+// The recursions of a block's 32 samples, warp 0 the backward and warp 1 the forward
+// one.  True for every thread once a sum was outside the fast reciprocal's range
+// (never with kSafe): one below it left NaN in seen, one above it zeros, and with
+// them such a sum or no unit sum at a half's end.
+template <bool kSafe>
+__device__ __forceinline__ bool chains_run(const GenParams &p, uint32_t s0, uint4 q) {
+  extern __shared__ __align__(16) unsigned char glp_chain_smem[];
+  ChainTiles *const tiles = reinterpret_cast<ChainTiles *>(glp_chain_smem);  // 0 backward
   const uint32_t lane = threadIdx.x & 31u;
   const bool fwd = threadIdx.x >= 32;
-  const uint32_t s = min(s0 + lane, p.N - 1);
-  const uint4 q = make_uint4(p.quad_out[s], p.quad_out[p.N + s], p.quad_out[2 * (size_t)p.N + s],
-                             p.quad_out[3 * (size_t)p.N + s]);
   const int n = ((int)p.S + kChainTile - 1) / kChainTile, n_lo = n / 2, n_hi = n - n_lo;
   float seen = 0.f;
   States v = fwd ? States{dup2(0.25f), dup2(0.25f)} : States{dup2(1.f), dup2(1.f)};
+  auto special = [&]() {
+    return !kSafe && !(seen == 0.f && v.P.x + v.P.y + v.Q.x + v.Q.y > 0.5f);
+  };
   if (fwd)
-    chain_run<true, false>(p, tiles[1], lane, s0, q, v, seen, 0, n_lo);
+    chain_run<true, false, kSafe>(p, tiles[1], lane, s0, q, v, seen, 0, n_lo);
   else
-    chain_run<false, false>(p, tiles[0], lane, s0, q, v, seen, kChainTile * (n - 1), n_hi);
-  __syncthreads();  // both halves' vectors are stored
+    chain_run<false, false, kSafe>(p, tiles[0], lane, s0, q, v, seen, kChainTile * (n - 1), n_hi);
+  if (__syncthreads_or(special()))  // both halves' vectors are stored
+    return true;
   if (fwd)
-    chain_run<true, true>(p, tiles[1], lane, s0, q, v, seen, kChainTile * n_lo, n_hi);
+    chain_run<true, true, kSafe>(p, tiles[1], lane, s0, q, v, seen, kChainTile * n_lo, n_hi);
   else
-    chain_run<false, true>(p, tiles[0], lane, s0, q, v, seen, kChainTile * (n_lo - 1), n_lo);
-  // a sum below the fast reciprocal's range left NaN in seen; one above it left
-  // zeros, and with them such a sum (or no unit sum at the end)
-  const bool special = !(seen == 0.f && v.P.x + v.P.y + v.Q.x + v.Q.y > 0.5f);
-  if (__syncthreads_or(special) && !fwd)
-    chains_any_sum(p, s, q, s0 + lane < p.N);
+    chain_run<false, true, kSafe>(p, tiles[0], lane, s0, q, v, seen, kChainTile * (n_lo - 1),
+                                  n_lo);
+  return __syncthreads_or(special()) != 0;
+}
+
+// A block's samples s0 .. s0 + 31 of one chunk.  A block with a sum outside the fast
+// reciprocal's range starts over; the first halves cover every site, so it mostly
+// shows at the middle.  With such a site in every block hmm_work takes 0.187 ms for
+// 0.117 at 40 x 1,024, 0.207 for 0.129 at 2,000 x 1,024 and 0.73 for 0.53 at 10,000 x
+// 2,048 (by one warp, its rows not staged, it took 1.16, 1.79 and 5.2).  Both forms
+// are inlined: as a function of its own the second took a third longer.
+__device__ __forceinline__ void work_chains(const GenParams &p, uint32_t s0) {
+  const uint32_t s = min(s0 + (threadIdx.x & 31u), p.N - 1);
+  const uint4 q = make_uint4(p.quad_out[s], p.quad_out[p.N + s], p.quad_out[2 * (size_t)p.N + s],
+                             p.quad_out[3 * (size_t)p.N + s]);
+  if (chains_run<false>(p, s0, q))
+    chains_run<true>(p, s0, q);
 }
 
 inline __device__ __noinline__ float4 pow4(const float4 c, float pen) {
@@ -2066,10 +2064,9 @@ constexpr size_t kChainSmem = 2 * sizeof(ChainTiles);  // dynamic: one per recur
 
 template <class Src>
 __device__ __forceinline__ void chains_body(const Src &src) {
-  extern __shared__ __align__(16) unsigned char glp_chain_smem[];
   uint32_t c, s0;
   src.locate_block(blockIdx.x, c, s0);
-  work_chains(src.chunk(c), s0, reinterpret_cast<ChainTiles *>(glp_chain_smem));
+  work_chains(src.chunk(c), s0);
 }
 
 template <class Src>
