@@ -27,6 +27,7 @@
 #include "glp_server_core.h"
 #include "glp_knn.cuh"
 #include "glp_knn_gemm.cuh"
+#include "glp_knn_plan.h"
 #include "glp_launch.h"
 #include "glp_tally.cuh"
 #include "glp_vq.cuh"
@@ -761,34 +762,12 @@ int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
 
 namespace {
 
-// How a neighbour table is built: the samples whose distances are held at a
-// time, and for the Hamming metric the operand rows.
-struct KnnPlan {
-  bool tract = false, whole = false, sym = false;
-  uint32_t pitch = 0;    // entries of a row of distances
-  uint32_t chunk = 0;    // samples
-  uint32_t bytes = 0;    // of an operand row
-  uint32_t slab = 0;     // operand rows of queries, and of haplotypes, at a time
-};
-// The whole panel's operand is kept when it takes at most 1 GB (20,000 x 4,096:
-// 82 MB), else slabs of queries and of haplotypes share that.  With all distances
-// in at most 1 GB (and the operand whole), only the tiles on and above the
-// diagonal are computed; else chunks of 256 MB of distances.
-constexpr size_t kKnnOperandBytes = (size_t)1 << 30, kKnnSymBytes = (size_t)1 << 30;
-
-KnnPlan knn_plan(uint32_t H, uint32_t S, bool tract) {
-  KnnPlan p;
-  p.tract = tract;
-  p.pitch = glp::knn_pitch(H);
-  p.bytes = glp::knn_operand_pitch(S);
-  p.whole = (size_t)H * p.bytes <= kKnnOperandBytes;
-  p.slab = p.whole ? H : (uint32_t)(kKnnOperandBytes / 2 / p.bytes / 256 * 256);
-  p.sym = (tract || p.whole) && (size_t)H * p.pitch * sizeof(uint16_t) <= kKnnSymBytes;
-  p.chunk = p.sym ? H / 2
-                  : (uint32_t)std::min<size_t>(
-                        H / 2, std::max<size_t>(64, ((size_t)256 << 20) / (4 * (size_t)p.pitch)));
-  return p;
-}
+using glp::KnnPlan;
+// Most device memory that a neighbour table is planned with.
+#ifndef GLP_KNN_LIMIT
+#define GLP_KNN_LIMIT (~(size_t)0)
+#endif
+constexpr size_t kKnnLimit = GLP_KNN_LIMIT;
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                    const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -826,14 +805,22 @@ int expand_rows(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t h0,
   return GLP_OK;
 }
 
-// Workspace of the Hamming distances, the number of common sites, and the whole
-// panel's operand when it is kept.
+// The device memory of a plan; what is too small of it is given back first.
+int knn_reserve(glp_ctx *c, const KnnPlan &p) {
+  int rc = ensure(c, c->d_knn_dist, c->knn_dist_cap, p.dist_bytes() / sizeof(uint16_t));
+  if (!rc && !p.tract && !(rc = ensure(c, c->d_knn_sites, c->knn_sites_cap, 1)))
+    rc = ensure(c, c->d_knn_ops, c->knn_ops_cap, p.operand_bytes() / sizeof(uint4));
+  if (rc) {  // a smaller plan may follow
+    release(c->d_knn_dist);
+    release(c->d_knn_ops);
+    c->knn_dist_cap = c->knn_ops_cap = 0;
+    cudaGetLastError();
+  }
+  return rc;
+}
+
+// The number of common sites, and the whole panel's operand when it is kept.
 int knn_operands(glp_ctx *c, const KnnPlan &p, const uint64_t *haps, uint32_t H, uint32_t wn) {
-  int rc;
-  const size_t rows = p.whole ? (size_t)H : 2 * (size_t)p.slab;
-  if ((rc = ensure(c, c->d_knn_ops, c->knn_ops_cap, rows * (p.bytes / 16))) ||
-      (rc = ensure(c, c->d_knn_sites, c->knn_sites_cap, 1)))
-    return rc;
   GLP_CUDA(c, cudaFuncSetAttribute(glp::knn_gemm_kernel<false>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)glp::kGemmSmem));
@@ -1854,10 +1841,12 @@ int glp_knn_neighbors(glp_ctx *c, const uint64_t *haps, uint32_t H, uint32_t S, 
                 : H <= 5 * per ? glp::knn_select_kernel<5>
                                : glp::knn_select_kernel<13>;
   static_assert(13 * 8 * glp::kKnnThreads >= glp::kKnnMaxHaps, "the widest selection");
-  const KnnPlan plan = knn_plan(H, S, c->knn_metric == GLP_KNN_TRACT);
-  const uint32_t pitch = plan.pitch;
-  if ((rc = ensure(c, c->d_knn_dist, c->knn_dist_cap, (size_t)2 * plan.chunk * pitch)))
+  KnnPlan plan;
+  if ((rc = glp::knn_fitting_plan(H, S, c->knn_metric == GLP_KNN_TRACT, kKnnLimit,
+                                  GLP_ERR_NOMEM,
+                                  [&](const KnnPlan &p) { return knn_reserve(c, p); }, &plan)))
     return rc;
+  const uint32_t pitch = plan.pitch;
   if (!plan.tract && (rc = knn_operands(c, plan, haps, H, wn)))
     return rc;
   for (uint32_t s0 = 0; s0 < H / 2; s0 += plan.chunk) {

@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "glp_knn_plan.h"
 #include "glp_tract.h"
 
 namespace glp {
@@ -503,8 +504,5 @@ __global__ void __launch_bounds__(kKnnThreads)
     out[2 * i + 1] = chosen[kKnnMaxHalf + i];
   }
 }
-
-// Row length of the distances, in entries: whole 16-byte vectors.
-inline uint32_t knn_pitch(uint32_t H) { return (H + 127u) & ~127u; }
 
 }  // namespace glp

@@ -27,16 +27,13 @@
 
 namespace glp {
 
-constexpr uint32_t kGemmM = 128, kGemmN = 256, kGemmK = 128;  // K in sites = bytes
+constexpr uint32_t kGemmM = 128, kGemmN = 256, kGemmK = kKnnOperandStep;  // sites = bytes
 constexpr uint32_t kGemmStages = 2;
 constexpr uint32_t kGemmABytes = kGemmM * kGemmK, kGemmBBytes = kGemmN * kGemmK;
 constexpr uint32_t kGemmStageBytes = kGemmABytes + kGemmBBytes;
 constexpr int kGemmThreads = 192;  // producer, product and four epilogue warps
 constexpr size_t kGemmSmem = 1024 + (size_t)kGemmStages * kGemmStageBytes;
 constexpr uint64_t kGemmWaitNs = 2000000000ull;  // after which a wait gives up
-
-// Operand row length in bytes: whole steps of K.
-inline uint32_t knn_operand_pitch(uint32_t S) { return (S + kGemmK - 1) / kGemmK * kGemmK; }
 
 // Rows h0 .. h0 + rows - 1 of the panel as operand rows of `pitch` bytes, 16
 // sites a thread.  Bound: the stores (20,000 x 4,096: 82 MB).

@@ -332,7 +332,10 @@ void glp_server_destroy(glp_server *server);
  * insti -T, src/kNN.cpp:157-164).  haps and neighbors ([H/2][2*ceil(K/2)])
  * are DEVICE pointers; asynchronous, finish with glp_finish().  Replaces
  * KNN::KNN / KNN::ClusterHaps (src/kNN.cpp:7-206).  Needs H <= 50000 and
- * 2*ceil(K/2) <= H - 2. */
+ * 2*ceil(K/2) <= H - 2.  The context keeps the table's workspace: up to 1 GB
+ * of distances and 1 GB of operands (20,000 x 4,096: 886 MB); where that cannot
+ * be had the table is built in pieces of 256 MB in all, or less, and is the
+ * same.  If the device reports an error, the lists hold 0xffffffff. */
 int glp_knn_neighbors(glp_ctx *ctx, const uint64_t *haps, uint32_t num_haps, uint32_t num_sites,
                       uint32_t k, double freq_lb, double freq_ub, int use_maf,
                       uint32_t *neighbors);
