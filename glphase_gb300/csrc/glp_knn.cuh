@@ -221,7 +221,8 @@ template <int kV>
 __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, uint32_t H,
                                                uint32_t half, uint32_t dmax,
                                                const uint32_t *taken, uint32_t want,
-                                               uint32_t *keys, uint32_t *red, uint32_t *out) {
+                                               uint32_t *keys, uint32_t *red, uint32_t *out,
+                                               const int *error, int &flags) {
   const uint32_t tid = threadIdx.x;
   __shared__ uint32_t found;
   uint4 v[kV];
@@ -230,7 +231,16 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
     const uint32_t h = 8 * (i * kKnnThreads + tid);
     v[i] = h < H ? __ldg(reinterpret_cast<const uint4 *>(d + h))
                  : make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+    if (h < H && h + 8 > H) {  // H is even: whole pairs of entries past it
+      if (h + 2 >= H)
+        v[i].y = 0xffffffffu;
+      if (h + 4 >= H)
+        v[i].z = 0xffffffffu;
+      v[i].w = 0xffffffffu;
+    }
   }
+  if (error)  // beside the row's loads
+    flags = *error;
   if (tid == 0)
     found = 0;
   // the least distance of each thread; the pitch's padding is excluded like an own
@@ -262,7 +272,7 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
         const uint32_t dist = (x[j >> 1] >> (16 * (j & 1))) & 0xffffu;
         if (dist <= u) {
           const uint32_t h = 8 * (i * kKnnThreads + tid) + j;
-          if (h < H && !(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
+          if (!(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
             const uint32_t n = atomicAdd(&found, 1u);
             if (n < kSelectMost)
               keys[n] = (dist << 16) | h;
@@ -307,10 +317,10 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
 // each word's longest run found on its own, whose cost is the same for all
 // haplotypes (tract_exact_chunks).
 // Bound: the ALU instructions of a pair's word (89 % of that pipe).  4,990
-// haplotypes x 1,024 sites, a table: 2.14 ms with all tiles in one pass, 0.76 with
+// haplotypes x 1,024 sites, a table: 2.14 ms with all tiles in one pass, 0.74 with
 // the tiles of one half in two, 0.87 with the first chunk exact; of haplotypes that
 // agree at half of the sites at random (no long runs: `best` rises for longer, and
-// every lane waits) 2.14, 1.17 and 1.06.  20,000 x 4,096 119 -> 33 ms.
+// every lane waits) 2.14, 1.06 and 0.99.  20,000 x 4,096 119 -> 33 ms.
 constexpr uint32_t kTractQ = 32, kTractH = 64, kDistW = 8, kDistThreads = 256;
 template <bool kSym>
 __global__ void __launch_bounds__(kDistThreads)
@@ -328,7 +338,7 @@ __global__ void __launch_bounds__(kDistThreads)
   const uint32_t chunks = (wn + kDistW - 1) / kDistW;
   const bool all_exact = chunks <= exact;
   uint32_t common = 0;
-  int form = 0;  // of the runs inside: tract_inside32, _mid, _long
+  int form = 0;  // of the test inside: 0 tract_inside32, 1 _mid, 2 _long, 3 _any
   OpenRun run[2][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -375,9 +385,10 @@ __global__ void __launch_bounds__(kDistThreads)
                 least = min(least, run[i][j].best);
                 most = max(most, run[i][j].best);
               }
-            form = __all_sync(0xffffffffu, least >= kRunLong)                        ? 2
-                   : __all_sync(0xffffffffu, least >= kRunMid && most <= kRunMost) ? 1
-                                                                                   : 0;
+            form = __all_sync(0xffffffffu, least >= kRunLong)  ? 2
+                   : !__all_sync(0xffffffffu, least >= kRunMid) ? 0
+                   : __all_sync(0xffffffffu, most <= kRunMost)  ? 1
+                                                                : 3;
           }
           auto inside_word = [&](auto test) {
 #pragma unroll
@@ -390,6 +401,8 @@ __global__ void __launch_bounds__(kDistThreads)
           };
           if (form == 2)
             inside_word([](uint32_t &best, uint32_t x) { tract_inside32_long(best, x); });
+          else if (form == 3)
+            inside_word([](uint32_t &best, uint32_t x) { tract_inside32_any(best, x); });
           else if (form == 1)
             inside_word([](uint32_t &best, uint32_t x) { tract_inside32_mid(best, x); });
           else
@@ -453,15 +466,15 @@ __global__ void __launch_bounds__(kDistThreads)
 
 // The chunks of 8 words that knn_tract_dist_kernel takes exactly: the first where
 // it is all of the words (`best` would rise inside most of them), where all tiles are
-// computed, or where fewer tiles than SMs leave a pair's chain of words to wait for;
-// none where tiles of one half fill the GPU.  Tables in ms with none / one, typical
-// haplotypes and (random ones): 14,000 x 64 2.13 / 0.84 (1.67 / 0.85), 14,000 x 512
-// 3.57 / 3.88 (5.82 / 3.90), 14,000 x 1,024 5.24 / 6.17 (8.38 / 7.80); all tiles,
-// 24,000 x 1,024 29.7 / 35.4 (48.2 / 44.5); few, 200 x 1,000 0.086 / 0.078 (0.114 /
-// 0.091), 600 x 1,024 0.100 / 0.095 (0.123 / 0.110).  In one pass over all tiles, as
-// before either: 2.29, 9.05, 15.9, 45.4, 0.097 and 0.120.
+// computed and it is more than half of the words, and where fewer tiles than SMs
+// leave a pair's chain of words to wait for; else none.  Tables in ms with none /
+// one, typical haplotypes and (random ones), and in one pass over all tiles, as
+// before either: 14,000 x 64 2.21 / 0.82 (1.73 / 0.84), 2.29; 14,000 x 512 3.58 / 3.87
+// (5.95 / 3.89), 8.84; 14,000 x 1,024 5.31 / 6.21 (7.60 / 7.09), 15.9; all tiles,
+// 24,000 x 1,024 30.0 / 35.4 (43.4 / 40.4), 45.3; few, 200 x 1,000 0.074 / 0.072 (0.104
+// / 0.087), 0.098; 800 x 1,024 0.107 / 0.118 (0.130 / 0.121), 0.151.
 inline uint32_t tract_exact_chunks(uint32_t wn, bool sym, uint64_t tiles, int sms) {
-  return wn <= kDistW || !sym || tiles <= (uint64_t)sms ? 1 : 0;
+  return wn <= kDistW || (!sym && wn < 2 * kDistW) || tiles <= (uint64_t)sms ? 1 : 0;
 }
 
 // The neighbour lists of the samples s0 + blockIdx.x from their rows of
@@ -474,7 +487,7 @@ inline uint32_t tract_exact_chunks(uint32_t wn, bool sym, uint64_t tiles, int sm
 template <int kV>
 __global__ void __launch_bounds__(kKnnThreads)
     knn_select_kernel(const uint16_t *__restrict__ dist, uint32_t pitch, uint32_t H, uint32_t s0,
-                      uint32_t half, uint32_t dmax, const int *__restrict__ error,
+                      uint32_t half, uint32_t dmax, const int *error,
                       uint32_t *__restrict__ neighbors) {
   __shared__ __align__(16) uint32_t keys[kKnnMaxHalf];
   __shared__ uint32_t chosen[2 * kKnnMaxHalf];
@@ -484,24 +497,21 @@ __global__ void __launch_bounds__(kKnnThreads)
   const uint32_t tid = threadIdx.x;
   const uint16_t *const row = dist + (size_t)2 * blockIdx.x * pitch;
   uint32_t *const out = neighbors + (size_t)(s0 + blockIdx.x) * 2 * half;
-  if (*error & kGemmTimeout) {
-    for (uint32_t i = tid; i < 2 * half; i += kKnnThreads)
-      out[i] = kKnnNoHap;
-    return;
-  }
+  int flags = 0;
   for (uint32_t i = tid; i < (H + 31) / 32; i += kKnnThreads)
     taken[i] = 0;
-  select_nearest<kV>(row, H, half, dmax, nullptr, half, keys, red, chosen);
+  select_nearest<kV>(row, H, half, dmax, nullptr, half, keys, red, chosen, error, flags);
   for (uint32_t i = tid; i < half; i += kKnnThreads)
     if (chosen[i] < H)
       atomicOr(&taken[chosen[i] >> 5], 1u << (chosen[i] & 31u));
   __syncthreads();
   // at most `half` of the second row's nearest are taken
   select_nearest<kV>(row + pitch, H, half, dmax, taken, 2 * half, keys, red,
-                     chosen + kKnnMaxHalf);
+                     chosen + kKnnMaxHalf, nullptr, flags);
+  const bool failed = (flags & kGemmTimeout) != 0;
   for (uint32_t i = tid; i < half; i += kKnnThreads) {
-    out[2 * i] = chosen[i];
-    out[2 * i + 1] = chosen[kKnnMaxHalf + i];
+    out[2 * i] = failed ? kKnnNoHap : chosen[i];
+    out[2 * i + 1] = failed ? kKnnNoHap : chosen[kKnnMaxHalf + i];
   }
 }
 

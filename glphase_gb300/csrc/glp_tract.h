@@ -166,6 +166,19 @@ GLP_TRACT_FN void tract_inside32_mid(uint32_t &best, uint32_t x) {
     tract_inside32(best, x);
 }
 
+// The same for `best` from kRunMid, without that bound.
+GLP_TRACT_FN void tract_inside32_any(uint32_t &best, uint32_t x) {
+  const uint32_t r1 = ~x, r2 = r1 & (r1 >> 1), r4 = r2 & (r2 >> 2), r8 = r4 & (r4 >> 4),
+                 r16 = r8 & (r8 >> 8);
+  for (;;) {
+    const uint32_t from = best < 7 ? r4 : best < 15 ? r8 : r16,
+                   by = best - (best < 7 ? 3u : best < 15 ? 7u : 15u);
+    if (!(from & (from >> (by < 31u ? by : 31u))))
+      break;
+    ++best;
+  }
+}
+
 // The same for `best` of at least kRunLong.
 GLP_TRACT_FN void tract_inside32_long(uint32_t &best, uint32_t x) {
   const uint32_t r1 = ~x, r2 = r1 & (r1 >> 1), r4 = r2 & (r2 >> 2), r8 = r4 & (r4 >> 4),
