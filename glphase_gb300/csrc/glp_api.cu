@@ -137,7 +137,7 @@ struct glp_ctx {
   int knn_metric = GLP_KNN_HAMMING;  // glp_set_knn_metric
   bool short_blocks = false;
   // resident threads per lane width (1 .. 32), per [multi-chunk][VQ] kernel
-  double resident[2][2][8] = {};  // by the logarithm of the lanes
+  double resident[2][2][glp::kWidths] = {};  // by the logarithm of the lanes
   bool resident_known[2][2] = {};
   uint32_t lanes_used = 4;
   double last_accept = -1.0;  // acceptance rate of the last generation
@@ -454,100 +454,13 @@ double resident_threads(Fn fn, uint32_t P, int sms) {
 // Acceptance rate of a generation that nothing is known of.
 constexpr double kUsualRate = 0.12;
 
-// The positions that a chain goes on a round, on average: the chances that the
-// scored nodes of its speculation tree are reached.
-double steps_a_round(double a, uint32_t P) {
-  static constexpr glp::SpecTrees trees = glp::make_spec_trees();
-  static constexpr glp::TeamTrees teams = glp::make_team_trees();
-  int rate = std::min((int)(a * 16.0 + 0.5), glp::kSpecRates - 1);
-  if (!glp::kSpecTree((int)P))
-    rate = 0;
-  double sum = 0.0;
-  for (uint32_t i = 0; i < P / 2; ++i) {
-    int accepted, depth;
-    if (P > 32) {
-      const glp::TeamNode &t = teams.node[rate][i];
-      accepted = __builtin_popcount(t.taken[0]) + __builtin_popcount(t.taken[1]);
-      depth = (int)(t.desc & 255u);
-    } else {
-      const glp::SpecNode &t = trees.node[rate][i];
-      accepted = __builtin_popcount(t.accept);
-      depth = __builtin_popcount(t.path);
-    }
-    sum += std::pow(a, accepted) * std::pow(1.0 - a, depth - accepted);
-  }
-  return sum;
-}
-
-// Speculation width for N samples at acceptance rate a.  A generation lasts as
-// long as its longest chain while every sample has a group of its own, so the
-// rule compares, for each width, the rounds of a chain whose rate is off the
-// average, a or a' = a + min(a, 0.12), whichever goes on fewer positions a round,
-// times what a warp's round costs at the warps a scheduler holds.  Measured
-// (1,024 sites, a = 0.12, times of a generation kernel relative to one warp a
-// scheduler): 1.44 at two, 2.0 at three, beyond that in proportion (whole blocks of
-// four warps, so the steps are at multiples of the SM count).  Narrow groups stage
-// more rows a lane and read a row for fewer evaluations: at 4 lanes 1.25, on VQ
-// codes 1.5, and where the rows exceed half of L2 1.9 (measured against 8 lanes 1.5
-// to 2.2: 20,000 x 512 at 8 lanes 1.65 ms, 4: 2.37; 15,000 x 2,048 4.66 and 8.28;
-// 40,000 x 100, whose rows stay, 2.36 and 2.02); at 2 lanes, one block an SM, 2.7;
-// at 8 lanes 1.05, and 1.1 for such rows (2,000 x 4,096 2.65 ms, 16: 2.35); on VQ
-// codes, whose table reads conflict more in a wide group, 1.15 from 32.  The widths
-// this picks, against others: 256 samples 64 lanes 0.27 ms (32: 0.36, 8: 0.55),
-// 1,000 samples 16 lanes 0.55 (0.76; 32: 0.64), 1,500 x 2,048 8 lanes 1.07 (16:
-// 1.14), 2,500 x 2,048 16 lanes 1.42 (8: 1.51), 3,001 x 4,000 from codes 16 lanes
-// 3.47 (8: 3.68; 32: 4.52), 10,000 samples 8 lanes 2.05 (16: 2.49).
-// 64 and 128 lanes are teams of two and four warps, for one chunk alone.  They are
-// picked while every warp has a scheduler of its own: 152 x 1,024 128 lanes 0.237 ms
-// (32: 0.369), 300 64 lanes 0.281 (0.355), 400 32 lanes 0.353.
-constexpr int kWidths = 8;  // 1 << 0 .. 1 << 7 lanes
-double lane_round_cost(uint32_t P, bool vq, bool streams) {
-  switch (P) {
-    case 2: return 2.7;
-    case 4: return vq ? 1.5 : streams ? 1.9 : 1.25;
-    case 8: return streams ? 1.1 : 1.05;
-    case 16: return 1.0;
-    default: return vq ? 1.15 : 1.0;
-  }
-}
-
+// Resident threads for each width (kWidths of them, by the logarithm of the lanes)
+// up to `widest`, 0 for one lane.
 template <class FnOf>
-uint32_t pick_lanes(double a, uint64_t N, int sms, bool vq, bool streams, uint32_t widest,
-                    FnOf kernel_for, double *cache = nullptr, bool *known = nullptr) {
-  double local[kWidths] = {};
-  double *res = cache ? cache : local;
-  if (!known || !*known) {
-    res[0] = 0.0;
-    for (int i = 1; 1u << i <= widest; ++i)
-      res[i] = resident_threads(kernel_for(1u << i), 1u << i, sms);
-    if (known)
-      *known = true;
-  }
-  const double as = std::min(a + std::min(a, 0.12), 1.0);
-  uint32_t best = 8;
-  double best_time = 0;
-  for (int i = 1; 1u << i <= widest; ++i) {
-    if (res[i] <= 0)
-      continue;
-    const uint32_t P = 1u << i;
-    const double consumed = std::min(steps_a_round(a, P), steps_a_round(as, P));
-    const uint64_t per_block = (uint64_t)glp::kThreads / P;
-    const uint64_t blocks = (N + per_block - 1) / per_block;
-    // blocks an SM holds at a time, and for one warp a scheduler in each
-    const double most = std::max(1.0, res[i] / ((double)glp::kThreads * sms));
-    const double held = (double)((blocks + sms - 1) / sms);
-    auto warps_cost = [](double w) { return w <= 1 ? 1.0 : w <= 2 ? 1.44 : w * (2.0 / 3.0); };
-    const double warps = held <= most
-                             ? warps_cost(held * glp::kWarps / 4.0)
-                             : warps_cost(most * glp::kWarps / 4.0) * ((double)blocks / sms) / most;
-    const double cost = lane_round_cost(P, vq, streams);
-    const double time = warps * cost / consumed;
-    if (best_time == 0 || time < best_time * 0.98) {
-      best_time = time;
-      best = P;
-    }
-  }
-  return best;
+void resident_widths(double *res, uint32_t widest, int sms, FnOf kernel_for) {
+  res[0] = 0.0;
+  for (int i = 1; 1u << i <= widest; ++i)
+    res[i] = resident_threads(kernel_for(1u << i), 1u << i, sms);
 }
 
 // The acceptance rate that a launch with penalty pen is expected to have: the last
@@ -560,14 +473,26 @@ double expected_rate(const glp_ctx *c, float pen) {
 uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bool streams) {
   if (c->lanes)
     return c->lanes;
-  return pick_lanes(
-      expected_rate(c, pen), N, c->sms, vq, streams, multi ? 32u : 128u,
-      [&](uint32_t P) {
-        Shape sh;
-        sh.P = P;
-        return multi ? (const void *)multi_kernel(sh, vq) : (const void *)single_kernel(sh, vq);
-      },
-      c->resident[multi][vq], &c->resident_known[multi][vq]);
+  const uint32_t widest = multi ? 32u : 128u;
+  double *const resident = c->resident[multi ? 1 : 0][vq ? 1 : 0];
+  bool &known = c->resident_known[multi ? 1 : 0][vq ? 1 : 0];
+  if (!known)
+    resident_widths(resident, widest, c->sms, [&](uint32_t P) {
+      Shape sh;
+      sh.P = P;
+      return multi ? (const void *)multi_kernel(sh, vq) : (const void *)single_kernel(sh, vq);
+    });
+  known = true;
+  glp::WidthAsk ask;
+  ask.rate = expected_rate(c, pen);
+  ask.samples = N;
+  ask.sms = c->sms;
+  ask.vq = vq;
+  ask.streams = streams;
+  ask.widest = widest;
+  ask.block_threads = glp::kThreads;
+  ask.resident = resident;
+  return glp::pick_lanes(ask);
 }
 
 // Lanes from choose_lanes (a request below two lanes gets two: one
@@ -1960,7 +1885,7 @@ struct NoallocSetup {
   unsigned char *base = nullptr;
   int sms = 0;
   size_t l2_bytes = 0;
-  double resident[kWidths] = {};
+  double resident[glp::kWidths] = {};
 };
 constexpr int kNoallocContexts = 16;
 std::mutex g_noalloc_mutex;
@@ -2024,13 +1949,14 @@ int noalloc_setup(NoallocSetup *out) {
       allow_chain_smem() != cudaSuccess)
     return GLP_ERR_CUDA;
   e.l2_bytes = (size_t)l2;
-  for (int i = 1; i < kWidths; ++i) {  // also sets each kernel's shared-memory attribute
-    Shape sh;
-    sh.P = 1u << i;
-    e.resident[i] = resident_threads(single_kernel(sh, false), sh.P, e.sms);
+  resident_widths(e.resident, 128u, e.sms, [](uint32_t P) {  // also sets each kernel's
+    Shape sh;                                                  // shared-memory attribute
+    sh.P = P;
+    return (const void *)single_kernel(sh, false);
+  });
+  for (int i = 1; i < glp::kWidths; ++i)
     if (e.resident[i] <= 0)
       return GLP_ERR_CUDA;
-  }
   // the lookup above made a context current if there was none
   e.ctx_id = id ? id : current_ctx_id();
   if (e.ctx_id) {
@@ -2149,16 +2075,15 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   // choose_lanes without a context's history), from the resident threads
   // measured at set-up.  Without hmm_work the scratch bounds no rows: they may
   // exceed L2 (20,000 x 512 at 8 lanes 1.70 ms; as for rows in L2, at 4, 2.33).
-  bool known = true;
-  const bool streams = mark_stream(su.l2_bytes, sms, &p, 1);
-  const uint32_t P = pick_lanes(
-      kUsualRate, N, sms, false, streams, 128u,
-      [](uint32_t w) {
-        Shape s1;
-        s1.P = w;
-        return (const void *)single_kernel(s1, false);
-      },
-      su.resident, &known);
+  glp::WidthAsk ask;
+  ask.rate = kUsualRate;
+  ask.samples = N;
+  ask.sms = sms;
+  ask.streams = mark_stream(su.l2_bytes, sms, &p, 1);
+  ask.widest = 128u;
+  ask.block_threads = glp::kThreads;
+  ask.resident = su.resident;
+  const uint32_t P = glp::pick_lanes(ask);
   Shape sh;
   sh.P = P;
   SingleFn fn = single_kernel(sh, false);

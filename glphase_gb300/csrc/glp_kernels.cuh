@@ -46,6 +46,7 @@
 
 #include "glp_join.h"
 #include "glp_rng.h"
+#include "glp_width.h"
 
 namespace glp {
 
@@ -1168,43 +1169,6 @@ struct SpecNode {
   uint32_t accept;  // those of them whose proposal it has accepted
   uint32_t desc;    // [0, 4) depth, [4, 8) the last of those, [8, 24) their depths
 };
-constexpr int kSpecNodes = 16;  // a warp's lane pairs
-constexpr int kTeamNodes = 64;  // a team's of four warps
-constexpr int kSpecRates = 17;  // tree i is made for a = i / 16
-// Node n of a tree hangs from node parent[n], by acceptance or refusal.
-struct SpecShape {
-  int parent[kTeamNodes];
-  bool accept[kTeamNodes];
-};
-constexpr SpecShape make_spec_shape(int i) {
-  const double a = i == 0 ? 0.02 : i == 16 ? 0.98 : i / 16.0;
-  SpecShape t{};
-  double prob[kTeamNodes] = {};
-  double weight[kTeamNodes][2] = {};  // of the two children, 0 once they are there
-  prob[0] = 1.0;
-  weight[0][0] = 1 - a;
-  weight[0][1] = a;
-  for (int n = 1; n < kTeamNodes; ++n) {
-    int from = 0, dec = 0;
-    for (int v = 0; v < n; ++v)
-      for (int d = 0; d < 2; ++d)
-        if (weight[v][d] > weight[from][dec]) {
-          from = v;
-          dec = d;
-        }
-    t.parent[n] = from;
-    t.accept[n] = dec != 0;
-    prob[n] = prob[from] * (dec ? a : 1 - a);
-    weight[n][0] = prob[n] * (1 - a);
-    weight[n][1] = prob[n] * a;
-    // beside a refusal's child a quarter of an acceptance's is not needed: the next
-    // position replaces the same slot (generation_body)
-    if (!dec && weight[from][1] > 0.0)
-      weight[from][1] *= 0.75;
-    weight[from][dec] = 0.0;
-  }
-  return t;
-}
 struct SpecTrees {
   SpecNode node[kSpecRates][kSpecNodes];
 };
@@ -1262,12 +1226,6 @@ static __device__ const TeamTrees kTeamTrees = make_team_trees();
 // A chain's rate moves with weight 1 / 24 a cycle from the generation's (with 1 / 6,
 // chains of 10,000 samples took 0.8 % more rounds, 3 x 3 sites 1 % fewer).
 constexpr float kRateWeight = 24.0f;
-// Kernels that start with 16 lanes a sample or more take trees.  Below, four nodes
-// or fewer differ from the line of refusals only where a chain accepts more than 40
-// % of its proposals, and the kernel without them is the faster one (3,001 x 4,000
-// from codes at 8 lanes 4.39 and 4.46 ms, 10,000 x 4,096 7.36 and 7.40).
-constexpr bool kSpecTree(int P) { return P >= 16; }
-
 // The accept rule compares a uniform u with a float f: f > u for a float f exactly
 // when f > bound, and u = 0 has the bound -0.
 __device__ __forceinline__ float accept_bound(double u) {
