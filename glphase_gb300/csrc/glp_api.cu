@@ -473,7 +473,7 @@ double expected_rate(const glp_ctx *c, float pen) {
 uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bool streams) {
   if (c->lanes)
     return c->lanes;
-  const uint32_t widest = multi ? 32u : 128u;
+  const uint32_t widest = multi ? 32u : glp::kWidest;
   double *const resident = c->resident[multi ? 1 : 0][vq ? 1 : 0];
   bool &known = c->resident_known[multi ? 1 : 0][vq ? 1 : 0];
   if (!known)
@@ -1949,12 +1949,12 @@ int noalloc_setup(NoallocSetup *out) {
       allow_chain_smem() != cudaSuccess)
     return GLP_ERR_CUDA;
   e.l2_bytes = (size_t)l2;
-  resident_widths(e.resident, 128u, e.sms, [](uint32_t P) {  // also sets each kernel's
+  resident_widths(e.resident, glp::kWidest, e.sms, [](uint32_t P) {  // also sets each kernel's
     Shape sh;                                                  // shared-memory attribute
     sh.P = P;
     return (const void *)single_kernel(sh, false);
   });
-  for (int i = 1; i < glp::kWidths; ++i)
+  for (int i = 1; 1u << i <= glp::kWidest; ++i)
     if (e.resident[i] <= 0)
       return GLP_ERR_CUDA;
   // the lookup above made a context current if there was none
@@ -2080,7 +2080,7 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   ask.samples = N;
   ask.sms = sms;
   ask.streams = mark_stream(su.l2_bytes, sms, &p, 1);
-  ask.widest = 128u;
+  ask.widest = glp::kWidest;
   ask.block_threads = glp::kThreads;
   ask.resident = su.resident;
   const uint32_t P = glp::pick_lanes(ask);

@@ -55,6 +55,8 @@ namespace glp {
 #endif
 constexpr int kWarps = GLP_GEN_WARPS;  // warps per generation block
 constexpr int kThreads = 32 * kWarps;
+// Most lanes per sample: teams of two and four warps are whole parts of a block.
+constexpr uint32_t kWidest = kWarps % 4 == 0 ? 128 : kWarps % 2 == 0 ? 64 : 32;
 // Resident blocks per SM the generation kernels are compiled for (the launch
 // bound's minimum): with 3 the compiler may use up to 168 registers a thread and
 // takes 120-136, so 3 blocks of the 8- and 16-lane kernels fit.  A bound of 4 (a cap
@@ -1847,6 +1849,7 @@ struct __align__(16) TeamShare {
 template <int W, class E, int kSub>
 __device__ __forceinline__ void generation_team(const GenParams &p, const float4 *vq_smem) {
   static_assert(W == 2 || W == 4, "W");
+  static_assert(kWarps % W == 0, "a block holds whole teams");
   constexpr unsigned FULL = 0xffffffffu;
   constexpr uint32_t kNodes = (uint32_t)(kSpecNodes * W), kLanes = 32u * W;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, wt = warp % W,

@@ -41,7 +41,8 @@ MultiFn multi_kernel_vq_sub4(uint32_t P);
       default: return KERNEL<32, EMIT, SUB>;                 \
     }                                                        \
   }
-#define GLP_GEN_TEAMS(KERNEL, EMIT, SUB)   \
-  case 64: return KERNEL<64, EMIT, SUB>;   \
-  case 128: return KERNEL<128, EMIT, SUB>;
+// Teams wider than a block of the build's warps holds (kWidest) are not there.
+#define GLP_GEN_TEAMS(KERNEL, EMIT, SUB)                                  \
+  case 64: return KERNEL<(kWidest >= 64 ? 64 : 32), EMIT, SUB>;           \
+  case 128: return KERNEL<(kWidest >= 128 ? 128 : 32), EMIT, SUB>;
 #define GLP_GEN_NO_TEAMS(KERNEL, EMIT, SUB)
