@@ -1839,8 +1839,8 @@ struct __align__(16) TeamShare {
 // tree.  The chains are as long as before in evaluations and shorter in rounds (at
 // a = 0.12 a round goes on 7.3, 8.8 and 10.6 positions with 16, 32 and 64 nodes), and
 // the added warps run on schedulers that would stand idle.  Each warp stages the
-// sample's rows for itself; the warps meet at three barriers a round, for the
-// likelihoods, the votes and the nodes reached.  Where a round ends with an
+// sample's rows for itself; the warps meet at four barriers a round: for the
+// draws, the likelihoods, the votes and the nodes reached.  Where a round ends with an
 // acceptance the chain starts its next one there: the tree has that child mostly.
 // Measured, a team against one warp a chain: 60 x 1,024 0.351 and 0.234 ms (four
 // warps), 256 x 1,024 0.356 and 0.265 (two), 100 x 8,192 2.55 and 1.47, 3 x 3 0.056
@@ -1894,7 +1894,10 @@ __device__ __forceinline__ void generation_team(const GenParams &p, const float4
           window[cyc & wmask] = make_draw(p, s, cyc, p.error);
         drawn += kLanes;
       }
-      meet();  // the draws are there, and what the last round shared is read
+      // The draws are there.  And every warp has read what the last round shared: its
+      // likelihoods, quadruples, votes and nodes reached are written over below, and
+      // nothing but this barrier stands between.
+      meet();
       uint4 myq = q;
       float u = 0.0f;
       if (scores) {
