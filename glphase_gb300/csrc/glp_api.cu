@@ -470,7 +470,28 @@ double expected_rate(const glp_ctx *c, float pen) {
                                                       : std::max(c->last_accept, 1e-3);
 }
 
-uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bool streams) {
+// What the width rule is asked for `count` chunks.
+glp::WidthAsk width_ask(const glp::GenParams *chunks, uint32_t count, double rate, bool vq,
+                        int sms, size_t l2_bytes) {
+  glp::WidthAsk ask;
+  double sites = 0.0, cycles = 0.0;
+  for (uint32_t i = 0; i < count; ++i) {
+    ask.samples += chunks[i].N;
+    sites += (double)chunks[i].N * chunks[i].S;
+    cycles += (double)chunks[i].N * chunks[i].C;
+  }
+  ask.rate = rate;
+  ask.sites = sites / (double)ask.samples;
+  ask.cycles = cycles / (double)ask.samples;
+  ask.vq = vq;
+  ask.sms = sms;
+  ask.l2_bytes = (double)l2_bytes;
+  ask.block_threads = glp::kThreads;
+  return ask;
+}
+
+uint32_t choose_lanes(glp_ctx *c, const glp::GenParams *chunks, uint32_t count, bool multi,
+                      bool vq) {
   if (c->lanes)
     return c->lanes;
   const uint32_t widest = multi ? 32u : glp::kWidest;
@@ -483,24 +504,20 @@ uint32_t choose_lanes(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bo
       return multi ? (const void *)multi_kernel(sh, vq) : (const void *)single_kernel(sh, vq);
     });
   known = true;
-  glp::WidthAsk ask;
-  ask.rate = expected_rate(c, pen);
-  ask.samples = N;
-  ask.sms = c->sms;
-  ask.vq = vq;
-  ask.streams = streams;
+  glp::WidthAsk ask =
+      width_ask(chunks, count, expected_rate(c, chunks[0].pen), vq, c->sms, c->l2_bytes);
   ask.widest = widest;
-  ask.block_threads = glp::kThreads;
   ask.resident = resident;
   return glp::pick_lanes(ask);
 }
 
 // Lanes from choose_lanes (a request below two lanes gets two: one
 // evaluation a round), normalisation block from the context's rule.
-Shape choose_shape(glp_ctx *c, uint64_t N, bool multi, bool vq, float pen, bool streams) {
+Shape choose_shape(glp_ctx *c, const glp::GenParams *chunks, uint32_t count, bool multi,
+                   bool vq) {
   Shape sh;
-  sh.P = std::max<uint32_t>(2u, choose_lanes(c, N, multi, vq, pen, streams));
-  c->launch_pen = pen;
+  sh.P = std::max<uint32_t>(2u, choose_lanes(c, chunks, count, multi, vq));
+  c->launch_pen = chunks[0].pen;
   if (c->block_sites == 4 || (c->block_sites == 0 && c->short_blocks))
     sh.sub = 2;
   return sh;
@@ -641,8 +658,7 @@ uint64_t emission_bytes(const glp::GenParams &p) {
 // 8-lane warps a scheduler, or chunks of different lengths, whose longest ends
 // alone (2,000 x 8,192: 6.30 -> 5.64 ms a generation, eight uneven chunks 14.4 ->
 // 14.1; with the GPU full, 10,000 x 4,096, 7.39 -> 7.43).
-// Returns whether they exceed half of L2 (a half serves the SMs beside it).
-bool mark_stream(size_t l2_bytes, int sms, glp::GenParams *chunks, uint32_t count) {
+void mark_stream(size_t l2_bytes, int sms, glp::GenParams *chunks, uint32_t count) {
   uint64_t bytes = 0, samples = 0;
   for (uint32_t i = 0; i < count; ++i) {
     bytes += emission_bytes(chunks[i]);
@@ -651,7 +667,6 @@ bool mark_stream(size_t l2_bytes, int sms, glp::GenParams *chunks, uint32_t coun
   const bool few = count > 1 || samples * 8 <= (uint64_t)2 * 128 * sms;
   for (uint32_t i = 0; i < count; ++i)
     chunks[i].stream = bytes > l2_bytes && few ? 1u : 0u;
-  return 2 * bytes > l2_bytes;
 }
 
 int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
@@ -660,8 +675,8 @@ int launch_single(glp_ctx *c, glp_problem *pb, const glp_generation_args *a) {
   if (rc)
     return rc;
   const bool vq = (a->flags & GLP_GEN_VQ) != 0;
-  const bool streams = mark_stream(c->l2_bytes, c->sms, &p, 1);
-  const Shape sh = choose_shape(c, a->num_samples, false, vq, a->pen, streams);
+  mark_stream(c->l2_bytes, c->sms, &p, 1);
+  const Shape sh = choose_shape(c, &p, 1, false, vq);
   const uint32_t P = sh.P;
   SingleFn fn = single_kernel(sh, vq);
   const unsigned grid = grid_for(c, fn, a->num_samples, P, &rc);
@@ -1055,7 +1070,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
     if (total > 0xffffffffull)
       return fail(c, GLP_ERR_ARG, "a batch holds at most 2^32-1 samples");
   }
-  const bool streams = mark_stream(c->l2_bytes, c->sms, c->h_table, count);
+  mark_stream(c->l2_bytes, c->sms, c->h_table, count);
   const WorkGrids work = batch_tables(c->h_table, count, c->h_offsets);
   if ((rc = ensure(c, c->d_table, c->table_cap, count)) ||
       (rc = ensure(c, c->d_offsets, c->offsets_cap, glp::batch_words(count))))
@@ -1072,7 +1087,7 @@ int glp_run_batch(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   mp.counter = &c->d_record->counter;
   mp.stats = c->d_record->stats;
   mp.error = &c->d_record->error;
-  const Shape sh = choose_shape(c, total, true, vq, c->h_table[0].pen, streams);
+  const Shape sh = choose_shape(c, c->h_table, count, true, vq);
   const uint32_t P = sh.P;
   MultiFn fn = multi_kernel(sh, vq);
   const unsigned grid = grid_for(c, fn, total, P, &rc);
@@ -1175,7 +1190,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   glp_batch *b = new glp_batch();
   b->c = c;
   b->count = count;
-  const bool streams = mark_stream(c->l2_bytes, c->sms, table.data(), count);
+  mark_stream(c->l2_bytes, c->sms, table.data(), count);
   b->work = batch_tables(table.data(), count, offsets.data());
   b->chain_cycles = chain_cycles;
   cudaStream_t cs = nullptr;
@@ -1199,7 +1214,7 @@ int glp_batch_prepare(glp_ctx *c, uint32_t count, glp_problem *const *problems,
   b->mp.counter = &c->d_record->counter;
   b->mp.stats = c->d_record->stats;
   b->mp.error = &c->d_record->error;
-  const Shape sh = choose_shape(c, total, true, vq, table[0].pen, streams);
+  const Shape sh = choose_shape(c, table.data(), count, true, vq);
   b->P = sh.P;
   b->fn = multi_kernel(sh, vq);
   b->grid = grid_for(c, b->fn, total, b->P, &rc);
@@ -2080,13 +2095,9 @@ extern "C" int glp_run_generation_noalloc(const glp_generation_args *a, const fl
   // choose_lanes without a context's history), from the resident threads
   // measured at set-up.  Without hmm_work the scratch bounds no rows: they may
   // exceed L2 (20,000 x 512 at 8 lanes 1.70 ms; as for rows in L2, at 4, 2.33).
-  glp::WidthAsk ask;
-  ask.rate = kUsualRate;
-  ask.samples = N;
-  ask.sms = sms;
-  ask.streams = mark_stream(su.l2_bytes, sms, &p, 1);
+  mark_stream(su.l2_bytes, sms, &p, 1);
+  glp::WidthAsk ask = width_ask(&p, 1, kUsualRate, false, sms, su.l2_bytes);
   ask.widest = glp::kWidest;
-  ask.block_threads = glp::kThreads;
   ask.resident = su.resident;
   const uint32_t P = glp::pick_lanes(ask);
   Shape sh;

@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 
 namespace glp {
 
@@ -56,9 +57,11 @@ constexpr SpecShape make_spec_shape(int i) {
 constexpr bool kSpecTree(int P) { return P >= 16; }
 
 // The positions that a chain goes on a round, on average, at acceptance rate a with
-// P lanes: the chances that the first P / 2 nodes of its tree are reached.  For all
-// widths in one pass, a node's from its parent's: steps[i] for 2^i lanes (as powers
-// of a and 1 - a, node by node and width by width, they took 14 us a launch).
+// P lanes: the chances that the first P / 2 nodes of its tree are reached.  On a line
+// of refusals (kernels without trees) an acceptance does not end the round where the
+// next positions replace the same slot, each with a chance of a quarter.  For all
+// widths in one pass, a node's chance from its parent's: steps[i] for 2^i lanes; line
+// [i] is that of a line of a node less (a chain's first round, after its root).
 constexpr int kWidths = 8;  // 1 << 0 .. 1 << 7 lanes
 struct SpecShapes {
   SpecShape of[kSpecRates];
@@ -69,91 +72,138 @@ constexpr SpecShapes make_spec_shapes() {
     t.of[i] = make_spec_shape(i);
   return t;
 }
-inline void steps_a_round(double a, double (&steps)[kWidths]) {
+inline void steps_a_round(double a, double (&steps)[kWidths], double (&line)[kWidths]) {
   static constexpr SpecShapes shapes = make_spec_shapes();
   const SpecShape &tree = shapes.of[std::min((int)(a * 16.0 + 0.5), kSpecRates - 1)];
-  double chance[kTeamNodes], sum = 0.0, line = 0.0, refused = 1.0;
-  steps[0] = 0.0;
+  double chance[kTeamNodes], sum = 0.0;
+  // of the line: the chances of its nodes, and of them those whose runs have
+  // 4^-k left (k nodes on)
+  double refusals = 0.0, runs = 0.0, refused = 1.0, last = 0.0;
+  steps[0] = line[0] = 0.0;
   for (int n = 0, next = 1; n < kTeamNodes; ++n) {
     chance[n] = n == 0 ? 1.0 : chance[tree.parent[n]] * (tree.accept[n] ? a : 1.0 - a);
     sum += chance[n];
-    line += refused;
+    refusals += refused;
+    runs = 0.25 * runs + refused;
     refused *= 1.0 - a;
+    // sum over the nodes of chance (1 + a (1/4 + 1/16 + ... to the line's end))
+    const double all = refusals + a / 3.0 * (refusals - runs);
     if (n + 1 == 1 << (next - 1)) {
-      steps[next] = kSpecTree(1 << next) ? sum : line;
+      steps[next] = kSpecTree(1 << next) ? sum : all;
+      line[next] = last;
       ++next;
     }
+    last = all;
   }
 }
 
 // What a launch is asked a width for.
 struct WidthAsk {
-  double rate = 0.12;        // acceptance rate, about
-  uint64_t samples = 0;      // of all chunks
-  int sms = 0;
-  bool vq = false, streams = false;  // rows beyond half of L2
+  double rate = 0.12;     // acceptance rate, about
+  uint64_t samples = 0;   // of all chunks
+  double sites = 0;       // of a sample, on average
+  double cycles = 0;      // of a chain, on average
+  bool vq = false;
   uint32_t widest = 32;
-  const double *resident = nullptr;  // threads, for 2^i lanes
+  int sms = 0;
+  double l2_bytes = 0;
+  const double *resident = nullptr;  // threads that the GPU holds, for 2^i lanes
   uint32_t block_threads = 128;
 };
 
-// Speculation width for N samples at acceptance rate a.  A generation lasts as
-// long as its longest chain while every sample has a group of its own, so the
-// rule compares, for each width, the rounds of a chain whose rate is off the
-// average, a or a' = a + min(a, 0.12), whichever goes on fewer positions a round,
-// times what a warp's round costs at the warps a scheduler holds.  Measured
-// (1,024 sites, a = 0.12, times of a generation kernel relative to one warp a
-// scheduler): 1.44 at two, 2.0 at three, beyond that in proportion (whole blocks of
-// four warps, so the steps are at multiples of the SM count).  Narrow groups stage
-// more rows a lane and read a row for fewer evaluations: at 4 lanes 1.25, on VQ
-// codes 1.5, and where the rows exceed half of L2 1.9 (measured against 8 lanes 1.5
-// to 2.2: 20,000 x 512 at 8 lanes 1.65 ms, 4: 2.37; 15,000 x 2,048 4.66 and 8.28;
-// 40,000 x 100, whose rows stay, 2.36 and 2.02); at 2 lanes, one block an SM, 2.7;
-// at 8 lanes 1.05, and 1.1 for such rows (2,000 x 4,096 2.65 ms, 16: 2.35); on VQ
-// codes, whose table reads conflict more in a wide group, 1.15 from 32.  The widths
-// this picks, against others: 256 samples 64 lanes 0.27 ms (32: 0.36, 8: 0.55),
-// 1,000 samples 16 lanes 0.55 (0.76; 32: 0.64), 1,500 x 2,048 8 lanes 1.07 (16:
-// 1.14), 2,500 x 2,048 16 lanes 1.42 (8: 1.51), 3,001 x 4,000 from codes 16 lanes
-// 3.47 (8: 3.68; 32: 4.52), 10,000 samples 8 lanes 2.05 (16: 2.49).
-// 64 and 128 lanes are teams of two and four warps, for one chunk alone.  They are
-// picked while every warp has a scheduler of its own: 152 x 1,024 128 lanes 0.237 ms
-// (32: 0.369), 300 64 lanes 0.281 (0.355), 400 32 lanes 0.353.
-inline double lane_round_cost(uint32_t P, bool vq, bool streams) {
-  switch (P) {
-    case 2: return 2.7;
-    case 4: return vq ? 1.5 : streams ? 1.9 : 1.25;
-    case 8: return streams ? 1.1 : 1.05;
-    case 16: return 1.0;
-    default: return vq ? 1.15 : 1.0;
-  }
+// Speculation width of a launch: the width with the least time by a model of a
+// generation, fitted to the times of every width from 4 lanes on at 2,496 points (3 to
+// 40,000 samples of 3 to 8,192 sites, 5 to 100 cycles, acceptance rates 0.1 to 0.99,
+// emission rows and codes), those of 50 cycles and more at rates below 0.7 with the
+// most weight.  Its picks take 1.0 % longer than the best width on average, 17 % at the
+// 99th percentile (at those 0.5 and 8 %); the rule before it, which knew neither the
+// cycles nor what of the rows is in use at a time, 4.5 %, 60 % and at worst 125 %.
+//
+// A chain of C cycles has C + 1 positions.  Its first round goes over the starting
+// quadruple and a line of refusals, the others as far as steps_a_round says.  While
+// every sample has a group of its own, the generation lasts as long as its longest
+// chain: one whose rate is off the average, a or a + min(a, kOff), whichever takes
+// more rounds.  A round takes as much longer as blocks share an SM's schedulers (one
+// block is a warp on each; between whole blocks kBetween of the way up to the next),
+// the less the fewer sites it has, since its other parts wait more than they compute.
+// Beyond the blocks that fit, groups take samples in turn: the mean chain's rounds
+// times the turns, and kTail of the longest chain's.  Narrow groups stage more rows a
+// lane and have fewer warps to wait for them, which costs where the rows in use exceed
+// half of L2 -- those of the resident samples, not of all.  From 16 lanes on the trees
+// add to every round.
+//
+// What it decides, in ms (width: time): 256 x 1,024 64: 0.27 (32: 0.36); 1,000 x 1,024
+// 16: 0.42 (8: 0.57, 32: 0.48); 800 x 2,048 16: 0.73 (32: 0.85); 2,000 x 4,096 16: 2.16
+// (8: 2.58); 5,000 x 1,024 8: 1.10 (16: 1.14); 10,000 x 4,096 8 (16: 1.9 times as long);
+// 10,000 x 100 4: 0.66 (8: 0.72, 16: 0.93); 20,000 x 300 at a rate of 0.46, 20 cycles,
+// 4: 0.54 (8: 0.64, 16: 0.84); 40,000 x 1,024 8 (4: 1.6 times).  2 lanes, one block an SM,
+// were never the best.
+constexpr double kOff = 0.513;
+struct WidthCost {
+  double alone;   // a round where an SM holds one block, beside 16 lanes
+  double shared;  // added for each further block
+  double alone_beyond, shared_beyond;  // both grow so with the rows in use beyond kFrom
+};
+inline double generation_time(const WidthAsk &ask, int width, const double *mean,
+                              const double *mean_line, const double *off,
+                              const double *off_line) {
+  static constexpr WidthCost kRows[kWidths] = {{},
+                                               {},
+                                               {1.077, 0.315, 1.07, 0.734},
+                                               {0.92, 0.404, 0.56, 0.017},
+                                               {1.0, 0.382, 0, 0},
+                                               {0.999, 0.412, 0, 0},
+                                               {0.996, 0.485, 0, 0},
+                                               {0.994, 0.474, 0, 0}};
+  static constexpr WidthCost kCodes[kWidths] = {{},
+                                                {},
+                                                {0.959, 0.528, 0, 0},
+                                                {0.952, 0.409, 0, 0},
+                                                {1.0, 0.317, 0, 0},
+                                                {1.145, 0.283, 0, 0},
+                                                {0.987, 0.383, 0, 0},
+                                                {0.977, 0.513, 0, 0}};
+  constexpr double kTail = 0.372, kBetween = 0.734, kFrom = 0.476, kSpan = 0.28;  // of L2
+  constexpr double kWaits = 68.201, kTrees = 27.377, kTreesOf = 50.0;             // sites
+  const WidthCost cost = ask.vq ? kCodes[width] : kRows[width];
+  const uint32_t P = 1u << width;
+  auto rounds = [&](const double *steps, const double *line) {
+    const double left = ask.cycles + 1.0 - (1.0 + line[width]);
+    return left <= 0.0 ? 1.0 : 1.0 + std::max(left / steps[width], left > 0.5 ? 1.0 : left);
+  };
+  const double average = rounds(mean, mean_line),
+               longest = std::max(average, rounds(off, off_line));
+  const double groups = (double)ask.block_threads / P;
+  const double blocks = std::ceil((double)ask.samples / groups);
+  const double fit = std::max(1.0, ask.resident[width] / ((double)ask.block_threads * ask.sms));
+  const double in_use =  // of L2, by the resident samples' rows
+      std::min((double)ask.samples, fit * ask.sms * groups) * ask.sites * 16.0 / ask.l2_bytes;
+  const double beyond = std::min(std::max(in_use - kFrom, 0.0), kSpan);
+  const double alone = cost.alone * (1.0 + cost.alone_beyond * beyond);
+  const double more = cost.shared * (1.0 + cost.shared_beyond * beyond) * ask.sites /
+                      (ask.sites + kWaits);
+  auto shared = [&](double held) { return 1.0 + more * (held - 1.0); };
+  const double exact = blocks / ask.sms, whole = std::ceil(exact);
+  const double time = whole <= fit
+                          ? longest * shared(std::max(1.0, exact + kBetween * (whole - exact)))
+                          : shared(fit) * (average * exact / fit + kTail * longest);
+  return time * alone * (kSpecTree((int)P) ? 1.0 + kTrees / (ask.sites + kTreesOf) : 1.0);
 }
 
 inline uint32_t pick_lanes(const WidthAsk &ask) {
-  const double a = ask.rate, as = std::min(a + std::min(a, 0.12), 1.0);
-  double mean[kWidths], off[kWidths];
-  steps_a_round(a, mean);
-  steps_a_round(as, off);
+  const double a = ask.rate, as = std::min(a + std::min(a, kOff), 1.0);
+  double mean[kWidths], off[kWidths], mean_line[kWidths], off_line[kWidths];
+  steps_a_round(a, mean, mean_line);
+  steps_a_round(as, off, off_line);
   uint32_t best = 8;
   double best_time = 0;
-  for (int i = 1; 1u << i <= ask.widest; ++i) {
+  for (int i = 2; 1u << i <= ask.widest; ++i) {
     if (ask.resident[i] <= 0)
       continue;
-    const uint32_t P = 1u << i;
-    const double consumed = std::min(mean[i], off[i]);
-    const uint64_t per_block = ask.block_threads / P;
-    const uint64_t blocks = (ask.samples + per_block - 1) / per_block;
-    // blocks an SM holds at a time, and for one warp a scheduler in each
-    const double most = std::max(1.0, ask.resident[i] / ((double)ask.block_threads * ask.sms));
-    const double held = (double)((blocks + ask.sms - 1) / ask.sms);
-    auto warps_cost = [](double w) { return w <= 1 ? 1.0 : w <= 2 ? 1.44 : w * (2.0 / 3.0); };
-    const double a_block = ask.block_threads / 128.0;  // warps a scheduler
-    const double warps = held <= most
-                             ? warps_cost(held * a_block)
-                             : warps_cost(most * a_block) * ((double)blocks / ask.sms) / most;
-    const double time = warps * lane_round_cost(P, ask.vq, ask.streams) / consumed;
-    if (best_time == 0 || time < best_time * 0.98) {
+    const double time = generation_time(ask, i, mean, mean_line, off, off_line);
+    if (best_time == 0 || time < best_time) {
       best_time = time;
-      best = P;
+      best = 1u << i;
     }
   }
   return best;
