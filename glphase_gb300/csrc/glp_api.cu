@@ -1635,8 +1635,14 @@ int glp_tally(glp_ctx *c, const uint64_t *haps, uint32_t N, uint32_t S, uint32_t
     return rc;
   if (!haps || !hsum || N == 0 || S == 0)
     return fail(c, GLP_ERR_ARG, "haps, hsum, num_samples and num_sites are required");
-  auto fn = (S & 3u) == 0 && ((uintptr_t)hsum & 15u) == 0 ? glp::replace_kernel<4>
-                                                          : glp::replace_kernel<1>;
+  const bool aligned = (S & 3u) == 0 && ((uintptr_t)hsum & 15u) == 0;
+  const int hold = glp::tally_hold(S);
+  auto fn = aligned ? (hold == 1   ? glp::replace_kernel<1, true>
+                       : hold == 2 ? glp::replace_kernel<2, true>
+                                   : glp::replace_kernel<4, true>)
+                    : (hold == 1   ? glp::replace_kernel<1, false>
+                       : hold == 2 ? glp::replace_kernel<2, false>
+                                   : glp::replace_kernel<4, false>);
   fn<<<N, glp::tally_threads(S), 0, c->stream>>>(haps, N, S, (S + 63) / 64, hsum);
   GLP_CUDA(c, cudaGetLastError());
   return GLP_OK;
