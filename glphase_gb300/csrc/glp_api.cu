@@ -1656,6 +1656,14 @@ int glp_result(glp_ctx *c, const uint32_t *hsum, uint32_t N, uint32_t S, uint32_
   if (!hsum || !prob_out || N == 0 || S == 0 || sn == 0)
     return fail(c, GLP_ERR_ARG, "hsum, prob_out, sizes and sampling_generations are required");
   const float norm = (float)(1.0 / sn);
+  const uint64_t entries = (uint64_t)2 * N * S;
+  if (entries <= glp::kResultSmall) {
+    constexpr uint32_t threads = glp::kResultSmallThreads;
+    glp::result_small_kernel<<<(unsigned)((entries + threads - 1) / threads), threads, 0,
+                               c->stream>>>(hsum, 2 * N, S, norm, prob_out);
+    GLP_CUDA(c, cudaGetLastError());
+    return GLP_OK;
+  }
   const uint32_t site_tiles = (uint32_t)(((uint64_t)S + glp::kResultTile - 1) / glp::kResultTile);
   const uint64_t tiles =
       site_tiles * (((uint64_t)2 * N + glp::kResultTile - 1) / glp::kResultTile);

@@ -171,6 +171,18 @@ __global__ void __launch_bounds__(kHold == 4 ? 1024 : 128)
 // (impute.cpp:599-613), binary32.  Tiles of 64 haplotypes x 64 sites turned in
 // shared memory, so that both sides move 256 bytes a row.  Bound: HBM (10,000 x
 // 4,096: 388 us with one thread an entry reading down a column, 114 us, 5.8 TB/s).
+// Few entries, whose columns stay in L1, take one thread each, without a tile's
+// two trips: 500 x 3 2.9 us (4.2 by tiles), 60 x 255 3.8 (4.2), level at 2^18 entries.
+constexpr uint64_t kResultSmall = (uint64_t)1 << 18;
+constexpr uint32_t kResultSmallThreads = 256;
+__global__ void __launch_bounds__(kResultSmallThreads)
+    result_small_kernel(const uint32_t *__restrict__ hsum, uint32_t H, uint32_t S, float norm,
+                        float *__restrict__ prob_out) {
+  const uint32_t i = blockIdx.x * kResultSmallThreads + threadIdx.x, m = i / H, h = i % H;
+  if (m < S)
+    prob_out[i] = (float)__ldg(hsum + h * S + m) * norm;
+}
+
 constexpr uint32_t kResultTile = 64, kResultThreads = 256;
 __global__ void __launch_bounds__(kResultThreads)
     result_kernel(const uint32_t *__restrict__ hsum, uint32_t N, uint32_t S, uint32_t site_tiles,

@@ -1,7 +1,8 @@
 """Tallies of rows of any length and alignment (vectors of each row's own, single
-sites at its ends, one to four vectors a thread, rows read twice), as the oracle gives
-them.  Rows that are short, or no multiple of four sites, take about as long as their
-neighbours that are neither."""
+sites at its ends, one to four vectors a thread, rows read twice), and probabilities
+around the size from which tiles are turned: as the oracle and numpy give them.  Rows
+that are short, or no multiple of four sites, take about as long as their neighbours
+that are neither."""
 import numpy as np
 import pytest
 
@@ -23,6 +24,10 @@ def dev():
 
 def tally(dev, haps, N, S, ptr):
     dev._c(dev.L.glp_tally(dev.ctx, haps.data_ptr(), N, S, ptr))
+
+
+def result(dev, ptr, N, S, prob):
+    dev._c(dev.L.glp_result(dev.ctx, ptr, N, S, 3, prob.data_ptr()))
 
 
 @pytest.mark.parametrize("offset", [0, 1, 2, 3])
@@ -49,17 +54,38 @@ def test_rows(oracle_lib, dev, S, offset):
     assert (got[:offset] == 77).all() and (got[offset + 2 * N * S:] == 77).all()
 
 
-def time_us(dev, N, S, n=50):
+@pytest.mark.parametrize("N,S", [(512, 255), (512, 256), (512, 257), (1, 131072), (1, 131073),
+                                 (131072, 1), (131073, 1), (2100, 63), (2100, 64), (2100, 65),
+                                 (33, 4001), (64, 6400)])
+def test_result(dev, N, S):
+    import torch
+    rng = np.random.default_rng(N + S)
+    cpu = rng.integers(0, 2**32, size=(2 * N, S), dtype=np.uint64).astype(np.uint32)
+    hsum = torch.from_numpy(cpu.view(np.int32)).cuda()
+    prob = torch.full((S + 1, 2 * N), -1.0, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    result(dev, hsum.data_ptr(), N, S, prob)
+    dev._c(dev.L.glp_finish(dev.ctx))
+    got = prob.cpu().numpy()
+    assert np.array_equal(got[:S], cpu.T.astype(np.float32) * np.float32(1.0 / 3))
+    assert (got[S] == -1.0).all()
+
+
+def time_us(dev, what, N, S, n=50):
     import torch
     haps = torch.randint(-2**62, 2**62, (2 * N, (S + 63) // 64), device="cuda")
     hsum = torch.randint(0, 20, (2 * N, S), device="cuda", dtype=torch.int32)
+    prob = torch.zeros((S, 2 * N), device="cuda")
     torch.cuda.synchronize()
     best = float("inf")
     for _ in range(8):
         a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
         a.record(dev.torch_stream)
         for _ in range(n):
-            tally(dev, haps, N, S, hsum.data_ptr())
+            if what == "tally":
+                tally(dev, haps, N, S, hsum.data_ptr())
+            else:
+                result(dev, hsum.data_ptr(), N, S, prob)
         b.record(dev.torch_stream)
         b.synchronize()
         best = min(best, a.elapsed_time(b) / n * 1e3)
@@ -68,4 +94,9 @@ def time_us(dev, N, S, n=50):
 
 @pytest.mark.parametrize("N,S,even", [(8000, 101, 100), (20000, 3, 64), (4000, 4097, 4096)])
 def test_tally_time(dev, N, S, even):
-    assert time_us(dev, N, S) < 1.6 * time_us(dev, N, even)
+    assert time_us(dev, "tally", N, S) < 1.6 * time_us(dev, "tally", N, even)
+
+
+def test_result_time(dev):
+    # few entries in less time than the least number that is turned in tiles
+    assert time_us(dev, "result", 500, 3) < 0.9 * time_us(dev, "result", 1100, 120)
