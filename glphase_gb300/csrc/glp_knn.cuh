@@ -130,14 +130,19 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *red,
 // comes from the threads' minima -- at least `half` distances are at most the
 // half-th smallest minimum -- by a binary search that costs one counting barrier a
 // step; the entries up to the bound are collected and put in (distance, index)
-// order by counting, for each, how many are smaller.  Rows that leave more
-// than kSelectMost entries (many equal distances) or have too few threads for a
-// useful bound take the general path: the exact threshold by a binary search over
-// all distances, ties in index order by a block scan, a bitonic sort.
+// order by counting, for each, how many are smaller.  Where fewer threads than
+// `half` hold a distance the bound is the half-th smallest itself, by a search that
+// counts all of the registers' distances, or, up to kSelectAll haplotypes, all are
+// collected (a table of 1,000 haplotypes x 1,000 sites, half = 200, takes 75 us with
+// the search and 175 with all collected; 400, 100, 62 and 66; 300, 100, 60 and 59; 100,
+// 25, 56 and 52).
+// Rows that leave more than kSelectMost entries (many equal distances) take the
+// general path: the exact threshold by a binary search over all distances, ties in
+// index order by a block scan, a bitonic sort.
 // Bound: instructions and the search's barriers (10,000 samples, 20,000
 // haplotypes, half = 100: 0.40 ms; 2.29 ms with the general path for every row,
 // one block an SM with its rows in shared memory).
-constexpr uint32_t kSelectMost = 1024;
+constexpr uint32_t kSelectMost = 1024, kSelectAll = 320;
 
 // The general path: the `half` smallest (d, index) of the entries of row d that
 // are not kKnnExcluded and not in `taken` (may be null), written sorted to
@@ -220,11 +225,11 @@ __device__ __noinline__ void select_general(const uint16_t *__restrict__ d, uint
 template <int kV>
 __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, uint32_t H,
                                                uint32_t half, uint32_t dmax,
-                                               const uint32_t *taken, uint32_t want,
-                                               uint32_t *keys, uint32_t *red, uint32_t *out,
-                                               const int *error, int &flags) {
+                                               const uint32_t *taken, uint32_t *keys,
+                                               uint32_t *red, uint32_t *out, const int *error,
+                                               int &flags) {
   const uint32_t tid = threadIdx.x;
-  __shared__ uint32_t found;
+  __shared__ uint32_t found, counts[3];
   uint4 v[kV];
 #pragma unroll
   for (int i = 0; i < kV; ++i) {
@@ -238,11 +243,18 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
         v[i].z = 0xffffffffu;
       v[i].w = 0xffffffffu;
     }
+    const uint32_t gone = kV == 1 && taken && h < H ? (taken[h >> 5] >> (h & 31u)) & 255u : 0u;
+    if (gone) {  // bits to halves of the words
+      v[i].x |= (gone & 1u) * 0xffffu | (gone >> 1 & 1u) * 0xffff0000u;
+      v[i].y |= (gone >> 2 & 1u) * 0xffffu | (gone >> 3 & 1u) * 0xffff0000u;
+      v[i].z |= (gone >> 4 & 1u) * 0xffffu | (gone >> 5 & 1u) * 0xffff0000u;
+      v[i].w |= (gone >> 6 & 1u) * 0xffffu | (gone >> 7 & 1u) * 0xffff0000u;
+    }
   }
   if (error)  // beside the row's loads
     flags = *error;
   if (tid == 0)
-    found = 0;
+    found = counts[0] = 0;
   // the least distance of each thread; the pitch's padding is excluded like an own
   // haplotype
   uint32_t least = 0xffffffffu;
@@ -251,18 +263,46 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
     least = __vminu2(least, __vminu2(__vminu2(v[i].x, v[i].y), __vminu2(v[i].z, v[i].w)));
   }
   least = min(least & 0xffffu, least >> 16);
-  // smallest u with at least `want` threads' minima <= u (all distances when
-  // there are too few)
+  // smallest u with at least `want` threads' minima <= u, or distances where too few
+  // threads hold one.  In wide rows the taken ones, at most `half`, are still there
+  // (taking them out of the registers first cost the fourth block an SM).
+  const int want = (int)(kV > 1 && taken ? 2 * half : half);
   uint32_t lo = 0, hi = dmax + 1;
-  const bool bounded = __syncthreads_count(least <= dmax) >= (int)want;
+  const bool bounded = __syncthreads_count(least <= dmax) >= want;
   while (bounded && lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (__syncthreads_count(least <= mid) >= (int)want)
+    if (__syncthreads_count(least <= mid) >= want)
       hi = mid;
     else
       lo = mid + 1;
   }
-  const uint32_t u = bounded ? lo : dmax;
+  if (!bounded)
+    lo = hi = dmax;
+  // wider rows give every thread a distance
+  if (kV == 1 && !bounded && H > kSelectAll) {
+    lo = 0;
+    // a step's count is cleared one step ahead, when all have read its last value
+    for (uint32_t now = 0; lo < hi;) {
+      const uint32_t mid = (lo + hi) >> 1, mid2 = mid | mid << 16, next = now == 2 ? 0 : now + 1;
+      uint32_t c = 0;
+#pragma unroll
+      for (int i = 0; i < kV; ++i)
+        c += __vsetleu2(v[i].x, mid2) + __vsetleu2(v[i].y, mid2) + __vsetleu2(v[i].z, mid2) +
+             __vsetleu2(v[i].w, mid2);
+      c = __reduce_add_sync(0xffffffffu, (c & 0xffffu) + (c >> 16));
+      if ((tid & 31u) == 0 && c)
+        atomicAdd(&counts[now], c);
+      if (tid == 0)
+        counts[next] = 0;
+      __syncthreads();
+      if (counts[now] >= half)
+        hi = mid;
+      else
+        lo = mid + 1;
+      now = next;
+    }
+  }
+  const uint32_t u = lo;
   if (least <= u) {
 #pragma unroll
     for (int i = 0; i < kV; ++i) {
@@ -272,7 +312,7 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
         const uint32_t dist = (x[j >> 1] >> (16 * (j & 1))) & 0xffffu;
         if (dist <= u) {
           const uint32_t h = 8 * (i * kKnnThreads + tid) + j;
-          if (!(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
+          if (kV == 1 || !(taken && ((taken[h >> 5] >> (h & 31u)) & 1u))) {
             const uint32_t n = atomicAdd(&found, 1u);
             if (n < kSelectMost)
               keys[n] = (dist << 16) | h;
@@ -500,14 +540,13 @@ __global__ void __launch_bounds__(kKnnThreads)
   int flags = 0;
   for (uint32_t i = tid; i < (H + 31) / 32; i += kKnnThreads)
     taken[i] = 0;
-  select_nearest<kV>(row, H, half, dmax, nullptr, half, keys, red, chosen, error, flags);
+  select_nearest<kV>(row, H, half, dmax, nullptr, keys, red, chosen, error, flags);
   for (uint32_t i = tid; i < half; i += kKnnThreads)
     if (chosen[i] < H)
       atomicOr(&taken[chosen[i] >> 5], 1u << (chosen[i] & 31u));
   __syncthreads();
-  // at most `half` of the second row's nearest are taken
-  select_nearest<kV>(row + pitch, H, half, dmax, taken, 2 * half, keys, red,
-                     chosen + kKnnMaxHalf, nullptr, flags);
+  select_nearest<kV>(row + pitch, H, half, dmax, taken, keys, red, chosen + kKnnMaxHalf, nullptr,
+                     flags);
   const bool failed = (flags & kGemmTimeout) != 0;
   for (uint32_t i = tid; i < half; i += kKnnThreads) {
     out[2 * i] = failed ? kKnnNoHap : chosen[i];
