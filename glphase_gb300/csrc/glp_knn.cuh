@@ -505,16 +505,18 @@ __global__ void __launch_bounds__(kDistThreads)
 }
 
 // The chunks of 8 words that knn_tract_dist_kernel takes exactly: the first where
-// it is all of the words (`best` would rise inside most of them), where all tiles are
-// computed and it is more than half of the words, and where fewer tiles than SMs
+// the words are six at most (`best` would rise inside most of them), where all tiles
+// are computed and it is more than half of the words, and where fewer tiles than SMs
 // leave a pair's chain of words to wait for; else none.  Tables in ms with none /
 // one, typical haplotypes and (random ones), and in one pass over all tiles, as
-// before either: 14,000 x 64 2.21 / 0.82 (1.73 / 0.84), 2.29; 14,000 x 512 3.58 / 3.87
-// (5.95 / 3.89), 8.84; 14,000 x 1,024 5.31 / 6.21 (7.60 / 7.09), 15.9; all tiles,
+// before either: 14,000 x 64 2.21 / 0.82 (1.73 / 0.84), 2.29; 14,000 x 384 3.33 / 3.10
+// (5.33 / 3.13), 7.13; 14,000 x 448 3.44 / 3.53 (5.78 / 3.60), 7.95; 14,000 x 500 4.53 /
+// 5.08 (8.29 / 7.14), 11.3; 14,000 x 1,024 5.31 / 6.21 (7.60 / 7.09), 15.9; all tiles,
 // 24,000 x 1,024 30.0 / 35.4 (43.4 / 40.4), 45.3; few, 200 x 1,000 0.074 / 0.072 (0.104
 // / 0.087), 0.098; 800 x 1,024 0.107 / 0.118 (0.130 / 0.121), 0.151.
+constexpr uint32_t kTractExactWords = 6;
 inline uint32_t tract_exact_chunks(uint32_t wn, bool sym, uint64_t tiles, int sms) {
-  return wn <= kDistW || (!sym && wn < 2 * kDistW) || tiles <= (uint64_t)sms ? 1 : 0;
+  return wn <= kTractExactWords || (!sym && wn < 2 * kDistW) || tiles <= (uint64_t)sms ? 1 : 0;
 }
 
 // The neighbour lists of the samples s0 + blockIdx.x from their rows of

@@ -1,6 +1,7 @@
 """Neighbour tables of panels whose rows fewer threads hold than a list has entries:
 identical to distances and a stable sort in numpy on both sides of the rules that
-choose the list's bound, and in times that grow with the lists' lengths and no faster."""
+choose the list's bound, and in times that grow with the lists' lengths and no faster.
+Tract distances of few words, around the number up to which they are taken exactly."""
 import time
 
 import numpy as np
@@ -10,6 +11,7 @@ from glphase_gb300 import model as mdl
 from glphase_gb300.hmmlike import HMMLikeCUDA
 from test_gpu_knn import gpu_knn
 from test_gpu_knn_edges import bits_of, want
+from test_gpu_knn_tract_forms import haplotypes
 
 pytestmark = pytest.mark.gpu
 
@@ -32,6 +34,15 @@ def test_lists(dev, H, S, K, kind):
     samples = sorted({0, H // 2 - 1, *rng.integers(0, H // 2, size=8).tolist()})
     got = gpu_knn(dev, mdl.pack_haplotypes(bits), S, K)
     assert np.array_equal(got[samples], want(bits, K, samples))
+
+
+@pytest.mark.parametrize("kind", ["half", "tracts", "none"])
+@pytest.mark.parametrize("S", [383, 384, 385, 448, 449, 512])
+def test_tract_words(dev, S, kind):
+    bits = haplotypes(1300, S, kind)
+    samples = [0, 1, 325, 649]
+    got = gpu_knn(dev, mdl.pack_haplotypes(bits), S, 60, metric="tract")
+    assert np.array_equal(got[samples], want(bits, 60, samples, "tract"))
 
 
 def table_us(dev, H, S, K):
