@@ -498,8 +498,10 @@ __device__ __forceinline__ void block8(FState &x, const E &em, const float4 *slo
 // Log-likelihood of one quadruple by a plain forward pass, site by site, with
 // the per-site power-of-two rescaling of fwd_step (the scheme of
 // impute.cpp:327-376), reading emission, transition and parent words straight
-// from global memory.  Used, rarely, for an evaluation whose blocked pass may
-// have lost range.
+// from global memory, four sites' rows at a time.  Used, rarely, for an evaluation
+// whose blocked pass may have lost range: a lone lane's walk, so that a generation
+// ends as late as its redos follow one another (400 x 2,048 with every evaluation made
+// again 4.10 ms, from codes 5.01; with one site's rows at a time 5.81 and 8.38).
 template <class E>
 __device__ __noinline__ double like_forward(const uint64_t *__restrict__ haps, uint32_t wn,
                                             uint32_t S, const float4 *__restrict__ tran4,
@@ -509,13 +511,27 @@ __device__ __noinline__ double like_forward(const uint64_t *__restrict__ haps, u
   for (uint32_t w = 0; w < wn; ++w) {
     const Parents pw = load_parents(haps, wn, q, w);
     const uint32_t end = min(S, (w + 1) * 64);
-    for (uint32_t m = w * 64; m < end; ++m) {
-      const uint32_t j = m & 63u;
+    auto site = [&](const float4 e, const float4 t, uint32_t j) {
       float s00, s01, s10, s11;
-      select4(em.get1(m), (pw.f0 >> j) & 1, (pw.f1 >> j) & 1, (pw.m0 >> j) & 1,
-              (pw.m1 >> j) & 1, s00, s01, s10, s11);
-      fwd_step(f, __ldg(tran4 + m), s00, s01, s10, s11);
+      select4(e, (pw.f0 >> j) & 1, (pw.f1 >> j) & 1, (pw.m0 >> j) & 1, (pw.m1 >> j) & 1, s00,
+              s01, s10, s11);
+      fwd_step(f, t, s00, s01, s10, s11);
+    };
+    uint32_t m = w * 64;
+#pragma unroll 1
+    for (; m + 4 <= end; m += 4) {  // four sites' rows loaded together
+      float4 e[4], t[4];
+      em.get4(m, e);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        t[j] = __ldg(tran4 + m + j);
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j)
+        site(e[j], t[j], (m & 63u) + j);
     }
+#pragma unroll 1
+    for (; m < end; ++m)
+      site(em.get1(m), __ldg(tran4 + m), m & 63u);
     fwd_guard(f);
   }
   const double sum = (((double)f.X.x + (double)f.X.y) + (double)f.Y.y) + (double)f.Y.x;
