@@ -357,10 +357,11 @@ __device__ __forceinline__ void select_nearest(const uint16_t *__restrict__ d, u
 // each word's longest run found on its own, whose cost is the same for all
 // haplotypes (tract_exact_chunks).
 // Bound: the ALU instructions of a pair's word (89 % of that pipe).  4,990
-// haplotypes x 1,024 sites, a table: 2.14 ms with all tiles in one pass, 0.74 with
-// the tiles of one half in two, 0.87 with the first chunk exact; of haplotypes that
-// agree at half of the sites at random (no long runs: `best` rises for longer, and
-// every lane waits) 2.14, 1.06 and 0.99.  20,000 x 4,096 119 -> 33 ms.
+// haplotypes x 1,024 sites, a table: 2.15 ms with all tiles in one pass, 0.77 with
+// the tiles of one half in two; of haplotypes that agree at half of the sites at random
+// (no long runs: `best` rises for longer, and every lane waits) 2.15 and 1.02.  The
+// test inside has three forms; with a fourth for `best` from 3 to 14 0.773 and 1.10
+// (more code to fetch), with two 0.792 and 1.20.  20,000 x 4,096 119 -> 34 ms.
 constexpr uint32_t kTractQ = 32, kTractH = 64, kDistW = 8, kDistThreads = 256;
 template <bool kSym>
 __global__ void __launch_bounds__(kDistThreads)
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(kDistThreads)
   const uint32_t chunks = (wn + kDistW - 1) / kDistW;
   const bool all_exact = chunks <= exact;
   uint32_t common = 0;
-  int form = 0;  // of the test inside: 0 tract_inside32, 1 _mid, 2 _long, 3 _any
+  int form = 0;  // of the test inside: 0 tract_inside32, 1 _any, 2 _long
   OpenRun run[2][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -417,18 +418,15 @@ __global__ void __launch_bounds__(kDistThreads)
         if (m == ~0ull) {
           // the form of the test that all of the warp's pairs may use
           if (form != 2) {
-            uint32_t least = run[0][0].best, most = least;
+            uint32_t least = run[0][0].best;
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
+              for (int j = 0; j < 4; ++j)
                 least = min(least, run[i][j].best);
-                most = max(most, run[i][j].best);
-              }
             form = __all_sync(0xffffffffu, least >= kRunLong)  ? 2
-                   : !__all_sync(0xffffffffu, least >= kRunMid) ? 0
-                   : __all_sync(0xffffffffu, most <= kRunMost)  ? 1
-                                                                : 3;
+                   : __all_sync(0xffffffffu, least >= kRunMid) ? 1
+                                                               : 0;
           }
           auto inside_word = [&](auto test) {
 #pragma unroll
@@ -441,10 +439,8 @@ __global__ void __launch_bounds__(kDistThreads)
           };
           if (form == 2)
             inside_word([](uint32_t &best, uint32_t x) { tract_inside32_long(best, x); });
-          else if (form == 3)
-            inside_word([](uint32_t &best, uint32_t x) { tract_inside32_any(best, x); });
           else if (form == 1)
-            inside_word([](uint32_t &best, uint32_t x) { tract_inside32_mid(best, x); });
+            inside_word([](uint32_t &best, uint32_t x) { tract_inside32_any(best, x); });
           else
             inside_word([](uint32_t &best, uint32_t x) { tract_inside32(best, x); });
         }

@@ -117,8 +117,8 @@ struct OpenRun {
   uint32_t open, best;
 };
 constexpr uint32_t kRunFloor = 1;
-// From which tract_inside32_mid (to kRunMost) and _long may be used.
-constexpr uint32_t kRunMid = 3, kRunMost = 14, kRunLong = 7;
+// From which tract_inside32_any and _long may be used.
+constexpr uint32_t kRunMid = 3, kRunLong = 7;
 
 // The stretch followed by one word (x the disagreements at common sites, m the
 // common sites).
@@ -157,16 +157,7 @@ GLP_TRACT_FN void tract_inside32(uint32_t &best, uint32_t x) {
   }
 }
 
-// The same for `best` from kRunMid: a test that lets words without a longer run
-// pass, and beyond kRunMost (up to 38) some others too.
-GLP_TRACT_FN void tract_inside32_mid(uint32_t &best, uint32_t x) {
-  const uint32_t r1 = ~x, r2 = r1 & (r1 >> 1), r4 = r2 & (r2 >> 2), r8 = r4 & (r4 >> 4);
-  const uint32_t from = best < 7 ? r4 : r8, by = best - (best < 7 ? 3u : 7u);
-  if (from & (from >> by))
-    tract_inside32(best, x);
-}
-
-// The same for `best` from kRunMid, without that bound.
+// The same for `best` of at least kRunMid.
 GLP_TRACT_FN void tract_inside32_any(uint32_t &best, uint32_t x) {
   const uint32_t r1 = ~x, r2 = r1 & (r1 >> 1), r4 = r2 & (r2 >> 2), r8 = r4 & (r4 >> 4),
                  r16 = r8 & (r8 >> 8);

@@ -13,25 +13,22 @@ from conftest import ROOT
 
 SRC = r'''
 #include "glp_tract.h"
-// form 0, 1, 2, 3: _inside32, _mid, _long, _any where `best` lets a word start with it
+// form 0, 1, 2: _inside32, _any, _long where `best` lets a word start with it
 extern "C" uint32_t longest(const uint64_t *x, uint32_t wn, int form) {
   glp::OpenRun r{0, glp::kRunFloor};
   for (uint32_t w = 0; w < wn; ++w)
     for (int h = 0; h < 64; h += 32)
       glp::tract_extend32(r, (uint32_t)(x[w] >> h));
   for (uint32_t w = 0; w < wn; ++w) {
-    const int f = form == 2 && r.best >= glp::kRunLong                               ? 2
-                  : form == 3 && r.best >= glp::kRunMid                              ? 3
-                  : form == 1 && r.best >= glp::kRunMid && r.best <= glp::kRunMost ? 1
-                                                                                   : 0;
+    const int f = form == 2 && r.best >= glp::kRunLong  ? 2
+                  : form == 1 && r.best >= glp::kRunMid ? 1
+                                                        : 0;
     for (int h = 0; h < 64; h += 32) {
       const uint32_t y = (uint32_t)(x[w] >> h);
       if (f == 2)
         glp::tract_inside32_long(r.best, y);
-      else if (f == 3)
-        glp::tract_inside32_any(r.best, y);
       else if (f == 1)
-        glp::tract_inside32_mid(r.best, y);
+        glp::tract_inside32_any(r.best, y);
       else
         glp::tract_inside32(r.best, y);
     }
@@ -68,7 +65,7 @@ def oracle(differ):
     return best
 
 
-@pytest.mark.parametrize("form", [0, 1, 2, 3])
+@pytest.mark.parametrize("form", [0, 1, 2])
 @pytest.mark.parametrize("p", [0.05, 0.2, 0.5, 0.8, 0.95])
 def test_random_pairs(longest, form, p):
     d = (np.random.default_rng(int(100 * p)).random((3000, 192)) < p).astype(np.uint8)
@@ -76,7 +73,7 @@ def test_random_pairs(longest, form, p):
     assert np.array_equal(longest(d, form), np.where(want > 1, want, 0))
 
 
-@pytest.mark.parametrize("form", [0, 1, 2, 3])
+@pytest.mark.parametrize("form", [0, 1, 2])
 def test_one_run_of_every_length_and_place(longest, form):
     """Among disagreements, and beside a run that `best` already has from a word's
     edge: the test of each form lets no longer run pass."""
