@@ -1298,25 +1298,6 @@ __device__ __forceinline__ void place_path(uint4 &q, const Draw *window, uint32_
   }
 }
 
-// L1 prefetch of the words of haplotype h that an evaluation starts with: word 0
-// (forward), the top whole word and the partial one (backward).
-__device__ __forceinline__ void prefetch_first(const GenParams &p, uint32_t h, bool fwd) {
-  const uint64_t *const row = p.haps + (size_t)h * p.wn;
-  if (fwd) {
-    prefetch_l1(row);
-  } else {
-    const uint32_t nw = p.S >> 6;
-    prefetch_l1(row + (nw ? nw - 1 : 0));
-    prefetch_l1(row + p.wn - 1);
-  }
-}
-__device__ __forceinline__ void prefetch_first(const GenParams &p, uint4 q, bool fwd) {
-  prefetch_first(p, q.x, fwd);
-  prefetch_first(p, q.y, fwd);
-  prefetch_first(p, q.z, fwd);
-  prefetch_first(p, q.w, fwd);
-}
-
 // Work sources.  One chunk: the kernel parameter.  Many chunks: a descriptor
 // table in global memory; the samples of all chunks form one queue, chunk by
 // chunk, so a group's neighbours in the queue usually share its chunk.
@@ -1609,16 +1590,16 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
     const bool lead_lane = (li & 1u) == 0;
     const uint32_t k = active ? min(npos, C + 1 - e) : 0u;  // positions, at most
     const bool valid = depth < k, scores = valid && ev > 0;
-    // The words that the evaluation starts with, for the parents known so far.
-    if (active)
-      prefetch_first(p, q, lead_lane);
     // Draws of cycle i at entry i mod 2 Pc of the group's window, made Pc cycles
     // at a time, one a lane, when the window does not reach this round's last one
     // (or another group of the warp draws and there is room): a chain makes each
     // draw once, and the other rounds only read them.  The generators' chain of
-    // integer products stood in front of every round (with it and without the
-    // prefetches above: 3 x 3 0.241 and 0.214 ms, 3,001 x 4,000 from codes 4.52
-    // and 4.45, 2,000 x 8,192 5.72 and 5.58).
+    // integer products stood in front of every round (3 x 3 0.241 and 0.214 ms, 3,001
+    // x 4,000 from codes 4.52 and 4.45, 2,000 x 8,192 5.72 and 5.58).  The first words
+    // of the proposals' rows are not asked for ahead: that was never faster (256 x
+    // 1,024 at 64 lanes 0.296 and without it 0.292, 2,000 x 2,048 1.076 and 1.072), and
+    // where all warps ask for the same few lines, as neighbour lists over few sites
+    // make them, slow (584 x 9 at 64 lanes 0.123 and 0.075).
     Draw *const window = draws + 2 * gbase;
     const uint32_t wmask = 2 * Pc - 1, next = max(e, 1u) - 1;  // the round's first cycle
     if (__any_sync(FULL, active && drawn < min(C, e + k - 1))) {
@@ -1641,11 +1622,9 @@ __device__ __forceinline__ void generation_body(const Src &src, uint32_t *counte
       phap = d.hap;
       u = d.u;
       set_slot(myq, slot, phap);
-      prefetch_first(p, phap, lead_lane);
       if (kTree && taken) {
         uint32_t have = 1u << slot;
         place_path(myq, window, wmask, e - 1, taken, have);
-        prefetch_first(p, myq, lead_lane);
       }
     }
     double L = 0.0;
@@ -1901,7 +1880,6 @@ __device__ __forceinline__ void generation_team(const GenParams &p, const float4
                      t1 = __ldg(&node->taken[1]);
       const uint32_t depth = desc & 255u, ev = e + depth, k = min(kNodes, C + 1 - e);
       const bool valid = depth < k, scores = valid && ev > 0;
-      prefetch_first(p, q, lead_lane);
       // draws as in generation_body, for the team
       constexpr uint32_t wmask = 2 * kLanes - 1;
       if (drawn < min(C, e + k - 1)) {
@@ -1920,12 +1898,10 @@ __device__ __forceinline__ void generation_team(const GenParams &p, const float4
         const Draw d = window[(ev - 1) & wmask];
         u = d.u;
         set_slot(myq, d.slot, d.hap);
-        prefetch_first(p, d.hap, lead_lane);
         if (t0 | t1) {
           uint32_t have = 1u << d.slot;
           place_path(myq, window, wmask, e + 31, t1, have);
           place_path(myq, window, wmask, e - 1, t0, have);
-          prefetch_first(p, myq, lead_lane);
         }
       }
       const double L = eval_pair<1, E, kSub, true, false>(p, em, myq, ring, lane, 32, FULL);
